@@ -36,7 +36,9 @@ struct DevLayout {
   int nttile;
   const int2 *phtile;
   int nphtile;
-  const int2 *vtile;            // tiles over V_pppp' elements
+  // 32 x 32 tiles on and above the diagonal of each V_pppp' block: vt_off[c] of them in
+  // the channels before c, column by column within a channel
+  const int *vt_off;
   int nvtile;
 };
 
@@ -48,6 +50,12 @@ struct DevOrbits {
   const int *nx, *ny, *nz, *sz, *tz;
   const double *kx, *ky, *kz, *e;
   double volume;
+  // Momenta on one cubic lattice (k_p - k_q = step (n_p - n_q) to rounding): per orbital
+  // (nx, ny, nz) in the signed low bytes, and spin up (bit 0) and isospin +1 (bit 1); null
+  // for any other set of momenta.  nq2: one more than the largest |n_p - n_q|^2.
+  const int2 *lat;
+  double step;
+  int nq2;
 };
 
 }  // namespace ccx

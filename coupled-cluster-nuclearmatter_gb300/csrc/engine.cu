@@ -447,7 +447,12 @@ class Engine final : public IEngine {
     pot.f32_literals = p.f32_literals;
     draw_lecs(p.lec_seed, pot.lec);
     const int npp = npp_total_, nhh = nhh_total_;
-    if (ScalarOf<S>::complex && p.kind == 1)
+    if (O_.lat) {
+      lat_.alloc((size_t)lattice_table_doubles(O_, p.kind) * sizeof(double), &bytes_);
+      launch_lattice_tables(O_, pot, lat_.as<double>(), st_);
+      pot.lat = lat_.as<double>();
+      ++launches_;
+    } else if (ScalarOf<S>::complex && p.kind == 1)
       pairf_.alloc(((size_t)npp + nhh + (size_t)D_.A * D_.NP) * sizeof(double) + 8, &bytes_);
     launch_generate<S>(D_, O_, pot, Vhp_.as<S>(), Vpp_.as<S>(), Vhh_.as<S>(), W_.as<S>(), fdiag_.as<S>(), f6_.as<S>(),
                        f7_.as<S>(), res_.as<double>(), pairf_.as<double>(), npp, nhh, st_);
@@ -825,7 +830,8 @@ class Engine final : public IEngine {
     const int nc = L.fam[3].count();
     std::vector<int> P(nc), H(nc), pp_off(nc), hh_off(nc);
     std::vector<int64_t> t_off(nc), vpp_off(nc), hh2_off(nc);
-    std::vector<int2> pp_orb, hh_orb, ttile, vtile;
+    std::vector<int2> pp_orb, hh_orb, ttile;
+    std::vector<int> vt_off(nc + 1, 0);
     std::vector<int> pp_row, hh_row, pp_sgn, hh_sgn;
     int64_t vacc = 0, hacc = 0;
     hhhh_to_hhpp_.assign(L.fam[1].count(), -1);
@@ -848,7 +854,8 @@ class Engine final : public IEngine {
       pp_sgn.insert(pp_sgn.end(), pk.pp_packed.begin(), pk.pp_packed.end());
       hh_sgn.insert(hh_sgn.end(), pk.hh_packed.begin(), pk.hh_packed.end());
       for (int64_t s = 0; s < (int64_t)pk.P * pk.H; s += kTileElems) ttile.push_back(make_int2(c, (int)s));
-      for (int64_t s = 0; s < (int64_t)pk.P * pk.P; s += kTileElems) vtile.push_back(make_int2(c, (int)s));
+      const int nvt = (pk.P + 31) / 32;
+      vt_off[c + 1] = vt_off[c] + nvt * (nvt + 1) / 2;
       if (pk.hhhh >= 0) hhhh_to_hhpp_[pk.hhhh] = c;
       max_stage_ = std::max<int64_t>(max_stage_, (int64_t)pk.n_pp * std::max(pk.n_pp, pk.n_hh));
     }
@@ -950,7 +957,7 @@ class Engine final : public IEngine {
     upload(dph_off_, ph_off, &bytes_); upload(dhp_off_, hp_off, &bytes_);
     upload(dph_orb_, ph_orb, &bytes_); upload(dhp_orb_, hp_orb, &bytes_);
     upload(dph_slot_, ph_slot, &bytes_); upload(dhp_slot_, hp_slot, &bytes_);
-    upload(dttile_, ttile, &bytes_); upload(dphtile_, phtile, &bytes_); upload(dvtile_, vtile, &bytes_);
+    upload(dttile_, ttile, &bytes_); upload(dphtile_, phtile, &bytes_); upload(dvtile_, vt_off, &bytes_);
     upload(pp_sgn_, pp_sgn, &bytes_); upload(hh_sgn_, hh_sgn, &bytes_);
     upload(n4_, n4, &bytes_); upload(hp4_slot_, hp4_slot, &bytes_);
     std::vector<int64_t> v4off(v4_off_h_.begin(), v4_off_h_.end());
@@ -967,6 +974,7 @@ class Engine final : public IEngine {
     O_.sz = osz_.as<int>(); O_.tz = otz_.as<int>();
     O_.kx = okx_.as<double>(); O_.ky = oky_.as<double>(); O_.kz = okz_.as<double>(); O_.e = oe_.as<double>();
     O_.volume = L.b.L * L.b.L * L.b.L;
+    build_lattice();
 
     DevLayout &D = D_;
     D.ns = ns; D.A = A; D.NP = NP; D.nch = nc;
@@ -985,8 +993,43 @@ class Engine final : public IEngine {
     D.ph_slot = dph_slot_.as<int2>(); D.hp_slot = dhp_slot_.as<int2>();
     D.ttile = dttile_.as<int2>(); D.nttile = (int)ttile.size();
     D.phtile = dphtile_.as<int2>(); D.nphtile = (int)phtile.size();
-    D.vtile = dvtile_.as<int2>(); D.nvtile = (int)vtile.size();
+    D.vt_off = dvtile_.as<int>(); D.nvtile = vt_off[nc];
     n_ttile_ = D.nttile;
+  }
+
+  // O_.lat and its range when the momenta are one cubic lattice: k_p - k_0 = step (n_p - n_0)
+  // on every axis within rounding, and no difference of two n's outside a signed byte.
+  void build_lattice() {
+    const Basis &B = L_->b;
+    const std::vector<int32_t> *n[3] = {&B.nx, &B.ny, &B.nz};
+    const std::vector<double> *k[3] = {&B.kx, &B.ky, &B.kz};
+    O_.lat = nullptr;
+    O_.step = 0.0;
+    int range[3] = {0, 0, 0}, wide = -1, lo = 0, hi = 0;
+    for (int d = 0; d < 3; ++d) {
+      const auto mm = std::minmax_element(n[d]->begin(), n[d]->end());
+      range[d] = *mm.second - *mm.first;
+      if (range[d] > 127 || *mm.first < -127 || *mm.second > 127) return;
+      if (wide < 0 || range[d] > range[wide]) {
+        wide = d;
+        lo = (int)(mm.first - n[d]->begin());
+        hi = (int)(mm.second - n[d]->begin());
+      }
+    }
+    if (range[wide] > 0) O_.step = ((*k[wide])[hi] - (*k[wide])[lo]) / range[wide];
+    for (int d = 0; d < 3; ++d) {
+      double big = std::fabs(O_.step) * range[d];
+      for (double x : *k[d]) big = std::max(big, std::fabs(x));
+      for (int p = 0; p < B.ns; ++p)
+        if (!(std::fabs(((*k[d])[p] - (*k[d])[0]) - O_.step * ((*n[d])[p] - (*n[d])[0])) <= 1e-15 * big * 8.0)) return;
+    }
+    std::vector<int2> lat(B.ns);
+    for (int p = 0; p < B.ns; ++p)
+      lat[p] = make_int2((B.nx[p] & 255) | (B.ny[p] & 255) << 8 | (B.nz[p] & 255) << 16,
+                         (B.sz[p] > 0 ? 1 : 0) | (B.tz[p] > 0 ? 2 : 0));
+    upload(olat_, lat, &bytes_);
+    O_.lat = olat_.as<int2>();
+    O_.nq2 = range[0] * range[0] + range[1] * range[1] + range[2] * range[2] + 1;
   }
 
   void alloc_state() {
@@ -2592,7 +2635,8 @@ class Engine final : public IEngine {
   DBuf onx_, ony_, onz_, osz_, otz_, okx_, oky_, okz_, oe_;
   // state
   DBuf T_, R_, Vhp_, Vpp_, Vhh_, X_, I9_, Tph_, Rph_, Vph_, W_, I4_, fdiag_, f6_, f7_, d2ij_, d2ab_, i6off_, i7off_;
-  DBuf pairf_;  // per-pair factors of the chiral-like generation
+  DBuf pairf_;  // per-pair factors of the chiral-like generation off a lattice
+  DBuf olat_, lat_;  // orbitals as lattice integers, element tables of the generated potential
   int npp_total_ = 0, nhh_total_ = 0;  // packed pp and hh pairs over all channels
   DBuf okey_, oof_;                    // orbital -> quantum-number slot, slot -> orbital
   int nkeys_ = 0;

@@ -1190,15 +1190,49 @@ template <typename S> void launch_build_vph(const DevLayout &L, const S *Vhp, S 
 // ============================================================================
 
 
-// antisymmetrised element; with pair factors (complex engines, chiral-like kind) the
-// relativity and regulator factors come from the per-pair table instead
-template <typename S>
-__device__ inline S gen_anti(const DevOrbits &O, const DevPotential &P, int p, int q, int r, int s, const double *fpq,
-                             const double *frs) {
-  if constexpr (ScalarOf<S>::complex) {
+// antisymmetrised element: from the lattice tables (LAT), or with pair factors (complex
+// engines, chiral-like kind: the relativity and regulator factors from the per-pair table),
+// or in full
+template <typename S, bool LAT>
+__device__ __forceinline__ S gen_anti(const DevOrbits &O, const DevPotential &P, int p, int q, int r, int s,
+                                      const double *fpq, const double *frs) {
+  if constexpr (!LAT && ScalarOf<S>::complex) {
     if (fpq) return pot::chiral_anti_factored(O, P, p, q, r, s, *fpq, *frs);
   }
-  return pot::vanti<S>(O, P, p, q, r, s);
+  return pot::anti_of<S, LAT>(O, P, p, q, r, s);
+}
+// The element tables of a lattice (pot::lat_anti), one thread per (row, squared integer).
+__global__ void k_lat_tables(DevOrbits O, DevPotential P, int rows, double *T) {
+  const int n = rows * O.nq2;
+  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
+    const int row = x / O.nq2, i2 = x - row * O.nq2;
+    double v = 0.0;
+    if (P.kind != 1) {
+      const int cs = row >> 2, ct = row & 3;
+      const double q2 = (O.step * O.step) * (double)i2;
+      v = pot::minnesota_at(P, q2, pot::class_delta(cs), pot::class_delta(ct), pot::class_dot(cs), pot::class_dot(ct),
+                            O.volume);
+    } else {
+      const double u = 0.5 * O.step * pot::kHbarc, u2 = u * u;  // q = 2 u D, k = u E
+      const double q2 = (4.0 * u2) * (double)i2, k2 = u2 * (double)i2;
+      const double *c = P.lec;
+      const int k = row & 3;
+      if (row < 4) {
+        const double c2 = (1.27 * 1.27) / (4.0 * 92.4 * 92.4);
+        const double ope = -1.0 * c2 / (q2 + 138.0 * 138.0);
+        v = (4.0 * u2) * (ope * pot::class_dot(k) + c[7] * pot::class_delta(k));
+      } else if (row < 8) {
+        v = pot::class_delta(k) * (c[0] + c[2] * q2) + pot::class_dot(k) * (c[1] + c[4] * q2);
+      } else if (row < 12) {
+        v = pot::class_delta(k) * (c[3] * k2) + pot::class_dot(k) * (c[5] * k2);
+      } else {  // sqrt(m (hbar c)^3 / volume) F of a pair, relative momentum u (n_p - n_q)
+        const double mn = pot::pair_mass(row == 12 ? -1 : row == 14 ? 1 : -1, row == 12 ? -1 : 1);
+        const double h3 = pot::kHbarc * pot::kHbarc * pot::kHbarc;
+        v = sqrt(mn * h3 / O.volume) * (exp(-(k2 * k2) * k2 / pot::kLambda6) / sqrt(sqrt(mn * mn + k2)));
+      }
+    }
+    T[x] = v;
+  }
 }
 // F(pq) (chiral_pair_factor) of every packed pp pair, every packed hh pair and every
 // (hole, particle) pair, once per generation: pairf = [pp | hh | hp (A x NP)]
@@ -1212,90 +1246,113 @@ __global__ void k_pair_factors(DevLayout L, DevOrbits O, int npp, int nhh, doubl
     pairf[x] = pot::chiral_pair_factor(O, p, q);
   }
 }
-template <typename S>
+template <typename S, bool LAT>
 __global__ void k_gen_tblocks(DevLayout L, DevOrbits O, DevPotential P, const double *ppf, const double *hhf, S *Vhp) {
   const int2 tl = L.ttile[blockIdx.x];
-  const int ch = tl.x, Pc = L.P[ch], H = L.H[ch];
-  const int64_t n = (int64_t)Pc * H, end = min((int64_t)tl.y + kTileElems, n);
-  for (int64_t e = tl.y + threadIdx.x; e < end; e += blockDim.x) {
-    const int ij = (int)(e / Pc), ab = (int)(e % Pc);  // Vhp'(ij', ab') at ij'*P + ab'
+  const int ch = tl.x, Pc = L.P[ch], n = Pc * L.H[ch];  // < 2^31 per channel
+  const int end = min(tl.y + kTileElems, n);
+  for (int e = tl.y + threadIdx.x; e < end; e += blockDim.x) {
+    const int ij = e / Pc, ab = e - ij * Pc;  // Vhp'(ij', ab') at ij'*P + ab'
     const int hi = L.hh_off[ch] + ij, pi = L.pp_off[ch] + ab;
     const int2 h = L.hh_orb[hi], p = L.pp_orb[pi];
-    Vhp[L.t_off[ch] + e] = gen_anti<S>(O, P, h.x, h.y, p.x, p.y, hhf ? hhf + hi : nullptr, ppf ? ppf + pi : nullptr);
+    Vhp[L.t_off[ch] + e] =
+        gen_anti<S, LAT>(O, P, h.x, h.y, p.x, p.y, hhf ? hhf + hi : nullptr, ppf ? ppf + pi : nullptr);
   }
 }
-// V_pppp' is Hermitian, <cd|V|ab> = conj(<ab|V|cd>): the elements on and above the
-// diagonal are generated and mirrored, which halves the FP64 work of the largest block
-// family.  The elements below the diagonal are written by the thread of their mirror.
-template <typename S>
-__global__ void k_gen_vpp(DevLayout L, DevOrbits O, DevPotential P, const double *ppf, S *Vpp) {
-  const int2 tl = L.vtile[blockIdx.x];
-  const int ch = tl.x, Pc = L.P[ch];
-  const int64_t n = (int64_t)Pc * Pc, end = min((int64_t)tl.y + kTileElems, n);
+// V_pppp' is Hermitian, <cd|V|ab> = conj(<ab|V|cd>): one block per 32 x 32 tile on or above
+// the diagonal generates it and writes it and its mirror image, both along rows (the mirror
+// through shared memory).
+constexpr int kVTile = 32;
+template <typename S, bool LAT>
+__global__ void __launch_bounds__(256) k_gen_vpp(DevLayout L, DevOrbits O, DevPotential P, const double *ppf, S *Vpp) {
+  __shared__ S tile[kVTile][kVTile + 1];
+  int ch = 0;
+  for (int lo = 0, hi = L.nch; hi - lo > 1;) {  // vt_off[ch] <= block < vt_off[ch + 1]
+    const int mid = (lo + hi) >> 1;
+    if (L.vt_off[mid] <= (int)blockIdx.x) lo = mid;
+    else hi = mid;
+    ch = lo;
+  }
+  const int loc = (int)blockIdx.x - L.vt_off[ch];
+  int ct = (int)((sqrtf(8.0f * (float)loc + 1.0f) - 1.0f) * 0.5f);
+  while (ct * (ct + 1) / 2 > loc) --ct;
+  while ((ct + 1) * (ct + 2) / 2 <= loc) ++ct;
+  const int rt = loc - ct * (ct + 1) / 2;
+  const int Pc = L.P[ch], r0 = rt * kVTile, c0 = ct * kVTile;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   S *V = Vpp + L.vpp_off[ch];
-  for (int64_t e = tl.y + threadIdx.x; e < end; e += blockDim.x) {
-    const int r = (int)(e / Pc), c = (int)(e % Pc);
-    if (r > c) continue;
-    const int ri = L.pp_off[ch] + r, ci = L.pp_off[ch] + c;
-    const int2 x = L.pp_orb[ri], y = L.pp_orb[ci];
-    const S v = gen_anti<S>(O, P, x.x, x.y, y.x, y.y, ppf ? ppf + ri : nullptr, ppf ? ppf + ci : nullptr);
-    V[e] = v;
-    if (r != c) V[(int64_t)c * Pc + r] = conj_(v);
+  const int poff = L.pp_off[ch], c = c0 + tx;
+  const int2 y = c < Pc ? L.pp_orb[poff + c] : make_int2(0, 0);
+#pragma unroll
+  for (int j = 0; j < kVTile; j += 8) {
+    const int r = r0 + ty + j;
+    if (c < Pc && r <= c) {
+      const int2 x = L.pp_orb[poff + r];
+      const S v = gen_anti<S, LAT>(O, P, x.x, x.y, y.x, y.y, ppf ? ppf + poff + r : nullptr, ppf ? ppf + poff + c : nullptr);
+      V[(int64_t)r * Pc + c] = v;
+      tile[ty + j][tx] = conj_(v);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kVTile; j += 8) {
+    const int r = c0 + ty + j, k = r0 + tx;  // element (r, k) below the diagonal
+    if (r < Pc && k < r) V[(int64_t)r * Pc + k] = tile[tx][ty + j];
   }
 }
-template <typename S>
+template <typename S, bool LAT>
 __global__ void k_gen_vhh(DevLayout L, DevOrbits O, DevPotential P, S *Vhh) {
   for (int ch = blockIdx.x; ch < L.nch; ch += gridDim.x) {
     const int H = L.H[ch];
     for (int e = threadIdx.x; e < H * H; e += blockDim.x) {
-      const int r = e % H, c = e / H;
+      const int c = e / H, r = e - c * H;
       const int2 x = L.hh_orb[L.hh_off[ch] + r], y = L.hh_orb[L.hh_off[ch] + c];
-      Vhh[L.hh2_off[ch] + e] = pot::vanti<S>(O, P, x.x, x.y, y.x, y.y);
+      Vhh[L.hh2_off[ch] + e] = pot::anti_of<S, LAT>(O, P, x.x, x.y, y.x, y.y);
     }
   }
 }
-template <typename S>
+template <typename S, bool LAT>
 __global__ void k_gen_w(DevLayout L, DevOrbits O, DevPotential P, const double *hpf, S *W) {
   for (int q = blockIdx.x; q < L.nph; q += gridDim.x) {
-    const int nhp = L.n_hp[q];
-    for (int64_t e = threadIdx.x; e < (int64_t)nhp * nhp; e += blockDim.x) {
-      const int r = (int)(e % nhp), c = (int)(e / nhp);
+    const int nhp = L.n_hp[q], n = nhp * nhp;
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+      const int c = e / nhp, r = e - c * nhp;
       const int2 ia = L.hp_orb[L.hp_off[q] + r], jb = L.hp_orb[L.hp_off[q] + c];
       // -<ib|V|ja>_A; pair factors F(ib), F(ja) from the (hole, particle) table
       const double *fib = hpf ? hpf + (int64_t)ia.x * L.NP + (jb.y - L.A) : nullptr;
       const double *fja = hpf ? hpf + (int64_t)jb.x * L.NP + (ia.y - L.A) : nullptr;
-      W[L.i4_off[q] + e] = S(0.0) - gen_anti<S>(O, P, ia.x, jb.y, jb.x, ia.y, fib, fja);
+      W[L.i4_off[q] + e] = S(0.0) - gen_anti<S, LAT>(O, P, ia.x, jb.y, jb.x, ia.y, fib, fja);
     }
   }
 }
 // Fock pieces: f(p,p), f(x, partner) for particles, f(partner, y) for holes;
-// normal_ordered_hamiltonian, ccm_main.f90:1586-1657.  E0 :1661-1684.
-template <typename S>
+// normal_ordered_hamiltonian, ccm_main.f90:1586-1657.  E0 :1661-1684.  One warp per orbital:
+// the lanes take the holes of the sums, reduced in a fixed order (one thread per orbital ran
+// 2 A elements in a row on a few SMs, 5.0 ms at SNM 132 nmax=3).
+template <typename S, bool LAT>
 __global__ void k_gen_fock(DevLayout L, DevOrbits O, DevPotential P, S *fdiag, S *f6, S *f7) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  const int p = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (p >= L.ns) return;
-  S d = S(O.e[p]);
-  for (int h = 0; h < L.A; ++h) d += pot::vanti<S>(O, P, h, p, h, p);
-  fdiag[p] = d;
   const int pb = L.partner[p];
-  if (p >= L.A) {
-    S o = S(0.0);
-    if (pb >= L.A)
-      for (int h = 0; h < L.A; ++h) o += pot::vanti<S>(O, P, h, p, h, pb);
-    f6[p - L.A] = o;
-  } else {
-    S o = S(0.0);
-    if (pb >= 0 && pb < L.A)
-      for (int h = 0; h < L.A; ++h) o += pot::vanti<S>(O, P, h, pb, h, p);
-    f7[p] = o;
+  const bool part = p >= L.A, off = part ? pb >= L.A : pb >= 0 && pb < L.A;
+  S d = S(0.0), o = S(0.0);
+  for (int h = lane; h < L.A; h += 32) {
+    d += pot::anti_of<S, LAT>(O, P, h, p, h, p);
+    if (off) o += part ? pot::anti_of<S, LAT>(O, P, h, p, h, pb) : pot::anti_of<S, LAT>(O, P, h, pb, h, p);
   }
+  d = from2<S>(warp_sum2(to2(d)));
+  o = from2<S>(warp_sum2(to2(o)));
+  if (lane) return;
+  fdiag[p] = S(O.e[p]) + d;
+  if (part) f6[p - L.A] = o;
+  else f7[p] = o;
 }
-template <typename S>
-__global__ void k_gen_e0(DevLayout L, DevOrbits O, DevPotential P, double *e0) {
+template <typename S, bool LAT>
+__global__ void __launch_bounds__(1024) k_gen_e0(DevLayout L, DevOrbits O, DevPotential P, double *e0) {
   double v[2] = {0.0, 0.0};
   for (int x = threadIdx.x; x < L.A * L.A; x += blockDim.x) {
     const int i = x / L.A, j = x % L.A;
-    const S w = pot::vanti<S>(O, P, i, j, i, j);
+    const S w = pot::anti_of<S, LAT>(O, P, i, j, i, j);
     v[0] += 0.5 * real_(w);
     v[1] += 0.5 * imag_(w);
   }
@@ -1303,27 +1360,48 @@ __global__ void k_gen_e0(DevLayout L, DevOrbits O, DevPotential P, double *e0) {
   block_partial<2>(v, e0);
 }
 
+template <typename S, bool LAT>
+void generate_all(const DevLayout &L, const DevOrbits &O, const DevPotential &pot, S *Vhp, S *Vpp, S *Vhh, S *W,
+                  S *fdiag, S *f6, S *f7, double *e0, const double *ppf, const double *hhf, const double *hpf,
+                  cudaStream_t st) {
+  if (L.nttile) k_gen_tblocks<S, LAT><<<L.nttile, 256, 0, st>>>(L, O, pot, ppf, hhf, Vhp);
+  if (L.nvtile) k_gen_vpp<S, LAT><<<L.nvtile, 256, 0, st>>>(L, O, pot, ppf, Vpp);
+  if (L.nch) k_gen_vhh<S, LAT><<<min(L.nch, 4096), 256, 0, st>>>(L, O, pot, Vhh);
+  if (L.nph) k_gen_w<S, LAT><<<min(L.nph, 4096), 256, 0, st>>>(L, O, pot, hpf, W);
+  k_gen_fock<S, LAT><<<(L.ns + 3) / 4, 128, 0, st>>>(L, O, pot, fdiag, f6, f7);
+  k_gen_e0<S, LAT><<<1, 1024, 0, st>>>(L, O, pot, e0);
+}
+
+int lattice_table_doubles(const DevOrbits &O, int kind) {
+  return (kind == 1 ? pot::kLatRowsChiral : pot::kLatRowsMinnesota) * O.nq2;
+}
+void launch_lattice_tables(const DevOrbits &O, const DevPotential &pot, double *lat, cudaStream_t st) {
+  const int rows = pot.kind == 1 ? pot::kLatRowsChiral : pot::kLatRowsMinnesota;
+  k_lat_tables<<<(rows * O.nq2 + 127) / 128, 128, 0, st>>>(O, pot, rows, lat);
+}
+
+// The lattice tables hold for momenta on one cubic lattice, whatever the twist (the layout of
+// ccx_layout_from_basis always; a caller's own orbitals where the engine's check of them
+// passes), and are then the faster form at every size; the elements in full serve the rest.
 template <typename S>
 void launch_generate(const DevLayout &L, const DevOrbits &O, const DevPotential &pot, S *Vhp, S *Vpp, S *Vhh, S *W,
                      S *fdiag, S *f6, S *f7, double *e0, double *pairf, int npp, int nhh, cudaStream_t st) {
+  if (pot.lat) {
+    generate_all<S, true>(L, O, pot, Vhp, Vpp, Vhh, W, fdiag, f6, f7, e0, nullptr, nullptr, nullptr, st);
+    return;
+  }
   const bool factored = ScalarOf<S>::complex && pot.kind == 1 && pairf;
-  double *ppf = factored ? pairf : nullptr, *hhf = factored ? pairf + npp : nullptr;
-  double *hpf = factored ? pairf + npp + nhh : nullptr;
   if (factored) k_pair_factors<<<1216, 256, 0, st>>>(L, O, npp, nhh, pairf);
-  if (L.nttile) k_gen_tblocks<S><<<L.nttile, 256, 0, st>>>(L, O, pot, ppf, hhf, Vhp);
-  if (L.nvtile) k_gen_vpp<S><<<L.nvtile, 256, 0, st>>>(L, O, pot, ppf, Vpp);
-  if (L.nch) k_gen_vhh<S><<<min(L.nch, 4096), 128, 0, st>>>(L, O, pot, Vhh);
-  if (L.nph) k_gen_w<S><<<min(L.nph, 4096), 128, 0, st>>>(L, O, pot, hpf, W);
-  k_gen_fock<S><<<(L.ns + 127) / 128, 128, 0, st>>>(L, O, pot, fdiag, f6, f7);
-  k_gen_e0<S><<<1, 256, 0, st>>>(L, O, pot, e0);
+  generate_all<S, false>(L, O, pot, Vhp, Vpp, Vhh, W, fdiag, f6, f7, e0, factored ? pairf : nullptr,
+                         factored ? pairf + npp : nullptr, factored ? pairf + npp + nhh : nullptr, st);
 }
 
-template <typename S>
+template <typename S, bool LAT>
 __global__ void k_gen_ordered(DevOrbits O, DevPotential P, const int2 *__restrict__ rows, const int2 *__restrict__ cols,
                               int nr, int nc, int swap, double *__restrict__ out) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)nr * nc; e += (int64_t)gridDim.x * blockDim.x) {
     const int2 x = rows[e % nr], y = cols[e / nr];
-    const S v = swap ? pot::vanti<S>(O, P, y.x, y.y, x.x, x.y) : pot::vanti<S>(O, P, x.x, x.y, y.x, y.y);
+    const S v = swap ? pot::anti_of<S, LAT>(O, P, y.x, y.y, x.x, x.y) : pot::anti_of<S, LAT>(O, P, x.x, x.y, y.x, y.y);
     out[2 * e] = real_(v);
     out[2 * e + 1] = imag_(v);
   }
@@ -1331,7 +1409,9 @@ __global__ void k_gen_ordered(DevOrbits O, DevPotential P, const int2 *__restric
 template <typename S>
 void launch_gen_ordered(const DevOrbits &O, const DevPotential &pot, const int2 *rows, const int2 *cols, int nr, int nc,
                         int swap, double *out, cudaStream_t st) {
-  if ((int64_t)nr * nc > 0) k_gen_ordered<S><<<1216, 256, 0, st>>>(O, pot, rows, cols, nr, nc, swap, out);
+  if ((int64_t)nr * nc <= 0) return;
+  if (pot.lat) k_gen_ordered<S, true><<<1216, 256, 0, st>>>(O, pot, rows, cols, nr, nc, swap, out);
+  else k_gen_ordered<S, false><<<1216, 256, 0, st>>>(O, pot, rows, cols, nr, nc, swap, out);
 }
 
 template <typename S>

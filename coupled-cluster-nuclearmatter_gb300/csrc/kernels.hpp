@@ -51,7 +51,12 @@ struct DevPotential {
   int kind;            // 0 Minnesota, 1 chiral-like
   int f32_literals;
   double lec[9];       // CS, CT, C1..C7 (MeV units)
+  const double *lat;   // element tables of a lattice (launch_lattice_tables), or null
 };
+// doubles of the element tables of a potential kind on a lattice (O.nq2 entries each)
+int lattice_table_doubles(const DevOrbits &O, int kind);
+// fills them; every element is then evaluated from its orbitals' integers and the tables
+void launch_lattice_tables(const DevOrbits &O, const DevPotential &pot, double *lat, cudaStream_t st);
 
 // ---- residual pieces --------------------------------------------------------
 template <typename S> void launch_gather_tph(const DevLayout &L, const S *T, S *Tph, cudaStream_t st);

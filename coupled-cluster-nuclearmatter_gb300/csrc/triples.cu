@@ -273,7 +273,7 @@ __global__ void k_finish2(const double *partial, int nb, double *out) {
 
 // generation of the V_hppp / V_hhhp blocks (setup_vnn_hppp_block NN part, ccm_iter.f90:1720-1760;
 // V_hhhp as ccm_iter.f90:885-930): vnn_hppp(kl, ij) = <ij|V|kl>, vnn_hhhp(ij, kd) = <ij|V|kd>
-template <typename S>
+template <typename S, bool LAT>
 __global__ void k_gen_block(DevOrbits O, DevPotential P, const int2 *__restrict__ rows, const int2 *__restrict__ cols,
                             const int64_t *__restrict__ off, const int *__restrict__ nr, const int *__restrict__ nc,
                             const int *__restrict__ roff, const int *__restrict__ coff, int nchan, int rows_are_ket,
@@ -283,7 +283,8 @@ __global__ void k_gen_block(DevOrbits O, DevPotential P, const int2 *__restrict_
     for (int64_t e = threadIdx.x; e < (int64_t)r * c; e += blockDim.x) {
       const int ri = (int)(e % r), ci = (int)(e / r);
       const int2 x = rows[roff[ch] + ri], y = cols[coff[ch] + ci];
-      V[off[ch] + e] = rows_are_ket ? pot::vanti<S>(O, P, y.x, y.y, x.x, x.y) : pot::vanti<S>(O, P, x.x, x.y, y.x, y.y);
+      V[off[ch] + e] =
+          rows_are_ket ? pot::anti_of<S, LAT>(O, P, y.x, y.y, x.x, x.y) : pot::anti_of<S, LAT>(O, P, x.x, x.y, y.x, y.y);
     }
   }
 }
@@ -419,12 +420,16 @@ class Triples final : public ITriples<S> {
   }
   void generate_v(const DevPotential &pot, cudaStream_t st) override {
     const int n5 = (int)off5_h_.size(), n2 = (int)off2_h_.size();
-    if (n5) k_gen_block<S><<<std::min(n5, 8192), 256, 0, st>>>(O_, pot, rows5_.as<int2>(), cols5_.as<int2>(), v5_off_.as<int64_t>(),
-                                                    n5_.as<int>(), nc5_.as<int>(), ro5_.as<int>(), co5_.as<int>(), n5, 1,
-                                                    V5_.as<S>());
-    if (n2) k_gen_block<S><<<std::min(n2, 8192), 256, 0, st>>>(O_, pot, rows2_.as<int2>(), cols2_.as<int2>(), v2_off_.as<int64_t>(),
-                                                    n2_.as<int>(), nc2_.as<int>(), ro2_.as<int>(), co2_.as<int>(), n2, 0,
-                                                    V2_.as<S>());
+    auto gen = [&](auto kernel) {
+      if (n5) kernel<<<std::min(n5, 8192), 256, 0, st>>>(O_, pot, rows5_.as<int2>(), cols5_.as<int2>(), v5_off_.as<int64_t>(),
+                                                         n5_.as<int>(), nc5_.as<int>(), ro5_.as<int>(), co5_.as<int>(), n5,
+                                                         1, V5_.as<S>());
+      if (n2) kernel<<<std::min(n2, 8192), 256, 0, st>>>(O_, pot, rows2_.as<int2>(), cols2_.as<int2>(), v2_off_.as<int64_t>(),
+                                                         n2_.as<int>(), nc2_.as<int>(), ro2_.as<int>(), co2_.as<int>(), n2,
+                                                         0, V2_.as<S>());
+    };
+    if (pot.lat) gen(k_gen_block<S, true>);
+    else gen(k_gen_block<S, false>);
     launches_ += 2;
     tck(cudaGetLastError(), "V_hppp/V_hhhp generation");
     have5_ = have2_ = true;
