@@ -44,6 +44,16 @@ struct DevLayout {
 
 constexpr int kTileElems = 1024;
 
+// The caller's ordered T2 blocks (n_pp x n_hh, one after the other from amp_off), for
+// unpacking: signed packed index + 1 of every ordered pair (0 for a = b), and tiles of
+// kTileElems ordered elements, tile_off[c] of them in the channels before c.
+struct DevOrdered {
+  const int *n_pp, *n_hh;
+  const int64_t *amp_off, *pp_sgn_off, *hh_sgn_off;
+  const int *pp_sgn, *hh_sgn;
+  const int *tile_off;
+};
+
 // Orbital data used by the device potentials.
 struct DevOrbits {
   int ns;

@@ -263,31 +263,51 @@ class Engine final : public IEngine {
 
   // one block; the host buffer is read before the call returns
   void set_vblock(int kind, int ch, const double *v) override {
-    if (double *dv = (kind == 1 || kind == 3 || kind == 6) ? device_view(v) : nullptr) set_vblock_direct(kind, ch, dv);
+    if (double *dv = (kind == 1 || kind == 3 || kind == 6) ? device_view(v) : nullptr) set_vblocks_direct(kind, 1, &ch, &dv);
     else set_vblock_async(kind, ch, v, 0);
     finish_vblocks();
   }
-  // a block in device-addressable host memory, packed in place on the compute stream
-  void set_vblock_direct(int kind, int ch, const double *src) {
+  // blocks in device-addressable host memory, packed in place on the compute stream: one
+  // launch for all of them (a channel given twice starts a new one, so that the last block
+  // given stays the one that counts)
+  void set_vblocks_direct(int kind, int n, const int *chs, double *const *src) {
     const Layout &L = *L_;
-    int rows = 0, target = -1, rp = 0, cp = 0;
-    if (kind == 3 || kind == 6) {
-      check_ch(ch, L.fam[3].count());
-      const auto &pk = L.pk[ch];
-      target = ch;
-      rows = kind == 3 ? pk.n_hh : pk.n_pp;
-      rp = kind == 3 ? pk.H : pk.P;
-      cp = pk.P;
-    } else {
-      check_ch(ch, L.fam[1].count());
-      rows = L.fam[1].side1[ch].size();
-      target = hhhh_to_hhpp_[ch];
-      if (target < 0) return;  // an hhhh channel without an hhpp partner is not used by CCD
-      rp = cp = L.pk[target].H;
-    }
     S *dst = kind == 3 ? Vhp_.as<S>() : kind == 6 ? Vpp_.as<S>() : Vhh_.as<S>();
-    launch_pack_vblock_host<S>(D_, kind, target, rows, rp, cp, src, dst, flag_.as<int>(), st_);
-    ++launches_;
+    std::vector<PackJob> jobs;
+    std::vector<char> seen(L.fam[3].count(), 0);
+    int units = 0;
+    auto flush = [&] {
+      if (!units) return;
+      copyjobs_.alloc(jobs.size() * sizeof(PackJob), &bytes_);
+      CK(cudaMemcpyAsync(copyjobs_.p, jobs.data(), jobs.size() * sizeof(PackJob), cudaMemcpyHostToDevice, st_));
+      launch_pack_jobs<S>(D_, kind, (const PackJob *)copyjobs_.p, (int)jobs.size(), units, dst, flag_.as<int>(), st_);
+      CK(cudaStreamSynchronize(st_));  // the job table on the host is reused or goes out of scope
+      ++launches_;
+      jobs.clear();
+      std::fill(seen.begin(), seen.end(), 0);
+      units = 0;
+    };
+    for (int i = 0; i < n; ++i) {
+      const int ch = chs[i];
+      check_ch(ch, L.fam[kind == 1 ? 1 : 3].count());
+      const int target = kind == 1 ? hhhh_to_hhpp_[ch] : ch;
+      if (target < 0) continue;  // an hhhh channel without an hhpp partner is not used by CCD
+      const auto &pk = L.pk[target];
+      if (seen[target]) flush();
+      seen[target] = 1;
+      PackJob j{};
+      j.src = src[i];
+      j.ch = target;
+      j.n_rows = kind == 3 ? pk.n_hh : kind == 6 ? pk.n_pp : L.fam[1].side1[ch].size();
+      j.rows = kind == 6 ? pk.P : pk.H;
+      j.cols = kind == 1 ? pk.H : pk.P;
+      j.first = units;
+      const int u = pack_units(kind, j.rows, j.cols);
+      if (!u) continue;
+      units += u;
+      jobs.push_back(j);
+    }
+    flush();
     dirty_ = true;
     user_set_ |= 1u << kind;
     ++v_version_;
@@ -296,15 +316,23 @@ class Engine final : public IEngine {
   void set_v4_direct(int n, const int *chs, double *const *src) {
     const Layout &L = *L_;
     adopt_hphp();
-    std::vector<CopyJob> jobs(n);
+    std::vector<CopyJob> jobs;
+    std::vector<int> job_of(L.fam[4].count(), -1);  // a channel given twice: the last block counts
     for (int i = 0; i < n; ++i) {
       check_ch(chs[i], L.fam[4].count());
       const int64_t m = L.fam[4].side1[chs[i]].size();
-      jobs[i] = CopyJob{src[i], v4_.as<double>() + 2 * v4_off_h_[chs[i]], m * m * 2};
+      const CopyJob j{src[i], v4_.as<double>() + 2 * v4_off_h_[chs[i]], m * m * 2};
+      int &at = job_of[chs[i]];
+      if (at >= 0) {
+        jobs[at] = j;
+      } else {
+        at = (int)jobs.size();
+        jobs.push_back(j);
+      }
     }
     copyjobs_.alloc(std::max<size_t>(jobs.size(), 1) * sizeof(CopyJob), &bytes_);
     CK(cudaMemcpyAsync(copyjobs_.p, jobs.data(), jobs.size() * sizeof(CopyJob), cudaMemcpyHostToDevice, st_));
-    launch_copy_jobs((const CopyJob *)copyjobs_.p, n, st_);
+    launch_copy_jobs((const CopyJob *)copyjobs_.p, (int)jobs.size(), st_);
     CK(cudaStreamSynchronize(st_));  // the job table on the host goes out of scope
     ++launches_;
     dirty_ = true;
@@ -326,7 +354,7 @@ class Engine final : public IEngine {
       for (int i = 0; i < n && direct; ++i) direct = (dv[i] = device_view(vs[i])) != nullptr;
       if (direct) {
         if (kind == 4) set_v4_direct(n, chs, dv.data());
-        else for (int i = 0; i < n; ++i) set_vblock_direct(kind, chs[i], dv[i]);
+        else set_vblocks_direct(kind, n, chs, dv.data());
         finish_vblocks();
         return;
       }
@@ -599,9 +627,7 @@ class Engine final : public IEngine {
     const Layout &L = *L_;
     check_ch(ch, L.fam[3].count());
     const auto &P = L.pk[ch];
-    launch_unpack_t<S>(D_, ch, P.n_pp, pp_sgn_.as<int>() + ppsgn_off_[ch], hh_sgn_.as<int>() + hhsgn_off_[ch], P.n_hh,
-                       src, stage_.as<double>(), st_);
-    ++launches_;
+    unpack(ch, ch + 1, src, stage_.as<double>());
     CK(cudaMemcpyAsync(out, stage_.p, (size_t)P.n_pp * P.n_hh * 2 * sizeof(double), cudaMemcpyDeviceToHost, st_));
     CK(cudaStreamSynchronize(st_));
   }
@@ -613,18 +639,35 @@ class Engine final : public IEngine {
   }
   void get_t2_all(double *t) override {
     const Layout &L = *L_;
+    const int nc = L.fam[3].count();
     if (double *dt = device_view(t)) {
-      // device-addressable host memory: every channel unpacked in place, one sync
-      for (int c = 0; c < L.fam[3].count(); ++c) {
-        const auto &P = L.pk[c];
-        launch_unpack_t<S>(D_, c, P.n_pp, pp_sgn_.as<int>() + ppsgn_off_[c], hh_sgn_.as<int>() + hhsgn_off_[c], P.n_hh,
-                           T_.as<S>(), dt + 2 * P.amp_off, st_);
-        ++launches_;
-      }
+      // device-addressable host memory: unpacked in place
+      unpack(0, nc, T_.as<S>(), dt);
       CK(cudaStreamSynchronize(st_));
       return;
     }
-    for (int c = 0; c < L.fam[3].count(); ++c) get_t2(c, t + 2 * L.pk[c].amp_off);
+    // as many channels at a time as the staging buffer holds (always one)
+    const int64_t cap = (int64_t)(stage_.bytes / (2 * sizeof(double)));
+    for (int c = 0; c < nc;) {
+      int e = c;
+      int64_t n = 0;
+      for (; e < nc; ++e) {
+        const int64_t m = (int64_t)L.pk[e].n_pp * L.pk[e].n_hh;
+        if (e > c && n + m > cap) break;
+        n += m;
+      }
+      unpack(c, e, T_.as<S>(), stage_.as<double>());
+      CK(cudaMemcpyAsync(t + 2 * L.pk[c].amp_off, stage_.p, (size_t)n * 2 * sizeof(double), cudaMemcpyDeviceToHost, st_));
+      CK(cudaStreamSynchronize(st_));
+      c = e;
+    }
+  }
+  // packed amplitudes of channels [c0, c1) into ordered blocks from out
+  void unpack(int c0, int c1, const S *src, double *out) {
+    if (c1 <= c0) return;
+    const bool vec = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    launch_unpack_t<S>(D_, DO_, c0, c1, otile_off_[c1] - otile_off_[c0], vec, src, out, st_);
+    ++launches_;
   }
   void get_denominators(double *d2ij, double *d2ab) override {
     const Layout &L = *L_;
@@ -831,7 +874,9 @@ class Engine final : public IEngine {
     std::vector<int> P(nc), H(nc), pp_off(nc), hh_off(nc);
     std::vector<int64_t> t_off(nc), vpp_off(nc), hh2_off(nc);
     std::vector<int2> pp_orb, hh_orb, ttile;
-    std::vector<int> vt_off(nc + 1, 0);
+    std::vector<int> vt_off(nc + 1, 0), onpp, onhh;
+    std::vector<int64_t> oamp;
+    otile_off_.assign(1, 0);
     std::vector<int> pp_row, hh_row, pp_sgn, hh_sgn;
     int64_t vacc = 0, hacc = 0;
     hhhh_to_hhpp_.assign(L.fam[1].count(), -1);
@@ -858,6 +903,10 @@ class Engine final : public IEngine {
       vt_off[c + 1] = vt_off[c] + nvt * (nvt + 1) / 2;
       if (pk.hhhh >= 0) hhhh_to_hhpp_[pk.hhhh] = c;
       max_stage_ = std::max<int64_t>(max_stage_, (int64_t)pk.n_pp * std::max(pk.n_pp, pk.n_hh));
+      onpp.push_back(pk.n_pp);
+      onhh.push_back(pk.n_hh);
+      oamp.push_back(pk.amp_off);
+      otile_off_.push_back(otile_off_.back() + (int)(((int64_t)pk.n_pp * pk.n_hh + kTileElems - 1) / kTileElems));
     }
     n_t_ = L.n_tpacked;
     n_vpp_ = vacc;
@@ -959,6 +1008,10 @@ class Engine final : public IEngine {
     upload(dph_slot_, ph_slot, &bytes_); upload(dhp_slot_, hp_slot, &bytes_);
     upload(dttile_, ttile, &bytes_); upload(dphtile_, phtile, &bytes_); upload(dvtile_, vt_off, &bytes_);
     upload(pp_sgn_, pp_sgn, &bytes_); upload(hh_sgn_, hh_sgn, &bytes_);
+    upload(onpp_, onpp, &bytes_); upload(onhh_, onhh, &bytes_); upload(oamp_, oamp, &bytes_);
+    upload(oppso_, ppsgn_off_, &bytes_); upload(ohhso_, hhsgn_off_, &bytes_); upload(otile_, otile_off_, &bytes_);
+    DO_ = DevOrdered{onpp_.as<int>(), onhh_.as<int>(), oamp_.as<int64_t>(), oppso_.as<int64_t>(), ohhso_.as<int64_t>(),
+                     pp_sgn_.as<int>(), hh_sgn_.as<int>(), otile_.as<int>()};
     upload(n4_, n4, &bytes_); upload(hp4_slot_, hp4_slot, &bytes_);
     std::vector<int64_t> v4off(v4_off_h_.begin(), v4_off_h_.end());
     upload(v4_off_, v4off, &bytes_);
@@ -2623,6 +2676,9 @@ class Engine final : public IEngine {
   int64_t bytes_ = 0, launches_ = 0;
   DevLayout D_{};
   DevOrbits O_{};
+  DevOrdered DO_{};
+  std::vector<int> otile_off_;
+  DBuf onpp_, onhh_, oamp_, oppso_, ohhso_, otile_;
   DevPotential pot_{};
   std::vector<int> partner_, hhhh_to_hhpp_;
   std::vector<int64_t> ppsgn_off_, hhsgn_off_, v4_off_h_;

@@ -103,15 +103,23 @@ void finish(const double *partial, int nb, int nv, double *out, cudaStream_t st)
 
 // An input value (re, im) in the engine's scalar.  Flag bits: 1 a non-zero imaginary
 // part given to a real engine, 2 a NaN or Inf.
+// One 16-byte load where the caller's block is 16-byte aligned (the same branch for a whole
+// block): host memory is read over the link.
+__device__ __forceinline__ double2 load_pair(const double *p) {
+  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) return *reinterpret_cast<const double2 *>(p);
+  return make_double2(p[0], p[1]);
+}
 template <typename S> __device__ inline S cvt_in(const double *p, int *flag);
 template <> __device__ inline double cvt_in<double>(const double *p, int *flag) {
-  if (p[1] != 0.0) atomicOr(flag, 1);
-  if (!isfinite(p[0]) || !isfinite(p[1])) atomicOr(flag, 2);
-  return p[0];
+  const double2 z = load_pair(p);
+  if (z.y != 0.0) atomicOr(flag, 1);
+  if (!isfinite(z.x) || !isfinite(z.y)) atomicOr(flag, 2);
+  return z.x;
 }
 template <> __device__ inline cplx cvt_in<cplx>(const double *p, int *flag) {
-  if (!isfinite(p[0]) || !isfinite(p[1])) atomicOr(flag, 2);
-  return cplx(p[0], p[1]);
+  const double2 z = load_pair(p);
+  if (!isfinite(z.x) || !isfinite(z.y)) atomicOr(flag, 2);
+  return cplx(z.x, z.y);
 }
 
 }  // namespace
@@ -1053,25 +1061,36 @@ void launch_pack_vblock(const DevLayout &L, int kind, int ch, int n_rows, const 
   k_pack_vblock<S><<<1216, 256, 0, st>>>(L, kind, ch, n_rows, stage, dst, flag);
 }
 
-// Kinds 3 and 6 from host memory: dst(r, c) at base + r * P + c (row-major) from the
-// reference block's (row_map[r], col_map[c]) element (column-major, leading dimension
-// n_rows).  A 32 x 32 tile is read down its columns (consecutive source rows, so each
-// host cache line is fetched once) and written along its rows.
+// The job of a unit of work: the last one whose first unit is not after it.
+__device__ __forceinline__ int job_of(const PackJob *__restrict__ jobs, int njobs, int unit) {
+  int lo = 0, hi = njobs;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (jobs[mid].first <= unit) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+// Kind 3 from host memory: dst(r, c) at base + r * P + c (row-major) from the reference
+// block's (row_map[r], col_map[c]) element (column-major, leading dimension n_rows).  A
+// 32 x 32 tile is read down its columns (consecutive source rows, so each host cache line is
+// fetched once) and written along its rows.
 template <typename S>
-__global__ void __launch_bounds__(256) k_pack_vblock_tr(DevLayout L, int kind, int ch, int n_rows, int R, int P,
-                                                        const double *__restrict__ src, S *__restrict__ dst, int *flag) {
+__global__ void __launch_bounds__(256) k_pack_vblock_tr(DevLayout L, const PackJob *__restrict__ jobs, int njobs,
+                                                        S *__restrict__ dst, int *flag) {
   __shared__ S tile[32][33];
-  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+  const PackJob J = jobs[job_of(jobs, njobs, blockIdx.x)];
+  const int ch = J.ch, R = J.rows, P = J.cols, nct = (P + 31) / 32, loc = (int)blockIdx.x - J.first;
+  const int r0 = loc / nct * 32, c0 = loc % nct * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  const int *row_map = kind == 3 ? L.hh_row + L.hh_off[ch] : L.pp_row + L.pp_off[ch];
-  const int *col_map = L.pp_row + L.pp_off[ch];
-  const int64_t base = kind == 3 ? L.t_off[ch] : L.vpp_off[ch];
+  const int *row_map = L.hh_row + L.hh_off[ch], *col_map = L.pp_row + L.pp_off[ch];
+  const int64_t base = L.t_off[ch];
   const int r = r0 + tx;
   const int64_t srow = r < R ? row_map[r] : 0;
 #pragma unroll
   for (int j = 0; j < 32; j += 8) {
     const int c = c0 + ty + j;
-    if (r < R && c < P) tile[ty + j][tx] = cvt_in<S>(src + 2 * (srow + (int64_t)n_rows * col_map[c]), flag);
+    if (r < R && c < P) tile[ty + j][tx] = cvt_in<S>(J.src + 2 * (srow + (int64_t)J.n_rows * col_map[c]), flag);
   }
   __syncthreads();
 #pragma unroll
@@ -1088,29 +1107,42 @@ __global__ void __launch_bounds__(256) k_pack_vblock_tr(DevLayout L, int kind, i
 // block (the tile kernel above) reach a fraction of the link rate on a family of tens of
 // GB.
 template <typename S>
-__global__ void __launch_bounds__(512) k_pack_vpp_cols(DevLayout L, int ch, int n_rows, int P,
-                                                       const double *__restrict__ src, S *__restrict__ dst, int *flag) {
-  const int *row_map = L.pp_row + L.pp_off[ch];
-  const int *col_map = L.pp_row + L.pp_off[ch];
-  const int64_t base = L.vpp_off[ch];
-  for (int c = blockIdx.x; c < P; c += gridDim.x) {
-    const double *col = src + 2 * (int64_t)n_rows * col_map[c];
-    for (int r = threadIdx.x; r < P; r += blockDim.x) dst[base + (int64_t)r * P + c] = cvt_in<S>(col + 2 * row_map[r], flag);
+__global__ void __launch_bounds__(512) k_pack_vpp_cols(DevLayout L, const PackJob *__restrict__ jobs, int njobs, int ncols,
+                                                       S *__restrict__ dst, int *flag) {
+  for (int u = blockIdx.x; u < ncols; u += gridDim.x) {
+    const PackJob J = jobs[job_of(jobs, njobs, u)];
+    const int P = J.cols, c = u - J.first;
+    const int *map = L.pp_row + L.pp_off[J.ch];
+    const int64_t base = L.vpp_off[J.ch];
+    const double *col = J.src + 2 * (int64_t)J.n_rows * map[c];
+    for (int r = threadIdx.x; r < P; r += blockDim.x) dst[base + (int64_t)r * P + c] = cvt_in<S>(col + 2 * map[r], flag);
   }
 }
+// Kind 1 from host memory: consecutive packed rows are consecutive source rows already
 template <typename S>
-void launch_pack_vblock_host(const DevLayout &L, int kind, int ch, int n_rows, int rows_packed, int cols_packed,
-                             const double *src, S *dst, int *flag, cudaStream_t st) {
-  if (rows_packed <= 0 || cols_packed <= 0) return;
-  if (kind == 6) {
-    k_pack_vpp_cols<S><<<std::min(cols_packed, 304), 512, 0, st>>>(L, ch, n_rows, cols_packed, src, dst, flag);
-  } else if (kind == 3) {
-    const dim3 grid((cols_packed + 31) / 32, (rows_packed + 31) / 32);
-    k_pack_vblock_tr<S><<<grid, dim3(32, 8), 0, st>>>(L, kind, ch, n_rows, rows_packed, cols_packed, src, dst, flag);
-  } else {
-    // kind 1 reads consecutive source rows already
-    k_pack_vblock<S><<<1216, 256, 0, st>>>(L, kind, ch, n_rows, src, dst, flag);
+__global__ void __launch_bounds__(256) k_pack_vhh_jobs(DevLayout L, const PackJob *__restrict__ jobs, int njobs,
+                                                       S *__restrict__ dst, int *flag) {
+  const PackJob J = jobs[job_of(jobs, njobs, blockIdx.x)];
+  const int H = J.rows, *map = L.hh_row + L.hh_off[J.ch];
+  const int beg = ((int)blockIdx.x - J.first) * kTileElems, end = min(beg + kTileElems, H * H);
+  for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
+    const int c = e / H, r = e - c * H;
+    dst[L.hh2_off[J.ch] + e] = cvt_in<S>(J.src + 2 * (map[r] + (int64_t)J.n_rows * map[c]), flag);
   }
+}
+int pack_units(int kind, int rows, int cols) {
+  if (rows <= 0 || cols <= 0) return 0;
+  if (kind == 6) return cols;
+  if (kind == 3) return (rows + 31) / 32 * ((cols + 31) / 32);
+  return (rows * cols + kTileElems - 1) / kTileElems;
+}
+template <typename S>
+void launch_pack_jobs(const DevLayout &L, int kind, const PackJob *jobs, int njobs, int units, S *dst, int *flag,
+                      cudaStream_t st) {
+  if (units <= 0) return;
+  if (kind == 6) k_pack_vpp_cols<S><<<std::min(units, 304), 512, 0, st>>>(L, jobs, njobs, units, dst, flag);
+  else if (kind == 3) k_pack_vblock_tr<S><<<units, dim3(32, 8), 0, st>>>(L, jobs, njobs, dst, flag);
+  else k_pack_vhh_jobs<S><<<units, 256, 0, st>>>(L, jobs, njobs, dst, flag);
 }
 
 // one CTA per job; 16-byte copies where both ends and the length allow
@@ -1514,23 +1546,46 @@ __global__ void k_pack_t(DevLayout L, int ch, int n_pp, const double *__restrict
 template <typename S> void launch_pack_t(const DevLayout &L, int ch, int n_pp, const double *stage, S *T, int *flag, cudaStream_t st) {
   k_pack_t<S><<<608, 256, 0, st>>>(L, ch, n_pp, stage, T, flag);
 }
-template <typename S>
-__global__ void k_unpack_t(DevLayout L, int ch, int n_pp, const int *__restrict__ pp_signed, const int *__restrict__ hh_signed,
-                            int n_hh, const S *__restrict__ T, double *stage) {
-  const int P = L.P[ch];
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n_pp * n_hh; e += (int64_t)gridDim.x * blockDim.x) {
-    const int r = (int)(e % n_pp), c = (int)(e / n_pp);
-    const int sp = pp_signed[r], sh = hh_signed[c];
+// One launch for all channels asked for: a launch a channel costs more than its copy (185
+// of them took 1.3 ms for the 129 MB of PNM 66 nmax=4, 0.62 ms in one).  An element is one
+// 16-byte store where the output allows: host memory is written over the link as the stores
+// come, and two 8-byte stores each fill half of what a line could hold.
+template <typename S, bool VEC>
+__global__ void __launch_bounds__(256) k_unpack_t(DevLayout L, DevOrdered O, int c0, int c1, const S *__restrict__ T,
+                                                  double *__restrict__ out) {
+  const int unit = (int)blockIdx.x + O.tile_off[c0];
+  int lo = c0, hi = c1;
+  while (hi - lo > 1) {  // tile_off[lo] <= unit < tile_off[lo + 1]
+    const int mid = (lo + hi) >> 1;
+    if (O.tile_off[mid] <= unit) lo = mid;
+    else hi = mid;
+  }
+  const int ch = lo, npp = O.n_pp[ch], P = L.P[ch];
+  const int64_t beg = (int64_t)(unit - O.tile_off[ch]) * kTileElems, n = (int64_t)npp * O.n_hh[ch];
+  const int cnt = (int)min((int64_t)kTileElems, n - beg);
+  const int cb = (int)(beg / npp), rb = (int)(beg - (int64_t)cb * npp);
+  const int *ps = O.pp_sgn + O.pp_sgn_off[ch], *hs = O.hh_sgn + O.hh_sgn_off[ch];
+  const S *Tc = T + L.t_off[ch];
+  double *o = out + 2 * (O.amp_off[ch] - O.amp_off[c0] + beg);
+  for (int x = threadIdx.x; x < cnt; x += blockDim.x) {
+    const int y = rb + x, dc = y / npp;
+    const int sp = ps[y - dc * npp], sh = hs[cb + dc];
     S v = S(0.0);
-    if (sp && sh) v = (ssign(sp) * ssign(sh)) * T[L.t_off[ch] + sidx(sp) + (int64_t)P * sidx(sh)];
-    stage[2 * e] = real_(v);
-    stage[2 * e + 1] = imag_(v);
+    if (sp && sh) v = (ssign(sp) * ssign(sh)) * Tc[sidx(sp) + (int64_t)P * sidx(sh)];
+    if constexpr (VEC) {
+      reinterpret_cast<double2 *>(o)[x] = to2(v);
+    } else {
+      o[2 * x] = real_(v);
+      o[2 * x + 1] = imag_(v);
+    }
   }
 }
 template <typename S>
-void launch_unpack_t(const DevLayout &L, int ch, int n_pp, const int *pp_signed, const int *hh_signed, int n_hh, const S *T,
-                     double *stage, cudaStream_t st) {
-  k_unpack_t<S><<<608, 256, 0, st>>>(L, ch, n_pp, pp_signed, hh_signed, n_hh, T, stage);
+void launch_unpack_t(const DevLayout &L, const DevOrdered &O, int c0, int c1, int ntiles, bool vec, const S *T, double *out,
+                     cudaStream_t st) {
+  if (ntiles <= 0) return;
+  if (vec) k_unpack_t<S, true><<<ntiles, 256, 0, st>>>(L, O, c0, c1, T, out);
+  else k_unpack_t<S, false><<<ntiles, 256, 0, st>>>(L, O, c0, c1, T, out);
 }
 
 // ---- explicit instantiations -------------------------------------------------
@@ -1559,8 +1614,7 @@ void launch_unpack_t(const DevLayout &L, int ch, int n_pp, const int *pp_signed,
   template void launch_diis_gram<S>(int64_t, const S *const *, int, double *, double *, cudaStream_t);                \
   template void launch_combine<S>(int64_t, const S *const *, const double *, int, S *, cudaStream_t);                 \
   template void launch_pack_vblock<S>(const DevLayout &, int, int, int, const double *, S *, int *, cudaStream_t);    \
-  template void launch_pack_vblock_host<S>(const DevLayout &, int, int, int, int, int, const double *, S *, int *,      \
-                                           cudaStream_t);                                                              \
+  template void launch_pack_jobs<S>(const DevLayout &, int, const PackJob *, int, int, S *, int *, cudaStream_t);       \
   template void launch_build_w<S>(const DevLayout &, const int2 *, const int64_t *, const int *, const double *, S *,  \
                                   int *, cudaStream_t);                                                                \
   template void launch_build_vph<S>(const DevLayout &, const S *, S *, cudaStream_t);                                 \
@@ -1573,7 +1627,7 @@ void launch_unpack_t(const DevLayout &L, int ch, int n_pp, const int *pp_signed,
                                       int, double *, cudaStream_t);                                                    \
   template void launch_unpack_vblock<S>(const DevLayout &, int, int, int, int, const int *, const int *, const S *,  \
                                         double *, cudaStream_t);                                                       \
-  template void launch_unpack_t<S>(const DevLayout &, int, int, const int *, const int *, int, const S *, double *,   \
+  template void launch_unpack_t<S>(const DevLayout &, const DevOrdered &, int, int, int, bool, const S *, double *,     \
                                    cudaStream_t);
 
 CCX_INST(double)

@@ -129,13 +129,21 @@ void launch_combine(int64_t n, const S *const *xs, const double *coef /* host, 2
 // ---- interaction -----------------------------------------------------------
 template <typename S>
 void launch_pack_vblock(const DevLayout &L, int kind, int ch, int n_rows, const double *stage, S *dst, int *flag, cudaStream_t st);
-// The same packing read straight from host memory the device can address (pinned and
-// mapped): reads follow the block's column-major order (consecutive rows), through a
-// shared-memory transpose where the packed layout is row-major (kinds 3 and 6).
-// rows_packed / cols_packed: the channel's packed extents (kind 3: H, P; 6: P, P; 1: H, H).
+// The same packing of many blocks of one kind in one launch, read straight from host
+// memory the device can address (pinned and mapped): reads follow each block's
+// column-major order (consecutive rows), through a shared-memory transpose where the packed
+// layout is row-major (kind 3).  first: units of work (pack_units) in the jobs before this
+// one; a channel occurs once in a list.
+struct PackJob {
+  const double *src;
+  int ch, n_rows;
+  int rows, cols;  // packed extents (kind 3: H, P; 6: P, P; 1: H, H)
+  int first;
+};
+int pack_units(int kind, int rows, int cols);
 template <typename S>
-void launch_pack_vblock_host(const DevLayout &L, int kind, int ch, int n_rows, int rows_packed, int cols_packed,
-                             const double *src, S *dst, int *flag, cudaStream_t st);
+void launch_pack_jobs(const DevLayout &L, int kind, const PackJob *jobs, int njobs, int units, S *dst, int *flag,
+                      cudaStream_t st);
 // Copies of many blocks in one launch (n doubles from src to dst per job); src may be
 // mapped host memory.
 struct CopyJob {
@@ -166,8 +174,10 @@ double measure_fp64_peak(int device);
 template <typename S> void launch_axpy(int64_t n, const S *x, S *y, cudaStream_t st);
 template <typename S> void launch_mp2(const DevLayout &L, const S *Vhp, const S *fdiag, S *T, cudaStream_t st);
 template <typename S> void launch_pack_t(const DevLayout &L, int ch, int n_pp, const double *stage, S *T, int *flag, cudaStream_t st);
+// the packed amplitudes of channels [c0, c1) into their ordered blocks, one after the other
+// from out (ntiles: their tiles); vec: out is 16-byte aligned
 template <typename S>
-void launch_unpack_t(const DevLayout &L, int ch, int n_pp, const int *pp_signed, const int *hh_signed, int n_hh, const S *T,
-                     double *stage, cudaStream_t st);
+void launch_unpack_t(const DevLayout &L, const DevOrdered &O, int c0, int c1, int ntiles, bool vec, const S *T, double *out,
+                     cudaStream_t st);
 
 }  // namespace ccx
