@@ -1121,10 +1121,10 @@ class Engine final : public IEngine {
     build_gemm_plans();
   }
 
-  // A grouped GEMM launch plan: problems, tile lists per tile shape, split-K problems.
+  // A grouped GEMM launch plan: problems and the warp tiles of both shapes.
   struct Plan {
-    DBuf probs, tiles[2], splits;
-    int ntiles[2] = {0, 0}, nsplit = 0;
+    DBuf probs, tiles;
+    int n8 = 0, n4 = 0;
   };
   // N buckets of the tile-shape choice: N <= 16, <= 32, <= 64, > 64
   static int n_bucket(int N) { return N <= 16 ? 0 : N <= 32 ? 1 : N <= 64 ? 2 : 3; }
@@ -1132,52 +1132,50 @@ class Engine final : public IEngine {
     const int *shape_of = nullptr;  // tile shape per N bucket
     int only_bucket = -1;           // >= 0: keep only the problems of this bucket
     std::vector<GemmProb<S>> probs;
-    std::vector<GemmTile> tiles[2];
-    std::vector<int> splits;
-    std::vector<int64_t> work;
-    void add(GemmProb<S> p, int64_t w) {
-      if (only_bucket >= 0 && n_bucket(p.N) != only_bucket) return;
-      const int shape = shape_of ? shape_of[n_bucket(p.N)] : (p.N <= 32 ? kShape128x32 : kShape64x64);
-      const int bm = gemm_bm(shape), bn = gemm_bn(shape);
-      const int id = (int)probs.size();
-      const int nsl = p.kchunk > 0 ? (p.seg[0].K + p.kchunk - 1) / p.kchunk : 1;
-      for (int ks = 0; ks < nsl; ++ks)
-        for (int m0 = 0; m0 < p.M; m0 += bm)
-          for (int n0 = 0; n0 < p.N; n0 += bn) tiles[shape].push_back(GemmTile{id, m0, n0, ks});
-      if (p.kchunk > 0) splits.push_back(id);
+    void add(const GemmProb<S> &p) {
+      if (p.M <= 0 || p.N <= 0 || (only_bucket >= 0 && n_bucket(p.N) != only_bucket)) return;
       probs.push_back(p);
-      work.push_back(p.kchunk > 0 ? w / nsl : w);
     }
   };
-  void finalize_plan(Plan &pl, PlanBuilder &b) {
-    // largest problems first for load balance across the SMs
+  // The tiles of a plan, longest first, so that the last ones to finish are short.  Lists
+  // beyond kGemmItems tiles give a warp several row tiles, which a list that long does not
+  // need for balance.
+  static constexpr int kGemmItems = 1 << 15;
+  void finalize_plan(Plan &pl, const PlanBuilder &b) {
+    auto rows = [](const GemmProb<S> &p, int sh) { return (p.M + gemm_rows(sh) - 1) / gemm_rows(sh); };
+    auto cols = [](const GemmProb<S> &p) { return (p.N + kGemmCols - 1) / kGemmCols; };
+    int64_t all8 = 0;
+    for (const auto &p : b.probs) all8 += (int64_t)rows(p, kShape8) * cols(p);
+    const int nm = (int)std::min<int64_t>(64, 1 + all8 / kGemmItems);
+    std::vector<int> order[2];
+    for (int i = 0; i < (int)b.probs.size(); ++i) order[b.shape_of[n_bucket(b.probs[i].N)]].push_back(i);
+    std::vector<GemmTile> tiles;
     for (int sh = 0; sh < 2; ++sh) {
-      std::stable_sort(b.tiles[sh].begin(), b.tiles[sh].end(),
-                       [&](const GemmTile &x, const GemmTile &y) { return b.work[x.prob] > b.work[y.prob]; });
-      upload(pl.tiles[sh], b.tiles[sh], &bytes_);
-      pl.ntiles[sh] = (int)b.tiles[sh].size();
+      auto steps = [&](int i) {  // K steps of a tile
+        int k = 0;
+        for (int s = 0; s < b.probs[i].nseg; ++s) k += b.probs[i].seg[s].K;
+        return k;
+      };
+      std::stable_sort(order[sh].begin(), order[sh].end(), [&](int x, int y) { return steps(x) > steps(y); });
+      for (int i : order[sh]) {
+        const GemmProb<S> &p = b.probs[i];
+        const int nc = cols(p), step = gemm_rows(sh) * nm;
+        for (int m0 = 0; m0 < p.M; m0 += step)
+          for (int c = 0; c < nc; ++c) {
+            const int n0 = (int)((int64_t)p.N * c / nc), n1 = (int)((int64_t)p.N * (c + 1) / nc);
+            const int left = (p.M - m0 + gemm_rows(sh) - 1) / gemm_rows(sh);
+            tiles.push_back(GemmTile{i, m0, n0, (int16_t)(n1 - n0), (int16_t)std::min(nm, left)});
+          }
+      }
+      (sh ? pl.n4 : pl.n8) = (int)tiles.size() - (sh ? pl.n8 : 0);
     }
     upload(pl.probs, b.probs, &bytes_);
-    upload(pl.splits, b.splits, &bytes_);
-    pl.nsplit = (int)b.splits.size();
+    upload(pl.tiles, tiles, &bytes_);
   }
   void run_plan(const Plan &pl, cudaStream_t s = nullptr) {
-    if (!s) s = st_;
-    const GemmProb<S> *pr = (const GemmProb<S> *)pl.probs.p;
-    for (int sh = 0; sh < 2; ++sh)
-      if (pl.ntiles[sh]) {
-        launch_gemm<S>(sh, pr, (const GemmTile *)pl.tiles[sh].p, pl.ntiles[sh], s);
-        ++launches_;
-      }
-    if (pl.nsplit) {
-      launch_splitk_reduce<S>(pr, (const int *)pl.splits.p, pl.nsplit, s);
-      ++launches_;
-    }
-  }
-  void run_x(cudaStream_t s = nullptr) {
-    launch_xdot<S>(D_, (const int4 *)xwork_.p, nxwork_, (const int4 *)xgroups_.p, nxgroups_, Vhp_.as<S>(), T_.as<S>(),
-                   xpart_.as<S>(), X_.as<S>(), s ? s : st_);
-    launches_ += 2;
+    if (pl.n8 + pl.n4 <= 0) return;
+    launch_gemm<S>((const GemmProb<S> *)pl.probs.p, (const GemmTile *)pl.tiles.p, pl.n8, pl.n4, s ? s : st_);
+    ++launches_;
   }
   void build_gemm_plans() {
     const Layout &L = *L_;
@@ -1191,110 +1189,97 @@ class Engine final : public IEngine {
       ni6rows_ = (int)rt.size();
       i6dots_.alloc((size_t)std::max<int64_t>(3 * n_t_, 1) * sizeof(S), &bytes_);
     }
-    {  // X = V_hhpp' T'  (H x H, K = P): column-dot items of at most kXSlice K each,
-       // longest first; their partial tiles are summed per X tile in slice order
-      std::vector<int4> w, gr;
-      std::vector<int> klen;
-      int slot = 0;
-      for (int c = 0; c < nc; ++c) {
-        const auto &pk = L.pk[c];
-        if (pk.H <= 0 || pk.P <= 0) continue;
-        const int nsl = (pk.P + kXSlice - 1) / kXSlice;
-        for (int m0 = 0; m0 < pk.H; m0 += kXM)
-          for (int j0 = 0; j0 < pk.H; j0 += kXJ) {
-            gr.push_back(make_int4(c, m0 | (j0 << 16), slot, nsl));
-            for (int ks = 0; ks < nsl; ++ks) {
-              w.push_back(make_int4(c, m0 | (j0 << 16), ks, slot++));
-              klen.push_back(std::min(pk.P, (ks + 1) * kXSlice) - ks * kXSlice);
-            }
-          }
-      }
-      std::vector<int> ord(w.size());
-      for (size_t i = 0; i < ord.size(); ++i) ord[i] = (int)i;
-      std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return klen[x] > klen[y]; });
-      std::vector<int4> ws(w.size());
-      for (size_t i = 0; i < ord.size(); ++i) ws[i] = w[ord[i]];
-      upload(xwork_, ws, &bytes_);
-      upload(xgroups_, gr, &bytes_);
-      nxwork_ = (int)ws.size();
-      nxgroups_ = (int)gr.size();
-      xpart_.alloc((size_t)std::max(slot, 1) * kXM * kXJ * sizeof(S), &bytes_);
-    }
-    build_fp64_plans(planLadder_, planI4_, planRing_, -1, nullptr);
+    build_fp64_plans(fp64_, -1, nullptr);
   }
   // The grouped FP64 GEMM plans of the residual; bucket >= 0 keeps only the problems of
-  // that N bucket, shapes overrides the engine's tile shape per bucket.
-  void build_fp64_plans(Plan &ladder, Plan &i4, Plan &ring, int bucket, const int *shapes) {
+  // that N bucket, shapes overrides the engine's tile shape per bucket.  The products of a
+  // residual run in two launches, X with I4 and the ring with the ladders, whose tiles fill
+  // each other's tails (the products apart, for the per-term timers, in four).
+  struct Fp64Plans {
+    Plan x, i4, ring, ladder, x_i4, ring_ladder;
+  };
+  void build_fp64_plans(Fp64Plans &P, int bucket, const int *shapes) {
     ++plan_epoch_;
     const Layout &L = *L_;
     const int nc = L.fam[3].count();
-    {  // R' += V_pppp' T' + T' I9'
-      PlanBuilder b;
-      b.shape_of = shapes ? shapes : gemm_shape_;
-      b.only_bucket = bucket;
-      int64_t hoff = 0, voff = 0;
-      for (int c = 0; c < nc; ++c) {
-        const auto &pk = L.pk[c];
-        if (pk.H > 0 && pk.P > 0) {
-          GemmProb<S> p{};
-          p.nseg = 2;
-          p.M = pk.P; p.N = pk.H;
-          p.seg[0] = GemmSeg<S>{Vpp_.as<S>() + voff, T_.as<S>() + pk.t_off, pk.P, 1, 1, pk.P, pk.P, 1.0};
-          p.seg[1] = GemmSeg<S>{T_.as<S>() + pk.t_off, I9_.as<S>() + hoff, 1, pk.P, 1, pk.H, pk.H, 1.0};
-          p.C = R_.as<S>() + pk.t_off; p.C0 = nullptr; p.sCm = 1; p.sCn = pk.P; p.accumulate = 1;
-          b.add(p, (int64_t)pk.P * pk.H * (pk.P + pk.H));
-        }
-        hoff += (int64_t)pk.H * pk.H;
-        voff += (int64_t)pk.P * pk.P;
-      }
-      finalize_plan(ladder, b);
+    PlanBuilder bx, bl, b4, br, bx4, brl;
+    for (PlanBuilder *b : {&bx, &bl, &b4, &br, &bx4, &brl}) {
+      b->shape_of = shapes ? shapes : gemm_shape_;
+      b->only_bucket = bucket;
     }
-    {  // I4 = W + 1/2 V_ph T_ph ; R_ph = T_ph I4
-      PlanBuilder b4, br;
-      b4.shape_of = br.shape_of = shapes ? shapes : gemm_shape_;
-      b4.only_bucket = br.only_bucket = bucket;
-      int64_t toff = 0, ioff = 0;
-      for (int q = 0; q < L.ph[1].count(); ++q) {
-        const int nph = L.ph[1].side1[q].size(), nhp = L.ph[1].side2[q].size();
-        if (nph > 0 && nhp > 0) {
-          GemmProb<S> a{};
-          a.nseg = 1;
-          a.M = nhp; a.N = nhp;
-          a.seg[0] = GemmSeg<S>{Vph_.as<S>() + toff, Tph_.as<S>() + toff, 1, nhp, 1, nph, nph, 0.5};
-          a.C = I4_.as<S>() + ioff; a.C0 = W_.as<S>() + ioff; a.sCm = 1; a.sCn = nhp; a.accumulate = 0;
-          b4.add(a, (int64_t)nhp * nhp * nph);
-          GemmProb<S> r{};
-          r.nseg = 1;
-          r.M = nph; r.N = nhp;
-          r.seg[0] = GemmSeg<S>{Tph_.as<S>() + toff, I4_.as<S>() + ioff, 1, nph, 1, nhp, nhp, 1.0};
-          r.C = Rph_.as<S>() + toff; r.C0 = nullptr; r.sCm = 1; r.sCn = nph; r.accumulate = 0;
-          br.add(r, (int64_t)nph * nhp * nhp);
-        }
-        toff += (int64_t)nph * nhp;
-        ioff += (int64_t)nhp * nhp;
+    int64_t hoff = 0, voff = 0;
+    for (int c = 0; c < nc; ++c) {
+      const auto &pk = L.pk[c];
+      if (pk.H > 0 && pk.P > 0) {
+        // R' = V_pppp' T' + T' I9'
+        GemmProb<S> p{};
+        p.nseg = 2;
+        p.M = pk.P; p.N = pk.H; p.alpha = 1.0;
+        p.seg[0] = GemmSeg<S>{Vpp_.as<S>() + voff, T_.as<S>() + pk.t_off, pk.P, 1, 1, pk.P, pk.P};
+        p.seg[1] = GemmSeg<S>{T_.as<S>() + pk.t_off, I9_.as<S>() + hoff, 1, pk.P, 1, pk.H, pk.H};
+        p.C = R_.as<S>() + pk.t_off; p.sCm = 1; p.sCn = pk.P;
+        bl.add(p);
+        brl.add(p);
+        // X(kl, ij) = sum_cd V_hhpp'(cd, kl) T'(cd, ij)
+        GemmProb<S> x{};
+        x.nseg = 1;
+        x.M = pk.H; x.N = pk.H; x.alpha = 1.0;
+        x.seg[0] = GemmSeg<S>{Vhp_.as<S>() + pk.t_off, T_.as<S>() + pk.t_off, pk.P, 1, 1, pk.P, pk.P};
+        x.C = X_.as<S>() + hoff; x.sCm = 1; x.sCn = pk.H;
+        bx.add(x);
+        bx4.add(x);
       }
-      finalize_plan(i4, b4);
-      finalize_plan(ring, br);
+      hoff += (int64_t)pk.H * pk.H;
+      voff += (int64_t)pk.P * pk.P;
     }
+    // I4 = W + 1/2 V_ph T_ph ; R_ph = T_ph I4
+    int64_t toff = 0, ioff = 0;
+    for (int q = 0; q < L.ph[1].count(); ++q) {
+      const int nph = L.ph[1].side1[q].size(), nhp = L.ph[1].side2[q].size();
+      if (nph > 0 && nhp > 0) {
+        GemmProb<S> a{};
+        a.nseg = 1;
+        a.M = nhp; a.N = nhp; a.alpha = 0.5;
+        a.seg[0] = GemmSeg<S>{Vph_.as<S>() + toff, Tph_.as<S>() + toff, 1, nhp, 1, nph, nph};
+        a.C = I4_.as<S>() + ioff; a.C0 = W_.as<S>() + ioff; a.sCm = 1; a.sCn = nhp;
+        b4.add(a);
+        bx4.add(a);
+        GemmProb<S> r{};
+        r.nseg = 1;
+        r.M = nph; r.N = nhp; r.alpha = 1.0;
+        r.seg[0] = GemmSeg<S>{Tph_.as<S>() + toff, I4_.as<S>() + ioff, 1, nph, 1, nhp, nhp};
+        r.C = Rph_.as<S>() + toff; r.sCm = 1; r.sCn = nph;
+        br.add(r);
+        brl.add(r);
+      }
+      toff += (int64_t)nph * nhp;
+      ioff += (int64_t)nhp * nhp;
+    }
+    finalize_plan(P.x, bx);
+    finalize_plan(P.i4, b4);
+    finalize_plan(P.ring, br);
+    finalize_plan(P.ladder, bl);
+    finalize_plan(P.x_i4, bx4);
+    finalize_plan(P.ring_ladder, brl);
   }
 
-  // Autotuner of the grouped FP64 GEMM: for each N bucket, time the residual's ladder,
-  // I4 and ring problems of that bucket with each tile shape (best of 3 launches, CUDA
-  // events on the engine stream), keep the faster shape and rebuild every plan.  The
-  // timed launches only write buffers that each residual evaluation rewrites.
+  // Autotuner of the grouped FP64 GEMM: for each N bucket, time the residual's two product
+  // launches on the problems of that bucket with each tile shape (best of 3, CUDA events on
+  // the engine stream), keep the faster shape and rebuild every plan.  The timed launches
+  // only write buffers that each residual evaluation rewrites.
   void autotune(int shapes[4], double ms[8]) override {
     require_ready();
     EventPair ev;
     const int64_t held = bytes_;  // the trial plans are freed again below
     for (int k = 0; k < 4; ++k) {
       double best = 1e300;
-      int pick = gemm_shape_[k];
+      int pick = kShape8;
       for (int sh = 0; sh < 2; ++sh) {
         const int tab[4] = {sh, sh, sh, sh};
-        Plan pl, p4, pr;
-        build_fp64_plans(pl, p4, pr, k, tab);
+        Fp64Plans P;
+        build_fp64_plans(P, k, tab);
         double t = 0.0;
-        for (const Plan *p : {&pl, &p4, &pr}) {
+        for (const Plan *p : {&P.x_i4, &P.ring_ladder}) {
           float tbest = 1e30f;
           for (int rep = 0; rep < 3; ++rep) tbest = std::min(tbest, ev.time(st_, [&] { run_plan(*p); }));
           t += tbest;
@@ -1306,7 +1291,7 @@ class Engine final : public IEngine {
       shapes[k] = pick;
     }
     bytes_ = held;
-    build_fp64_plans(planLadder_, planI4_, planRing_, -1, nullptr);
+    build_fp64_plans(fp64_, -1, nullptr);
     mixed_ready_ = false;  // the mixed residual's FP64 plans are rebuilt with the new shapes
     oz_ready_ = false;
   }
@@ -1408,11 +1393,12 @@ class Engine final : public IEngine {
     CK(cudaStreamWaitEvent(st_, xev_[ev], 0));
   }
   void residual(bool /*unused*/) {
+    const bool apart = timing_;  // one launch per product, for its own timer
     mark(0);
     launch_gather_tph<S>(D_, T_.as<S>(), Tph_.as<S>(), st_);
     mark(1);
     kbegin(kKX);
-    run_x();
+    run_plan(apart ? fp64_.x : fp64_.x_i4);
     kend();
     launch_i7<S>(D_, X_.as<S>(), fdiag_.as<S>(), f7_.as<S>(), d2ij_.as<S>(), i7off_.as<S>(), st_);
     launch_i9<S>(D_, n_hh2_, Vhh_.as<S>(), X_.as<S>(), I9_.as<S>(), st_);
@@ -1420,23 +1406,33 @@ class Engine final : public IEngine {
     launch_i6<S>(D_, (const int2 *)i6rows_.p, ni6rows_, i6dots_.as<S>(), T_.as<S>(), Vhp_.as<S>(), fdiag_.as<S>(),
                  f6_.as<S>(), d2ab_.as<S>(), i6off_.as<S>(), st_);
     mark(3);
-    kbegin(kKI4);
-    run_plan(planI4_);
-    kend();
+    if (apart) {
+      kbegin(kKI4);
+      run_plan(fp64_.i4);
+      kend();
+    }
     mark(4);
-    kbegin(kKRing);
-    run_plan(planRing_);
-    kend();
-    mark(5);
+    if (apart) {
+      kbegin(kKRing);
+      run_plan(fp64_.ring);
+      kend();
+      mark(5);
+      accumulate_timers(0, 5);
+      mark(6);
+      kbegin(kKLadder);
+      run_plan(fp64_.ladder);
+      kend();
+      mark(7);
+      accumulate_timers(6, 7);
+      mark(5);
+    } else {
+      run_plan(fp64_.ring_ladder);
+    }
     launch_rinit<S>(D_, omap_.as<int4>(), rmap_.as<int4>(), T_.as<S>(), Vhp_.as<S>(), Rph_.as<S>(), i6off_.as<S>(),
-                    i7off_.as<S>(), nullptr, nullptr, R_.as<S>(), st_);
+                    i7off_.as<S>(), nullptr, nullptr, true, R_.as<S>(), st_);
     mark(6);
-    kbegin(kKLadder);
-    run_plan(planLadder_);
-    kend();
-    mark(7);
     launches_ += 5;
-    if (timing_) accumulate_timers(0, 7);
+    if (apart) accumulate_timers(5, 6);
   }
   // Event pairs around individual launches (slots kK*), read back with the phase timers.
   void kbegin(int slot) {
@@ -2469,16 +2465,16 @@ class Engine final : public IEngine {
         if (pk.H > 0 && pk.P > 0) {
           GemmProb<S> a{};
           a.nseg = 1;
-          a.M = pk.P; a.N = pk.H;
-          a.seg[0] = GemmSeg<S>{Vpp_.as<S>() + voff, T_.as<S>() + pk.t_off, pk.P, 1, 1, pk.P, pk.P, 1.0};
-          a.C = PPb_.as<S>() + pk.t_off; a.sCm = 1; a.sCn = pk.P; a.accumulate = 0;
-          bp.add(a, (int64_t)pk.P * pk.P * pk.H);
+          a.M = pk.P; a.N = pk.H; a.alpha = 1.0;
+          a.seg[0] = GemmSeg<S>{Vpp_.as<S>() + voff, T_.as<S>() + pk.t_off, pk.P, 1, 1, pk.P, pk.P};
+          a.C = PPb_.as<S>() + pk.t_off; a.sCm = 1; a.sCn = pk.P;
+          bp.add(a);
           GemmProb<S> h{};
           h.nseg = 1;
-          h.M = pk.P; h.N = pk.H;
-          h.seg[0] = GemmSeg<S>{T_.as<S>() + pk.t_off, I9_.as<S>() + hoff, 1, pk.P, 1, pk.H, pk.H, 1.0};
-          h.C = HHb_.as<S>() + pk.t_off; h.sCm = 1; h.sCn = pk.P; h.accumulate = 0;
-          bh.add(h, (int64_t)pk.P * pk.H * pk.H);
+          h.M = pk.P; h.N = pk.H; h.alpha = 1.0;
+          h.seg[0] = GemmSeg<S>{T_.as<S>() + pk.t_off, I9_.as<S>() + hoff, 1, pk.P, 1, pk.H, pk.H};
+          h.C = HHb_.as<S>() + pk.t_off; h.sCm = 1; h.sCn = pk.P;
+          bh.add(h);
         }
         hoff += (int64_t)pk.H * pk.H;
         voff += (int64_t)pk.P * pk.P;
@@ -2527,7 +2523,7 @@ class Engine final : public IEngine {
     } else {
       xs = fork_side();
       kbegin(kKX);
-      run_x(xs);
+      run_plan(fp64_.x, xs);
       kend();
     }
     launch_i7<S>(D_, X_.as<S>(), fdiag_.as<S>(), f7_.as<S>(), d2ij_.as<S>(), i7off_.as<S>(), xs);
@@ -2554,18 +2550,18 @@ class Engine final : public IEngine {
       kend();
     } else {
       kbegin(kKI4);
-      run_plan(planI4_);
+      run_plan(fp64_.i4);
       kend();
       mark(4);
       kbegin(kKRing);
-      run_plan(planRing_);
+      run_plan(fp64_.ring);
       kend();
     }
     mark(5);
     join_side(xs);
     if (!digits && xs != st_) run_plan(planHH_, xs);  // HH_b = T' I9' beside the pp-ladder product
     launch_rinit<S>(D_, omap_.as<int4>(), rmap_.as<int4>(), T_.as<S>(), Vhp_.as<S>(), Rph_.as<S>(), i6off_.as<S>(),
-                    i7off_.as<S>(), nullptr, Rringb_.as<S>(), R_.as<S>(), st_);
+                    i7off_.as<S>(), nullptr, Rringb_.as<S>(), false, R_.as<S>(), st_);
     mark(6);
     if (digits) {
       // PP_b and then HH_b accumulate into PP_b (two launches in stream order)
@@ -2647,7 +2643,7 @@ class Engine final : public IEngine {
     mark(5);
     join_side(xs);
     launch_rinit<S>(D_, omap_.as<int4>(), rmap_.as<int4>(), T_.as<S>(), Vhp_.as<S>(), Rph_.as<S>(), i6off_.as<S>(),
-                    i7off_.as<S>(), Rringb_.as<S>(), nullptr, R_.as<S>(), st_);
+                    i7off_.as<S>(), Rringb_.as<S>(), nullptr, false, R_.as<S>(), st_);
     mark(6);
     kbegin(kKTcPP);
     run_tc(tcPP_);  // R' += PP_b + HH_b + V_pppp' dT' + dT' I9' + T_b' (I9' - I9_b')
@@ -2696,9 +2692,10 @@ class Engine final : public IEngine {
   int npp_total_ = 0, nhh_total_ = 0;  // packed pp and hh pairs over all channels
   DBuf okey_, oof_;                    // orbital -> quantum-number slot, slot -> orbital
   int nkeys_ = 0;
-  DBuf partial_, res_, flag_, stage_, hist_, hist_t_, hist_e_, xwork_, xgroups_, xpart_, i6rows_, i6dots_, omap_, rmap_;
-  int nxwork_ = 0, nxgroups_ = 0, ni6rows_ = 0;
-  Plan planLadder_, planI4_, planRing_, planPP_, planHH_;
+  DBuf partial_, res_, flag_, stage_, hist_, hist_t_, hist_e_, i6rows_, i6dots_, omap_, rmap_;
+  int ni6rows_ = 0;
+  Fp64Plans fp64_;
+  Plan planPP_, planHH_;
   // mixed precision
   bool mixed_ready_ = false;
   int tc_kind_ = 0;
@@ -2717,7 +2714,14 @@ class Engine final : public IEngine {
   SplitPlan gplan_;                                     // gather jobs (TcGatherJob) and chunks
   double *host_res_ = nullptr;
   int host_flag_ = 0;
-  int gemm_shape_[4] = {kShape128x32, kShape128x32, kShape64x64, kShape64x64};
+  // Warp tile per N bucket until the autotuner has measured this lattice.  4-row tiles, which
+  // put more lanes on K, are shorter and balance better: real lattices from PNM 14 nmax=1 to
+  // PNM 66 nmax=4 take 5 to 37% less with them in every bucket with more than a few products
+  // (PNM 66 nmax=4 6.80 against 7.32 ms, PNM 38 nmax=2 0.134 against 0.212).  Complex products
+  // of more than 32 columns are 1 to 3% faster in 8-row tiles (SNM 132 nmax=3, N > 64: 37.3
+  // against 37.6 ms), whose operands are read half as often.
+  int gemm_shape_[4] = {kShape4, kShape4, ScalarOf<S>::complex ? kShape8 : kShape4,
+                        ScalarOf<S>::complex ? kShape8 : kShape4};
   cudaStream_t cs_ = nullptr;       // copy stream of ccx_set_vblocks
   cudaEvent_t sev_[5] = {};         // copied[2], packed[2], compute-stream mark
   DBuf stage2_, copyjobs_;

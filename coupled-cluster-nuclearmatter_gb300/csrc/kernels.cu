@@ -41,6 +41,11 @@ __device__ inline void warp_reduce_scatter32(S (&v)[32], int lane) {
     }
   }
 }
+// a * b + c as FMAs
+__device__ __forceinline__ double madd(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ cplx madd(cplx a, cplx b, cplx c) {
+  return cplx(fma(a.re, b.re, fma(-a.im, b.im, c.re)), fma(a.re, b.im, fma(a.im, b.re, c.im)));
+}
 __device__ inline double2 to2(double x) { return make_double2(x, 0.0); }
 __device__ inline double2 to2(cplx x) { return make_double2(x.re, x.im); }
 template <typename S> __device__ inline S from2(double2 v);
@@ -125,117 +130,112 @@ template <> __device__ inline cplx cvt_in<cplx>(const double *p, int *flag) {
 }  // namespace
 
 // ============================================================================
-// grouped GEMM, FP64 FMA.  One CTA per BM x BN output tile of one problem; up to two
-// K segments share the accumulator (the pp-ladder and hh-ladder both add into R).
-// Thread (tm, tn) owns a TM x TN register tile, tm fastest; threads whose columns
-// lie beyond N skip the FMA loop, so narrow problems waste few FP64 lanes.
+// Grouped GEMM, FP64 FMA, for products of every shape the channels have (rows and columns
+// from 4 to some thousands, K from 4 on) in one launch.
+//
+// The FP64 pipe bounds it: two FMAs a clock on an SM, so a warp's FMA instruction holds its
+// scheduler's pipe for 64 clocks and operands straight from L1 keep up with it.  What costs is
+// an idle pipe: lanes beyond M, N or K, and SMs that wait for the longest tile.  So there is no
+// block tile and nothing in shared memory; each warp takes one small tile of its own, 32 / LK
+// rows by up to 8 columns (a column count of its own per tile, so N is cut without
+// remainder), its lanes splitting K by LK and reducing at the end.  A 64 x 64 block tile held
+// an SM for 1.7 ms at K = 472 (complex) while the whole product of the lattice takes 0.2 ms.
+// Whole plain FP64 solves: SNM 28 nmax=2 (complex) 108 to 12.1 ms, PNM 14 nmax=2 4.0 to 1.2
+// ms; two iterations of PNM 66 nmax=4 with the amplitudes read back 21.5 to 15.0 ms, the
+// products at 1.08 TFLOP/s of the 1.2 that a register-only FMA loop reaches.
 // ============================================================================
-template <typename S, int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(256) k_gemm(const GemmProb<S> *__restrict__ probs, const GemmTile *__restrict__ tiles) {
-  constexpr int BK = kGemmBK;
-  constexpr int NTM = BM / TM;  // threads along M
-  static_assert(NTM * (BN / TN) == 256, "256 threads");
-  __shared__ S As[BK][BM + 1];
-  __shared__ S Bs[BK][BN + 1];
-  const GemmTile tl = tiles[blockIdx.x];
-  const GemmProb<S> &pr = probs[tl.prob];
-  const int M = pr.M, N = pr.N, nseg = pr.nseg, kchunk = pr.kchunk;
-  const int tid = threadIdx.x;
-  const int tm = tid % NTM, tn = tid / NTM;
-  const bool active = (tl.m0 + tm * TM < M) && (tl.n0 + tn * TN < N);
-  S acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = S(0.0);
+template <int LK, int NJ, typename S>
+__device__ __forceinline__ void gemm_cols(const GemmProb<S> &pr, int m, int n0, int lk, S (&acc)[kGemmCols]) {
+  constexpr int U = ScalarOf<S>::complex ? 2 : 4;  // K steps whose loads are in flight together
+  const int nseg = pr.nseg;
   for (int s = 0; s < nseg; ++s) {
-    const S *A = pr.seg[s].A, *B = pr.seg[s].B;
-    const int64_t sAm = pr.seg[s].sAm, sAk = pr.seg[s].sAk, sBk = pr.seg[s].sBk, sBn = pr.seg[s].sBn;
-    const double alpha = pr.seg[s].alpha;
-    int kbeg = 0, kend = pr.seg[s].K;
-    if (kchunk > 0) {
-      kbeg = tl.kslice * kchunk;
-      kend = min(kend, kbeg + kchunk);
+    const GemmSeg<S> &g = pr.seg[s];
+    const int64_t sAk = g.sAk, sBk = g.sBk, sBn = g.sBn;
+    const S *A = g.A + (int64_t)m * g.sAm, *B = g.B + (int64_t)n0 * sBn;
+    const int K = g.K;
+    int k = lk;
+    for (; k + (U - 1) * LK < K; k += U * LK) {
+      S a[U], b[U][NJ];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        a[u] = A[(int64_t)(k + u * LK) * sAk];
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) b[u][j] = B[(int64_t)(k + u * LK) * sBk + j * sBn];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) acc[j] = madd(a[u], b[u][j], acc[j]);
     }
-    for (int k0 = kbeg; k0 < kend; k0 += BK) {
-      for (int x = tid; x < BM * BK; x += 256) {
-        int m, k;
-        if (sAm == 1) { m = x % BM; k = x / BM; } else { k = x % BK; m = x / BK; }
-        const int gm = tl.m0 + m, gk = k0 + k;
-        S v = S(0.0);
-        if (gm < M && gk < kend) v = alpha * A[(int64_t)gm * sAm + (int64_t)gk * sAk];
-        As[k][m] = v;
-      }
-      for (int x = tid; x < BK * BN; x += 256) {
-        int k, n;
-        if (sBk == 1) { k = x % BK; n = x / BK; } else { n = x % BN; k = x / BN; }
-        const int gk = k0 + k, gn = tl.n0 + n;
-        S v = S(0.0);
-        if (gk < kend && gn < N) v = B[(int64_t)gk * sBk + (int64_t)gn * sBn];
-        Bs[k][n] = v;
-      }
-      __syncthreads();
-      if (active) {
+    for (; k < K; k += LK) {
+      const S a = A[(int64_t)k * sAk];
+      S b[NJ];
 #pragma unroll
-        for (int k = 0; k < BK; ++k) {
-          S a[TM], b[TN];
+      for (int j = 0; j < NJ; ++j) b[j] = B[(int64_t)k * sBk + j * sBn];
 #pragma unroll
-          for (int i = 0; i < TM; ++i) a[i] = As[k][tm * TM + i];
-#pragma unroll
-          for (int j = 0; j < TN; ++j) b[j] = Bs[k][tn * TN + j];
-#pragma unroll
-          for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] += a[i] * b[j];
-        }
-      }
-      __syncthreads();
+      for (int j = 0; j < NJ; ++j) acc[j] = madd(a, b[j], acc[j]);
     }
   }
-  if (!active) return;
+}
+template <int LK, typename S>
+__device__ __forceinline__ void gemm_tile(const GemmProb<S> &pr, const GemmTile &tl, int lane) {
+  constexpr int ROWS = 32 / LK;
+  const int lk = lane % LK, lm = lane / LK;
+  for (int t = 0; t < tl.nm; ++t) {
+    const int row = tl.m0 + t * ROWS + lm;
+    const int m = min(row, pr.M - 1);  // rows beyond M repeat the last one and are not stored
+    S acc[kGemmCols];
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int m = tl.m0 + tm * TM + i;
-    if (m >= M) continue;
+    for (int j = 0; j < kGemmCols; ++j) acc[j] = S(0.0);
+    switch (tl.nj) {
+      case 8: gemm_cols<LK, 8>(pr, m, tl.n0, lk, acc); break;
+      case 7: gemm_cols<LK, 7>(pr, m, tl.n0, lk, acc); break;
+      case 6: gemm_cols<LK, 6>(pr, m, tl.n0, lk, acc); break;
+      case 5: gemm_cols<LK, 5>(pr, m, tl.n0, lk, acc); break;
+      case 4: gemm_cols<LK, 4>(pr, m, tl.n0, lk, acc); break;
+      case 3: gemm_cols<LK, 3>(pr, m, tl.n0, lk, acc); break;
+      case 2: gemm_cols<LK, 2>(pr, m, tl.n0, lk, acc); break;
+      default: gemm_cols<LK, 1>(pr, m, tl.n0, lk, acc); break;
+    }
+    // butterfly reduce-scatter over the LK lanes of a row: lane lk ends with the totals of
+    // columns lk * 8 / LK on
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int n = tl.n0 + tn * TN + j;
-      if (n >= N) continue;
-      if (kchunk > 0) {
-        pr.part[(int64_t)tl.kslice * M * N + m + (int64_t)M * n] = acc[i][j];
-        continue;
+    for (int o = LK / 2, n = kGemmCols; o >= 1; o >>= 1, n >>= 1) {
+      const bool upper = (lk & o) != 0;
+#pragma unroll
+      for (int i = 0; i < n / 2; ++i) {
+        const S give = upper ? acc[i] : acc[i + n / 2];
+        const S keep = upper ? acc[i + n / 2] : acc[i];
+        acc[i] = keep + shfl_xor(give, o);
       }
-      const int64_t o = (int64_t)m * pr.sCm + (int64_t)n * pr.sCn;
-      if (pr.accumulate) pr.C[o] += acc[i][j];
-      else pr.C[o] = (pr.C0 ? pr.C0[o] : S(0.0)) + acc[i][j];
+    }
+    if (row >= pr.M) continue;
+#pragma unroll
+    for (int i = 0; i < kGemmCols / LK; ++i) {
+      const int j = lk * (kGemmCols / LK) + i;
+      if (j >= tl.nj) break;
+      const int64_t o = (int64_t)row * pr.sCm + (int64_t)(tl.n0 + j) * pr.sCn;
+      const S v = pr.alpha == 1.0 ? acc[i] : pr.alpha * acc[i];
+      if (pr.accumulate) pr.C[o] += v;
+      else if (pr.C0) pr.C[o] = pr.C0[o] + v;
+      else pr.C[o] = v;
     }
   }
+}
+template <typename S>
+__global__ void __launch_bounds__(128) k_gemm(const GemmProb<S> *__restrict__ probs, const GemmTile *__restrict__ tiles,
+                                              int n8, int n) {
+  const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (w >= n) return;
+  const GemmTile tl = tiles[w];
+  if (w < n8) gemm_tile<4>(probs[tl.prob], tl, lane);
+  else gemm_tile<8>(probs[tl.prob], tl, lane);
 }
 
 template <typename S>
-void launch_gemm(int shape, const GemmProb<S> *probs, const GemmTile *tiles, int ntiles, cudaStream_t st) {
-  if (ntiles <= 0) return;
-  if (shape == kShape64x64) k_gemm<S, 64, 64, 4, 4><<<ntiles, 256, 0, st>>>(probs, tiles);
-  else k_gemm<S, 128, 32, 8, 2><<<ntiles, 256, 0, st>>>(probs, tiles);
-}
-
-template <typename S>
-__global__ void k_splitk_reduce(const GemmProb<S> *__restrict__ probs, const int *__restrict__ plist) {
-  const GemmProb<S> &pr = probs[plist[blockIdx.x]];
-  const int M = pr.M, N = pr.N;
-  const int ns = (pr.seg[0].K + pr.kchunk - 1) / pr.kchunk;
-  for (int e = threadIdx.x; e < M * N; e += blockDim.x) {
-    S acc = S(0.0);
-    for (int s = 0; s < ns; ++s) acc += pr.part[(int64_t)s * M * N + e];
-    const int m = e % M, n = e / M;
-    const int64_t o = (int64_t)m * pr.sCm + (int64_t)n * pr.sCn;
-    if (pr.accumulate) pr.C[o] += acc;
-    else pr.C[o] = (pr.C0 ? pr.C0[o] : S(0.0)) + acc;
-  }
-}
-template <typename S>
-void launch_splitk_reduce(const GemmProb<S> *probs, const int *plist, int n, cudaStream_t st) {
-  if (n > 0) k_splitk_reduce<S><<<n, 256, 0, st>>>(probs, plist);
+void launch_gemm(const GemmProb<S> *probs, const GemmTile *tiles, int n8, int n4, cudaStream_t st) {
+  if (n8 + n4 <= 0) return;
+  k_gemm<S><<<(n8 + n4 + 3) / 4, 128, 0, st>>>(probs, tiles, n8, n8 + n4);
 }
 
 // ============================================================================
@@ -289,112 +289,6 @@ __global__ void k_tph_map(DevLayout L, int32_t *__restrict__ map) {
 }
 void launch_tph_map(const DevLayout &L, int32_t *map, cudaStream_t st) {
   if (L.nphtile) k_tph_map<<<L.nphtile, 256, 0, st>>>(L, map);
-}
-
-// ============================================================================
-// X'(m, j) = sum_k V'(k, m) T'(k, j) per hhpp channel (the V_hhpp T product of the I9
-// ZGEMM, ccm_t2_eqn.f90:459, on packed pairs).  V_hhpp' and T' are P x H column-major,
-// so X(m, j) is the dot product of two contiguous columns of length P.  One CTA per
-// (channel, kXM rows, kXJ columns): the kXJ columns of T' are staged in shared memory
-// in K chunks, each warp owns rows m (lanes stride over k), and the lane partials are
-// reduced with shuffles at the end, in a fixed order.
-// ============================================================================
-template <typename S, int NJ>
-__device__ __forceinline__ void xdot_rows(const S *__restrict__ V, const S (*Ts)[kXK], int64_t off, int P, int H, int m0,
-                                          int k0, int kn, int warp, int lane, S (&acc)[kXM / 8][kXJ]) {
-  constexpr int RPW = kXM / 8;
-#pragma unroll
-  for (int r = 0; r < RPW; ++r) {
-    const int m = m0 + warp + 8 * r;
-    if (m >= H) break;
-    const S *vc = V + off + (int64_t)P * m + k0;
-    int k = lane;
-    // two independent loads in flight per iteration
-    for (; k + 32 < kn; k += 64) {
-      const S v0 = vc[k], v1 = vc[k + 32];
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        acc[r][j] += v0 * Ts[j][k];
-        acc[r][j] += v1 * Ts[j][k + 32];
-      }
-    }
-    if (k < kn) {
-      const S v = vc[k];
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) acc[r][j] += v * Ts[j][k];
-    }
-  }
-}
-
-template <typename S>
-__global__ void __launch_bounds__(256) k_xdot(DevLayout L, const int4 *__restrict__ work, const S *__restrict__ V,
-                                              const S *__restrict__ T, S *__restrict__ part) {
-  constexpr int RPW = kXM / 8;  // rows per warp
-  __shared__ S Ts[kXJ][kXK];
-  const int4 w = work[blockIdx.x];  // (channel, m0 | j0 << 16, K slice, partial slot)
-  const int ch = w.x, m0 = w.y & 0xffff, j0 = w.y >> 16;
-  const int H = L.H[ch];
-  const int kbeg = w.z * kXSlice;
-  const int P = min(L.P[ch], kbeg + kXSlice);  // this item's K range is [kbeg, P)
-  const int64_t off = L.t_off[ch];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nj = min(kXJ, H - j0);
-  S acc[RPW][kXJ];
-#pragma unroll
-  for (int r = 0; r < RPW; ++r)
-#pragma unroll
-    for (int j = 0; j < kXJ; ++j) acc[r][j] = S(0.0);
-  const int ld = L.P[ch];  // column length of V' and T'
-  for (int k0 = kbeg; k0 < P; k0 += kXK) {
-    const int kn = min(kXK, P - k0);
-    for (int x = threadIdx.x; x < kXJ * kXK; x += blockDim.x) {
-      const int j = x / kXK, k = x % kXK;
-      Ts[j][k] = (j < nj && k < kn) ? T[off + (int64_t)ld * (j0 + j) + k0 + k] : S(0.0);
-    }
-    __syncthreads();
-    // no FP64 work on the padding columns of a partial column block
-    switch (nj) {
-      case 8: xdot_rows<S, 8>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-      case 7: xdot_rows<S, 7>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-      case 6: xdot_rows<S, 6>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-      case 5: xdot_rows<S, 5>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-      case 4: xdot_rows<S, 4>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-      case 3: xdot_rows<S, 3>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-      case 2: xdot_rows<S, 2>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-      default: xdot_rows<S, 1>(V, Ts, off, ld, H, m0, k0, kn, warp, lane, acc); break;
-    }
-    __syncthreads();
-  }
-  // the item's kXM x kXJ partial tile, row-major, in its slot: lane l of the warp ends
-  // with value l = (r, j) = (l / kXJ, l % kXJ) of the warp's rows
-  static_assert(RPW * kXJ == 32, "one value per lane after the reduce-scatter");
-  S vals[32];
-#pragma unroll
-  for (int r = 0; r < RPW; ++r)
-#pragma unroll
-    for (int j = 0; j < kXJ; ++j) vals[r * kXJ + j] = acc[r][j];
-  warp_reduce_scatter32(vals, lane);
-  part[(int64_t)w.w * (kXM * kXJ) + (warp + 8 * (lane / kXJ)) * kXJ + lane % kXJ] = vals[0];
-}
-// X tile (channel, m0 | j0 << 16, first slot, slices): the K-slice partials summed in
-// slice order, so the result does not depend on which item finished first
-template <typename S>
-__global__ void __launch_bounds__(kXM * kXJ) k_xreduce(DevLayout L, const int4 *__restrict__ groups,
-                                                       const S *__restrict__ part, S *__restrict__ X) {
-  const int4 g = groups[blockIdx.x];
-  const int ch = g.x, m0 = g.y & 0xffff, j0 = g.y >> 16, H = L.H[ch];
-  const int mr = threadIdx.x / kXJ, j = threadIdx.x % kXJ;
-  if (m0 + mr >= H || j0 + j >= H) return;
-  S tot = part[(int64_t)g.z * (kXM * kXJ) + threadIdx.x];
-  for (int s = 1; s < g.w; ++s) tot += part[(int64_t)(g.z + s) * (kXM * kXJ) + threadIdx.x];
-  X[L.hh2_off[ch] + (m0 + mr) + (int64_t)H * (j0 + j)] = tot;
-}
-template <typename S>
-void launch_xdot(const DevLayout &L, const int4 *work, int nwork, const int4 *groups, int ngroups, const S *V,
-                 const S *T, S *part, S *X, cudaStream_t st) {
-  if (nwork <= 0) return;
-  k_xdot<S><<<nwork, 256, 0, st>>>(L, work, V, T, part);
-  k_xreduce<S><<<ngroups, kXM * kXJ, 0, st>>>(L, groups, part, X);
 }
 
 // ============================================================================
@@ -704,7 +598,7 @@ template <typename S>
 __global__ void k_rinit(DevLayout L, const int4 *__restrict__ omap, const int4 *__restrict__ rmap, const S *__restrict__ T,
                         const S *__restrict__ Vhp, const S *__restrict__ Rph, const S *__restrict__ i6off,
                         const S *__restrict__ i7off, const S *__restrict__ ring_base, S *__restrict__ ring_out,
-                        S *__restrict__ R) {
+                        int add, S *__restrict__ R) {
   const int2 tl = L.ttile[blockIdx.x];
   const int ch = tl.x;
   const int P = L.P[ch], H = L.H[ch];
@@ -731,14 +625,14 @@ __global__ void k_rinit(DevLayout L, const int4 *__restrict__ omap, const int4 *
     const S ring = at_or_zero(Rph, m.x) - at_or_zero(Rph, m.y) - at_or_zero(Rph, m.z) + at_or_zero(Rph, m.w);
     if (ring_out) ring_out[base + e] = ring;  // the ring term of this R_ph, kept per amplitude
     r += ring_base ? ring_base[base + e] + ring : ring;
-    R[base + e] = r;
+    R[base + e] = add ? R[base + e] + r : r;
   }
 }
 template <typename S>
 void launch_rinit(const DevLayout &L, const int4 *omap, const int4 *rmap, const S *T, const S *Vhp, const S *Rph,
-                  const S *i6off, const S *i7off, const S *ring_base, S *ring_out, S *R, cudaStream_t st) {
+                  const S *i6off, const S *i7off, const S *ring_base, S *ring_out, bool add, S *R, cudaStream_t st) {
   if (L.nttile)
-    k_rinit<S><<<L.nttile, 256, 0, st>>>(L, omap, rmap, T, Vhp, Rph, i6off, i7off, ring_base, ring_out, R);
+    k_rinit<S><<<L.nttile, 256, 0, st>>>(L, omap, rmap, T, Vhp, Rph, i6off, i7off, ring_base, ring_out, add, R);
 }
 
 // ============================================================================
@@ -1590,20 +1484,17 @@ void launch_unpack_t(const DevLayout &L, const DevOrdered &O, int c0, int c1, in
 
 // ---- explicit instantiations -------------------------------------------------
 #define CCX_INST(S)                                                                                                    \
-  template void launch_gemm<S>(int, const GemmProb<S> *, const GemmTile *, int, cudaStream_t);                         \
-  template void launch_splitk_reduce<S>(const GemmProb<S> *, const int *, int, cudaStream_t);                          \
+  template void launch_gemm<S>(const GemmProb<S> *, const GemmTile *, int, int, cudaStream_t);                         \
   template void launch_gather_tph<S>(const DevLayout &, const S *, S *, cudaStream_t);                                 \
   template void launch_i7<S>(const DevLayout &, const S *, const S *, const S *, S *, S *, cudaStream_t);             \
   template void launch_i7_direct<S>(const DevLayout &, const S *, const S *, S *, const S *, const S *, S *, S *,      \
                                     cudaStream_t);                                                                  \
   template void launch_i9b<S>(int64_t, const S *, const S *, const S *, S *, cudaStream_t);                         \
   template void launch_i9<S>(const DevLayout &, int64_t, const S *, const S *, S *, cudaStream_t);                     \
-  template void launch_xdot<S>(const DevLayout &, const int4 *, int, const int4 *, int, const S *, const S *, S *, S *, \
-                              cudaStream_t);        \
   template void launch_i6<S>(const DevLayout &, const int2 *, int, S *, const S *, const S *, const S *, const S *,   \
                              S *, S *, cudaStream_t);                                                                  \
   template void launch_rinit<S>(const DevLayout &, const int4 *, const int4 *, const S *, const S *, const S *,      \
-                               const S *, const S *, const S *, S *, S *, cudaStream_t);                                                         \
+                               const S *, const S *, const S *, S *, bool, S *, cudaStream_t);                      \
   template void launch_update<S>(const DevLayout &, int, S *, const S *, const S *, const S *, const S *, S *,         \
                                  typename StepOf<S>::type *,                                                            \
                                  double *, double *, cudaStream_t);                                                    \

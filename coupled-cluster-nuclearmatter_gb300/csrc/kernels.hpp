@@ -11,40 +11,37 @@
 namespace ccx {
 
 // ---- grouped GEMM (FP64 / complex FP64) ------------------------------------
-// C(m,n) [+]= sum_s alpha_s * sum_k A_s(m,k) B_s(k,n), element strides per operand.
+// C(m,n) = [C or C0 or 0] + alpha sum_s sum_k A_s(m,k) B_s(k,n), element strides per operand.
 template <typename S>
 struct GemmSeg {
   const S *A, *B;
   int64_t sAm, sAk, sBk, sBn;
   int K;
-  double alpha;
 };
 template <typename S>
 struct GemmProb {
   GemmSeg<S> seg[2];
   int nseg;
   int M, N;
+  double alpha;
   S *C;
   const S *C0;  // initial value when accumulate == 0 (nullptr: zero)
   int64_t sCm, sCn;
   int accumulate;
-  int kchunk;   // > 0: split-K over one segment; tile.kslice picks the chunk
-  S *part;      // split-K partial products, kslice-major, each M x N column-major
 };
+// The work of one warp: nm row tiles from m0 on, columns n0 .. n0 + nj - 1 (nj <= kGemmCols).
 struct GemmTile {
-  int prob, m0, n0, kslice;
+  int prob, m0, n0;
+  int16_t nj, nm;
 };
-constexpr int kGemmBK = 16;
-// two tile shapes: 64x64 (4x4 per thread) and 128x32 (8x2 per thread, for N <= 32)
-enum GemmShape { kShape64x64 = 0, kShape128x32 = 1 };
-inline int gemm_bm(int shape) { return shape == kShape64x64 ? 64 : 128; }
-inline int gemm_bn(int shape) { return shape == kShape64x64 ? 64 : 32; }
+constexpr int kGemmCols = 8;
+// two warp tiles: 8 rows with K over 4 lanes each, 4 rows with K over 8 lanes each
+enum GemmShape { kShape8 = 0, kShape4 = 1 };
+inline int gemm_rows(int shape) { return shape == kShape8 ? 8 : 4; }
 
+// tiles of shape 0 first (n8 of them), then n4 of shape 1
 template <typename S>
-void launch_gemm(int shape, const GemmProb<S> *probs, const GemmTile *tiles, int ntiles, cudaStream_t st);
-// C = (accumulate ? C : C0 or 0) + sum over the split-K partials, fixed order
-template <typename S>
-void launch_splitk_reduce(const GemmProb<S> *probs, const int *plist, int n, cudaStream_t st);
+void launch_gemm(const GemmProb<S> *probs, const GemmTile *tiles, int n8, int n4, cudaStream_t st);
 
 // ---- potentials -----------------------------------------------------------
 struct DevPotential {
@@ -62,14 +59,6 @@ void launch_lattice_tables(const DevOrbits &O, const DevPotential &pot, double *
 template <typename S> void launch_gather_tph(const DevLayout &L, const S *T, S *Tph, cudaStream_t st);
 // where each T_ph entry comes from: +/-(packed T' index + 1), 0 for a zero entry
 void launch_tph_map(const DevLayout &L, int32_t *map, cudaStream_t st);
-// X' = V_hhpp'^T T' per channel; work items (channel, first row, first column, 0)
-constexpr int kXM = 32, kXJ = 8, kXK = 256;
-constexpr int kXSlice = 512;  // K per X work item: long channels are split, partials summed in order
-// X = V_hhpp'^T T' as K-sliced column-dot items into partial slots, then the slices
-// summed in order (work and groups built by the engine)
-template <typename S>
-void launch_xdot(const DevLayout &L, const int4 *work, int nwork, const int4 *groups, int ngroups, const S *V,
-                 const S *T, S *part, S *X, cudaStream_t st);
 template <typename S> void launch_i7(const DevLayout &L, const S *X, const S *fdiag, const S *f7, S *d2ij, S *i7off, cudaStream_t st);
 template <typename S> void launch_i9(const DevLayout &L, int64_t n, const S *Vhh, const S *X, S *I9, cudaStream_t st);
 // I7 without X: the X entries it reads as 2 A^2 column dots of V_hhpp' and T' into xd
@@ -88,10 +77,11 @@ template <typename S> void launch_i6(const DevLayout &L, const int2 *rowtile, in
 // R' initialisation; omap / rmap (int4 per packed amplitude) from launch_rinit_maps.
 // The ring term gathered from Rph is stored per amplitude into ring_out when given, and
 // ring_base (per amplitude) is added to it when given: a ring split as R_ph,b + dR_ph.
+// add: R' += the terms (R' holds the ladders already) instead of R' = the terms.
 void launch_rinit_maps(const DevLayout &L, int4 *omap, int4 *rmap, cudaStream_t st);
 template <typename S>
 void launch_rinit(const DevLayout &L, const int4 *omap, const int4 *rmap, const S *T, const S *Vhp, const S *Rph,
-                  const S *i6off, const S *i7off, const S *ring_base, S *ring_out, S *R, cudaStream_t st);
+                  const S *i6off, const S *i7off, const S *ring_base, S *ring_out, bool add, S *R, cudaStream_t st);
 
 // ---- update / energy / norms (per-block partial sums, then a fixed-order finish) --
 // mode 0: reference update T <- 0.75 T + 0.25 R/D, history column written
