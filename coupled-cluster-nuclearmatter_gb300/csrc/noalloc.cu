@@ -4,10 +4,9 @@
 // buffer through its own pool (the Fortran host keeps t2_ccm and vnn_hhpp in arrays it
 // manages), or code running where an allocation would be an error.  For them this
 // entry point evaluates E = 1/4 sum_ch sum_{ab,ij} T(ab,ij) V(ij,ab) directly on their
-// buffers, in the reference's layout (ccm_energy.f90:4-71).  Its scratch -- per-channel
-// offsets and partial sums -- is the file-scope array g_energy_slots below, at most
-// kMaxChannels channels (512 KiB), held by every GPU that loads the library until the
-// process exits.
+// buffers, in the reference's layout (ccm_energy.f90:4-71).  Its scratch -- one partial sum
+// per block -- is in the file-scope array g_energy_slots below (512 KiB), held by every GPU
+// that loads the library until the process exits.
 //
 // Set-up: the first call in a CUDA context (with that context's device current) looks
 // up the device address of g_energy_slots with cudaGetSymbolAddress; make that first
@@ -31,9 +30,8 @@ constexpr int kMaxChannels = 16384;
 constexpr int kMaxDevices = 64;
 
 struct __align__(16) EnergySlot {
-  long long off;  // first element of the channel's blocks
-  double re, im;  // channel partial sum
-  long long pad;
+  double re, im;  // partial sum of a block
+  double pad[2];
 };
 
 static __device__ __align__(256) EnergySlot g_energy_slots[kMaxChannels];
@@ -71,85 +69,157 @@ unsigned long long current_context_id() {
   return id;
 }
 
-// exclusive prefix sum of n_hh * n_pp into the slot offsets (one block)
-__global__ void k_noalloc_offsets(int nch, const int *__restrict__ dims, EnergySlot *slots) {
-  __shared__ long long part[1024];
-  const int per = (nch + blockDim.x - 1) / blockDim.x;
-  const int lo = threadIdx.x * per, hi = min(nch, lo + per);
-  long long s = 0;
-  for (int c = lo; c < hi; ++c) s += (long long)dims[2 * c] * dims[2 * c + 1];
-  part[threadIdx.x] = s;
+// Partial sums of T(ab,ij) V(ij,ab), T (n_pp x n_hh) and V (n_hh x n_pp) of every channel.
+//
+// The sizes are on the device only, so the grid is fixed and every block finds the work by a
+// scan of dims, kScan channels at a time.  A warp's task is 32 ab by up to 8 ij of a channel:
+// its lanes read T along ab, and each its own 128-byte run of V, all sixteen loads in flight
+// at once.  One block per channel behind a scan kernel of its own left 25 blocks with a strided
+// V for a small lattice: 58 us a call at PNM 14 nmax=2 (1 MB of each), now 10.2; PNM 66 nmax=4
+// (129 MB of each) 1212 to 75 us.
+constexpr int kEnergyBlocks = 304, kEnergyThreads = 256, kScan = 4 * kEnergyThreads;
+// blocks of the call in progress that have written their partial sum: every launch counts it
+// round to 0 again
+static __device__ unsigned g_energy_done;
+__device__ __forceinline__ double2 energy_load(const double *p, bool vec) {
+  if (vec) return *reinterpret_cast<const double2 *>(p);
+  return make_double2(p[0], p[1]);
+}
+__global__ void __launch_bounds__(kEnergyThreads) k_noalloc_energy(int nch, const int *__restrict__ dims,
+                                                                   const double *__restrict__ t2,
+                                                                   const double *__restrict__ v, bool vec,
+                                                                   EnergySlot *slots, double *__restrict__ energy) {
+  __shared__ long long off[kScan];  // first element of each channel of the chunk
+  __shared__ int task[kScan + 1];   // first task of each
+  __shared__ long long wsum[kEnergyThreads / 32];
+  __shared__ int wtask[kEnergyThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int w = wid * kEnergyBlocks + blockIdx.x;  // few tasks go to as many SMs
+  constexpr int stride = kEnergyBlocks * (kEnergyThreads / 32);
+  long long off0 = 0;  // elements of the chunks before
+  int task0 = 0;       // and their tasks, modulo stride
+  double re = 0.0, im = 0.0, re1 = 0.0, im1 = 0.0;  // two chains of each: even and odd ij
+  for (int c0 = 0; c0 < nch; c0 += kScan) {
+    long long ne[4], es = 0;
+    int nt[4], ts = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int c = c0 + 4 * tid + q;
+      const int nh = c < nch ? dims[2 * c] : 0, np = c < nch ? dims[2 * c + 1] : 0;
+      ne[q] = es;
+      nt[q] = ts;
+      es += (long long)nh * np;
+      ts += ((np + 31) / 32) * ((nh + 7) / 8);
+    }
+    // exclusive scan of the threads' totals
+    long long ei = es;
+    int ti = ts;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long a = __shfl_up_sync(0xffffffffu, ei, o);
+      const int b = __shfl_up_sync(0xffffffffu, ti, o);
+      if (lane >= o) { ei += a; ti += b; }
+    }
+    __syncthreads();  // the previous chunk's tables are no longer read
+    if (lane == 31) { wsum[wid] = ei; wtask[wid] = ti; }
+    __syncthreads();
+    long long eb = 0, et = 0;
+    int tb = 0, tt = 0;
+#pragma unroll
+    for (int k = 0; k < kEnergyThreads / 32; ++k) {
+      if (k < wid) { eb += wsum[k]; tb += wtask[k]; }
+      et += wsum[k];
+      tt += wtask[k];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      off[4 * tid + q] = off0 + eb + ei - es + ne[q];
+      task[4 * tid + q] = tb + ti - ts + nt[q];
+    }
+    if (tid == 0) task[kScan] = tt;
+    __syncthreads();
+    // the warp's tasks of this chunk: global task numbers w, w + stride, ...
+    for (int g = w >= task0 ? w - task0 : w - task0 + stride; g < tt; g += stride) {
+      int lo = 0, hi = min(kScan, nch - c0);  // task[lo] <= g < task[lo + 1]
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (task[mid] <= g) lo = mid;
+        else hi = mid;
+      }
+      const long long nh = dims[2 * (c0 + lo)], np = dims[2 * (c0 + lo) + 1];
+      const int njb = (int)((nh + 7) / 8), loc = g - task[lo];
+      const long long ab = (long long)(loc / njb) * 32 + lane, ij0 = (long long)(loc % njb) * 8;
+      const int nj = (int)min(8ll, nh - ij0);
+      if (ab >= np) continue;
+      const double *t = t2 + 2 * (off[lo] + ab + np * ij0), *x = v + 2 * (off[lo] + ij0 + nh * ab);
+      double2 a[8], b[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const bool live = j < nj;
+        a[j] = live ? energy_load(t + 2 * np * j, vec) : make_double2(0.0, 0.0);
+        b[j] = live ? energy_load(x + 2 * j, vec) : make_double2(0.0, 0.0);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        re = fma(a[j].x, b[j].x, fma(-a[j].y, b[j].y, re));
+        im = fma(a[j].x, b[j].y, fma(a[j].y, b[j].x, im));
+        re1 = fma(a[j + 1].x, b[j + 1].x, fma(-a[j + 1].y, b[j + 1].y, re1));
+        im1 = fma(a[j + 1].x, b[j + 1].y, fma(a[j + 1].y, b[j + 1].x, im1));
+      }
+    }
+    off0 += et;
+    task0 = (int)(((long long)task0 + tt) % stride);
+  }
+  // The block's sum, halving the warps that add in each step: shuffles in every warp would
+  // be five FP64 additions a value on all eight, on a pipe of two a clock.
+  __shared__ double2 part[kEnergyThreads];
+  part[tid] = make_double2(re + re1, im + im1);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    long long acc = 0;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      const long long v = part[t];
-      part[t] = acc;
-      acc += v;
+#pragma unroll
+  for (int o = kEnergyThreads / 2; o >= 32; o >>= 1) {
+    if (tid < o) {
+      part[tid].x += part[tid + o].x;
+      part[tid].y += part[tid + o].y;
+    }
+    __syncthreads();
+  }
+  if (wid == 0) {
+    re = part[lane].x;
+    im = part[lane].y;
+    for (int o = 16; o > 0; o >>= 1) {
+      re += __shfl_xor_sync(0xffffffffu, re, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
     }
   }
+  __shared__ bool last;
+  if (tid == 0) {
+    __stcg(&slots[blockIdx.x].re, re);
+    __stcg(&slots[blockIdx.x].im, im);
+    __threadfence();
+    last = atomicInc(&g_energy_done, kEnergyBlocks - 1) == kEnergyBlocks - 1;
+  }
   __syncthreads();
-  long long off = part[threadIdx.x];
-  for (int c = lo; c < hi; ++c) {
-    slots[c].off = off;
-    off += (long long)dims[2 * c] * dims[2 * c + 1];
+  if (!last || wid) return;
+  // the block that finished last: 1/4 of the partials' sum, in a fixed order
+  __threadfence();
+  re = im = 0.0;
+  double2 got[(kEnergyBlocks + 31) / 32];  // every load in flight before the first addition
+#pragma unroll
+  for (int k = 0; k < (kEnergyBlocks + 31) / 32; ++k) {
+    const int c = lane + 32 * k;
+    got[k] = c < kEnergyBlocks ? __ldcg(reinterpret_cast<const double2 *>(&slots[c].re)) : make_double2(0.0, 0.0);
   }
-}
-
-// one block per channel: 1/4 sum T(ab,ij) V(ij,ab), T (n_pp x n_hh), V (n_hh x n_pp)
-__global__ void k_noalloc_channel(const int *__restrict__ dims, const double *__restrict__ t2,
-                                  const double *__restrict__ v, EnergySlot *slots) {
-  const int c = blockIdx.x;
-  const int nh = dims[2 * c], np = dims[2 * c + 1];
-  const long long off = slots[c].off;
-  double re = 0.0, im = 0.0;
-  for (long long e = threadIdx.x; e < (long long)nh * np; e += blockDim.x) {
-    const long long ab = e % np, ij = e / np;
-    const double *t = t2 + 2 * (off + ab + (long long)np * ij);
-    const double *w = v + 2 * (off + ij + (long long)nh * ab);
-    re += 0.25 * (t[0] * w[0] - t[1] * w[1]);
-    im += 0.25 * (t[0] * w[1] + t[1] * w[0]);
+#pragma unroll
+  for (int k = 0; k < (kEnergyBlocks + 31) / 32; ++k) {
+    re += got[k].x;
+    im += got[k].y;
   }
-  __shared__ double sr[32], si[32];
   for (int o = 16; o > 0; o >>= 1) {
     re += __shfl_xor_sync(0xffffffffu, re, o);
     im += __shfl_xor_sync(0xffffffffu, im, o);
   }
-  if ((threadIdx.x & 31) == 0) {
-    sr[threadIdx.x >> 5] = re;
-    si[threadIdx.x >> 5] = im;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0, b = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      a += sr[w];
-      b += si[w];
-    }
-    slots[c].re = a;
-    slots[c].im = b;
-  }
-}
-
-// fixed-order sum of the channel partials
-__global__ void k_noalloc_finish(int nch, const EnergySlot *slots, double *energy) {
-  __shared__ double sr[256], si[256];
-  double a = 0.0, b = 0.0;
-  for (int c = threadIdx.x; c < nch; c += blockDim.x) {
-    a += slots[c].re;
-    b += slots[c].im;
-  }
-  sr[threadIdx.x] = a;
-  si[threadIdx.x] = b;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double x = 0.0, y = 0.0;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      x += sr[t];
-      y += si[t];
-    }
-    energy[0] = x;
-    energy[1] = y;
+  if (lane == 0) {
+    energy[0] = 0.25 * re;
+    energy[1] = 0.25 * im;
   }
 }
 
@@ -190,9 +260,8 @@ extern "C" int ccx_ccd_energy_noalloc(int32_t nch, const int32_t *dims, const do
     slots = c.addr;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  k_noalloc_offsets<<<1, 1024, 0, st>>>(nch, dims, slots);
-  k_noalloc_channel<<<nch, 256, 0, st>>>(dims, t2, vhhpp, slots);
-  k_noalloc_finish<<<1, 256, 0, st>>>(nch, slots, energy);
+  const bool vec = ((reinterpret_cast<uintptr_t>(t2) | reinterpret_cast<uintptr_t>(vhhpp)) & 15) == 0;
+  k_noalloc_energy<<<kEnergyBlocks, kEnergyThreads, 0, st>>>(nch, dims, t2, vhhpp, vec, slots, energy);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     ccx::set_last_error(cudaGetErrorString(e));
