@@ -1,6 +1,7 @@
-// Learned warm start (see learner.hpp): feature extraction, FP32 training kernels
-// (strided SIMT GEMM with fused bias/SiLU epilogues, split-K weight gradients reduced in a
-// fixed order, Adam) and the fused BF16 tensor-core inference kernel.
+// Learned warm start (see learner.hpp): feature extraction, FP32 training kernels (a tile of
+// samples through all layers and back in one kernel, sliced weight gradients reduced in a fixed
+// order, Adam) and the fused BF16 tensor-core inference kernel.
+#include <cuda_pipeline.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -172,129 +173,387 @@ __global__ void k_ml_gather(const float *__restrict__ Xs, const float *__restric
 // ---------------------------------------------------------------- FP32 training
 __device__ __forceinline__ float sigm(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float silu(float z) { return z * sigm(z); }
-__device__ __forceinline__ float dsilu(float z) {
-  const float s = sigm(z);
-  return s * (1.0f + z * (1.0f - s));
+
+// A training pass is three kernels: k_ml_pass runs a tile of samples through all layers,
+// forward and back, k_ml_wgrad forms the weight gradients from the activations and
+// differences it left, k_ml_grad adds the partial sums up.
+//
+// k_ml_pass: 256 threads take a tile of 16 R samples; thread (tm, tn) owns samples
+// R tm .. R tm + R - 1 and the columns 4 tn .. 4 tn + 3 and 64 + 4 tn .. 64 + 4 tn + 3 of every
+// layer, so silu'(Z1), silu'(Z2), silu'(Z3) stay in its registers for the way back, and only the
+// 128-wide operand of the next product goes through shared memory (k-major).  The weights of a
+// product are copied while the one before it runs.  FP32 FMAs bound it: 1.7 GFLOP for 8192
+// samples.  The layers as 25 separate launches of a 64 x 64 tile GEMM, the gradients and column
+// sums among them on a few dozen blocks, took 966 us with the copies to and from the host; now 127.
+constexpr int kPassThreads = 256;
+constexpr int kWRow = kMlW;  // floats of one k of a weight operand in shared memory
+template <int R>
+struct PassTile {
+  static constexpr int kSamples = 16 * R;
+  static constexpr int kActRow = kSamples + 4;
+  static constexpr size_t kSmem = (2 * kMlW * kWRow + kMlW * kActRow + 16 * kMlW) * sizeof(float);
+};
+struct PassArgs {
+  const float *X, *y;     // samples (n x kMlIn) and targets; y null: forward only
+  int n;
+  const float *p, *pT;    // parameters, and W1, W2, W3 transposed ([in][out], at the same order)
+  float *out;             // forward only: the outputs
+  float *H1, *H2, *D1, *D2, *D3;  // activations and pre-activation differences (n x kMlW)
+  float *part;            // per tile: db1, db2, db3, dw4 (kMlW each), db4
+  double *loss;           // per tile: sum of squared differences
+};
+constexpr int kPartLen = 4 * kMlW + 1;
+constexpr int kPT1 = 0, kPT2 = kPT1 + kMlIn * kMlW, kPT3 = kPT2 + kMlW * kMlW, kPTLen = kPT3 + kMlW * kMlW;
+
+__device__ __forceinline__ void copy_weights(float *dst, const float *src, int floats) {
+  for (int x = 4 * threadIdx.x; x < floats; x += 4 * kPassThreads) __pipeline_memcpy_async(dst + x, src + x, 16);
+  __pipeline_commit();
+}
+// acc(m, c) = sum_k act[k][m] w[k][c] over the thread's samples and columns
+template <int R>
+__device__ __forceinline__ void pass_product(const float *act, const float *w, int K, int tm, int tn, float (&acc)[R][8]) {
+  constexpr int AR = PassTile<R>::kActRow;
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+#pragma unroll 4
+  for (int k = 0; k < K; ++k) {
+    float a[R], b[8];
+    if constexpr (R == 4) *reinterpret_cast<float4 *>(a) = *reinterpret_cast<const float4 *>(act + k * AR + 4 * tm);
+    else *reinterpret_cast<float2 *>(a) = *reinterpret_cast<const float2 *>(act + k * AR + 2 * tm);
+    *reinterpret_cast<float4 *>(b) = *reinterpret_cast<const float4 *>(w + k * kWRow + 4 * tn);
+    *reinterpret_cast<float4 *>(b + 4) = *reinterpret_cast<const float4 *>(w + k * kWRow + 64 + 4 * tn);
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+  }
+}
+__device__ __forceinline__ int pass_col(int tn, int j) { return j < 4 ? 4 * tn + j : 60 + 4 * tn + j; }
+// the thread's values as the next product's operand, and to global memory when g is given
+template <int R>
+__device__ __forceinline__ void pass_store(const float (&v)[R][8], float *act, float *g, int m0, int n, int tm, int tn) {
+  constexpr int AR = PassTile<R>::kActRow;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+#pragma unroll
+    for (int i = 0; i < R; ++i) act[pass_col(tn, j) * AR + R * tm + i] = v[i][j];
+  if (!g) return;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int m = m0 + R * tm + i;
+    if (m >= n) continue;
+    float *row = g + (int64_t)m * kMlW;
+    *reinterpret_cast<float4 *>(row + 4 * tn) = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+    *reinterpret_cast<float4 *>(row + 64 + 4 * tn) = make_float4(v[i][4], v[i][5], v[i][6], v[i][7]);
+  }
+}
+// column sums over the tile's samples of the thread sums s, to dst (kMlW); red: 16 x kMlW
+__device__ __forceinline__ void pass_colsum(const float (&s)[8], float *red, float *dst, int tm, int tn) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) red[tm * kMlW + pass_col(tn, j)] = s[j];
+  __syncthreads();
+  if (threadIdx.x < kMlW) {
+    float t = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) t += red[q * kMlW + threadIdx.x];
+    dst[threadIdx.x] = t;
+  }
+  __syncthreads();
 }
 
-// C(m,n) = sum_k A(m,k) B(k,n) over strided operands, 64 x 64 tiles, 4 x 4 per thread,
-// K split over blockIdx.z in chunks of kchunk (partials at C + z * M * N, dense).
-// mode 0: C (+ bias[n]); 1: C = Z + bias[n] and H = silu(Z); 2: C *= silu'(Zp(m,n)).
-struct SgArgs {
-  const float *A, *B;
-  int64_t sAm, sAk, sBk, sBn;
-  int M, N, K;
-  float *C;
-  int64_t sCm, sCn;
-  const float *bias;
-  float *H;
-  const float *Zp;
-  int mode, kchunk;
-};
-
-__global__ void __launch_bounds__(256) k_sgemm(SgArgs g) {
-  constexpr int BM = 64, BN = 64, BK = 16;
-  __shared__ float As[BK][BM + 1];
-  __shared__ float Bs[BK][BN + 1];
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const int tid = threadIdx.x, tm = tid % 16, tn = tid / 16;
-  int kb = 0, ke = g.K;
-  if (g.kchunk > 0) {
-    kb = blockIdx.z * g.kchunk;
-    ke = min(g.K, kb + g.kchunk);
+template <int R>
+__global__ void __launch_bounds__(kPassThreads, 1) k_ml_pass(PassArgs g) {
+  extern __shared__ __align__(16) float psm[];
+  constexpr int AR = PassTile<R>::kActRow;
+  float *w0 = psm, *w1 = psm + kMlW * kWRow, *act = w1 + kMlW * kWRow, *red = act + kMlW * AR;
+  const int tid = threadIdx.x, tm = tid >> 4, tn = tid & 15;
+  const int m0 = blockIdx.x * PassTile<R>::kSamples;
+  const bool back = g.y != nullptr;
+  copy_weights(w0, g.pT + kPT1, kMlIn * kMlW);
+  copy_weights(w1, g.pT + kPT2, kMlW * kMlW);
+  for (int x = tid; x < PassTile<R>::kSamples * kMlIn; x += kPassThreads) {
+    const int m = x / kMlIn, k = x - m * kMlIn;
+    act[k * AR + m] = m0 + m < g.n ? g.X[(int64_t)m0 * kMlIn + x] : 0.0f;
   }
-  float acc[4][4];
+  float b[8];
+  auto bias = [&](int off) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 8; ++j) b[j] = g.p[off + pass_col(tn, j)];
+  };
+  float z1[R][8], z2[R][8], z3[R][8], v[R][8];
+  // pre-activations z to v = silu(z), and z replaced by silu'(z), which is all the way back needs
+  auto activate = [&](float (&z)[R][8]) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-  for (int k0 = kb; k0 < ke; k0 += BK) {
-    for (int x = tid; x < BM * BK; x += 256) {
-      const int m = x % BM, k = x / BM;
-      const int gm = m0 + m, gk = k0 + k;
-      As[k][m] = (gm < g.M && gk < ke) ? g.A[(int64_t)gm * g.sAm + (int64_t)gk * g.sAk] : 0.0f;
-    }
-    for (int x = tid; x < BK * BN; x += 256) {
-      const int n = x % BN, k = x / BN;
-      const int gn = n0 + n, gk = k0 + k;
-      Bs[k][n] = (gn < g.N && gk < ke) ? g.B[(int64_t)gk * g.sBk + (int64_t)gn * g.sBn] : 0.0f;
-    }
-    __syncthreads();
+    for (int i = 0; i < R; ++i)
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float a[4], b[4];
+      for (int j = 0; j < 8; ++j) {
+        const float x = z[i][j] + b[j], sg = sigm(x);
+        v[i][j] = x * sg;
+        z[i][j] = sg * (1.0f + x * (1.0f - sg));
+      }
+  };
+  // layer 1
+  bias(kMlOffB1);
+  __pipeline_wait_prior(1);
+  __syncthreads();
+  pass_product<R>(act, w0, kMlIn, tm, tn, z1);
+  activate(z1);
+  __syncthreads();  // act and w0 are read
+  copy_weights(w0, g.pT + kPT3, kMlW * kMlW);
+  pass_store<R>(v, act, back ? g.H1 : nullptr, m0, g.n, tm, tn);
+  // layer 2
+  bias(kMlOffB2);
+  __pipeline_wait_prior(1);
+  __syncthreads();
+  pass_product<R>(act, w1, kMlW, tm, tn, z2);
+  activate(z2);
+  __syncthreads();
+  if (back) copy_weights(w1, g.p + kMlOffW3, kMlW * kMlW);
+  pass_store<R>(v, act, back ? g.H2 : nullptr, m0, g.n, tm, tn);
+  // layer 3 and the output
+  bias(kMlOffB3);
+  if (back) __pipeline_wait_prior(1);
+  else __pipeline_wait_prior(0);
+  __syncthreads();
+  pass_product<R>(act, w0, kMlW, tm, tn, z3);
+  activate(z3);
+  __syncthreads();
+  if (back) copy_weights(w0, g.p + kMlOffW2, kMlW * kMlW);
+  float w4[8], dout[R];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][tm * 4 + i];
+  for (int j = 0; j < 8; ++j) w4[j] = g.p[kMlOffW4 + pass_col(tn, j)];
+  const float b4 = g.p[kMlOffB4];
+  double sq = 0.0;
+  float db4 = 0.0f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[k][tn * 4 + j];
+  for (int i = 0; i < R; ++i) {
+    float o = 0.0f;
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 8; ++j) o = fmaf(v[i][j], w4[j], o);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  float *C = g.C + (g.kchunk > 0 ? (int64_t)blockIdx.z * g.M * g.N : 0);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + tm * 4 + i;
-    if (m >= g.M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tn * 4 + j;
-      if (n >= g.N) continue;
-      const int64_t o = (int64_t)m * g.sCm + (int64_t)n * g.sCn;
-      float v = acc[i][j];
-      if (g.bias) v += g.bias[n];
-      if (g.mode == 1) {
-        C[o] = v;
-        g.H[o] = silu(v);
-      } else if (g.mode == 2) {
-        C[o] = v * dsilu(g.Zp[o]);
-      } else {
-        C[o] = v;
+    for (int q = 8; q > 0; q >>= 1) o += __shfl_xor_sync(0xffffffffu, o, q);  // the 16 threads of these samples
+    o += b4;
+    const int m = m0 + R * tm + i;
+    dout[i] = 0.0f;
+    if (m < g.n) {
+      if (back) {
+        const float d = o - g.y[m];
+        dout[i] = 2.0f * d / (float)g.n;
+        sq += (double)d * d;
+        db4 += dout[i];
+      } else if (tn == 0) {
+        g.out[m] = o;
       }
     }
   }
-}
-
-// out[i] = sum_z part[z * len + i], fixed order
-__global__ void k_ml_reduce(const float *__restrict__ part, int nz, int len, float *__restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) {
-    float s = 0.0f;
-    for (int z = 0; z < nz; ++z) s += part[(int64_t)z * len + i];
-    out[i] = s;
+  if (!back) return;
+  float *part = g.part + (int64_t)blockIdx.x * kPartLen;
+  // output layer: dw4 = H3^T dout, db4 = sum dout, and the loss; dZ3 = dout w4^T silu'(Z3)
+  float s[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    s[j] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < R; ++i) s[j] = fmaf(v[i][j], dout[i], s[j]);
   }
-}
-
-// dout = 2 (out - y) / n; loss partials per block
-__global__ void k_ml_dloss(const float *__restrict__ out, const float *__restrict__ y, int n, float *__restrict__ dout,
-                           double *__restrict__ part) {
-  __shared__ double sh[256];
-  double s = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const float d = out[i] - y[i];
-    dout[i] = 2.0f * d / (float)n;
-    s += (double)d * d;
+  pass_colsum(s, red, part + 3 * kMlW, tm, tn);
+  if (tn == 0) {  // one thread per sample group
+    red[tm] = db4;
+    reinterpret_cast<double *>(red + 32)[tm] = sq;
   }
-  sh[threadIdx.x] = s;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
+  if (tid == 0) {
+    float t = 0.0f;
+    double l = 0.0;
+    for (int q = 0; q < 16; ++q) {
+      t += red[q];
+      l += reinterpret_cast<double *>(red + 32)[q];
+    }
+    part[4 * kMlW] = t;
+    g.loss[blockIdx.x] = l;
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+  __syncthreads();
+  auto difference = [&](const float (&dz)[R][8], float *dst, float *db) {  // v * silu': to dst, its column sums to db
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      s[j] = 0.0f;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        v[i][j] *= dz[i][j];
+        s[j] += v[i][j];
+      }
+    }
+    pass_store<R>(v, act, dst, m0, g.n, tm, tn);
+    pass_colsum(s, red, db, tm, tn);
+  };
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[i][j] = dout[i] * w4[j];
+  difference(z3, g.D3, part + 2 * kMlW);
+  // dZ2 = (dZ3 W3) silu'(Z2), dZ1 = (dZ2 W2) silu'(Z1)
+  __pipeline_wait_prior(1);
+  __syncthreads();
+  pass_product<R>(act, w1, kMlW, tm, tn, v);
+  __syncthreads();
+  difference(z2, g.D2, part + kMlW);
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  pass_product<R>(act, w0, kMlW, tm, tn, v);
+  __syncthreads();
+  difference(z1, g.D1, part);
 }
-__global__ void k_ml_loss_finish(const double *__restrict__ part, int nb, int n, double *__restrict__ loss) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int i = 0; i < nb; ++i) s += part[i];
-    *loss = s / n;
+
+// Weight gradients dW(o, k) = sum_m D(m, o) H(m, k), one slice of the samples a block
+// (blockIdx.y: W3, W2, W1), 8 x 8 outputs a thread (W1: 8 x 2 of its 18 columns, padded), to
+// the slice's partial sums in the parameters' order.
+constexpr int kGradK = 16;      // samples staged at a time
+constexpr int kGradStages = 3;  // stages in flight: a stage's FMAs take about as long as its loads
+struct WgradArgs {
+  const float *X, *H1, *H2, *D1, *D2, *D3;
+  int n, per;              // samples, samples of a slice (a multiple of kGradK)
+  float *part;             // per slice: W1, W2, W3
+};
+constexpr int kGradLen = kMlIn * kMlW + 2 * kMlW * kMlW;
+__global__ void __launch_bounds__(256) k_ml_wgrad(WgradArgs g) {
+  __shared__ __align__(16) float As[kGradStages][kGradK][kMlW], Bs[kGradStages][kGradK][kMlW];
+  const int which = blockIdx.y;  // 0: W3, 1: W2, 2: W1
+  const float *A = which == 0 ? g.D3 : which == 1 ? g.D2 : g.D1;
+  const float *B = which == 0 ? g.H2 : which == 1 ? g.H1 : g.X;
+  const int nb = which == 2 ? kMlIn : kMlW;
+  const int tid = threadIdx.x, tm = tid >> 4, tn = tid & 15;
+  const int beg = blockIdx.x * g.per, end = min(g.n, beg + g.per);
+  auto stage = [&](int s, int m) {
+    for (int x = 4 * tid; x < kGradK * kMlW; x += 4 * 256) {
+      const int r = x / kMlW, c = x % kMlW;
+      if (m + r < end) {
+        __pipeline_memcpy_async(&As[s][r][c], A + (int64_t)(m + r) * kMlW + c, 16);
+        if (which != 2) __pipeline_memcpy_async(&Bs[s][r][c], B + (int64_t)(m + r) * kMlW + c, 16);
+      } else {
+        *reinterpret_cast<float4 *>(&As[s][r][c]) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (which != 2) *reinterpret_cast<float4 *>(&Bs[s][r][c]) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+    }
+    if (which == 2)
+      for (int x = tid; x < kGradK * 32; x += 256) {
+        const int r = x >> 5, c = x & 31;
+        Bs[s][r][c] = m + r < end && c < kMlIn ? B[(int64_t)(m + r) * kMlIn + c] : 0.0f;
+      }
+    __pipeline_commit();
+  };
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+  // every iteration commits a group (an empty one past the end), so that the groups count stages
+  for (int q = 0; q < kGradStages - 1; ++q) {
+    if (beg + q * kGradK < end) stage(q, beg + q * kGradK);
+    else __pipeline_commit();
+  }
+  int s = 0;
+  for (int m = beg; m < end; m += kGradK, s = s + 1 == kGradStages ? 0 : s + 1) {
+    __pipeline_wait_prior(kGradStages - 2);
+    __syncthreads();  // this stage is in place, and the one before it is read
+    const int mn = m + (kGradStages - 1) * kGradK, sn = s == 0 ? kGradStages - 1 : s - 1;
+    if (mn < end) stage(sn, mn);
+    else __pipeline_commit();
+#pragma unroll
+    for (int k = 0; k < kGradK; ++k) {
+      float a[8], b[8];
+      *reinterpret_cast<float4 *>(a) = *reinterpret_cast<const float4 *>(&As[s][k][4 * tm]);
+      *reinterpret_cast<float4 *>(a + 4) = *reinterpret_cast<const float4 *>(&As[s][k][64 + 4 * tm]);
+      if (which != 2) {
+        *reinterpret_cast<float4 *>(b) = *reinterpret_cast<const float4 *>(&Bs[s][k][4 * tn]);
+        *reinterpret_cast<float4 *>(b + 4) = *reinterpret_cast<const float4 *>(&Bs[s][k][64 + 4 * tn]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      } else {
+        *reinterpret_cast<float2 *>(b) = *reinterpret_cast<const float2 *>(&Bs[s][k][2 * tn]);
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+      }
+    }
+  }
+  float *out = g.part + (int64_t)blockIdx.x * kGradLen +
+               (which == 2 ? 0 : kMlIn * kMlW + (which == 1 ? 0 : kMlW * kMlW));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float *row = out + pass_col(tm, i) * nb;
+    if (which != 2) {
+      *reinterpret_cast<float4 *>(row + 4 * tn) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+      *reinterpret_cast<float4 *>(row + 64 + 4 * tn) = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
+    } else if (2 * tn < kMlIn) {
+      *reinterpret_cast<float2 *>(row + 2 * tn) = make_float2(acc[i][0], acc[i][1]);
+    }
   }
 }
 
-__global__ void k_ml_adam(float *__restrict__ p, float *__restrict__ m, float *__restrict__ v, const float *__restrict__ g,
-                          int n, float lr, float b1t, float b2t) {
+// the gradient in the parameters' order from the partial sums of the slices (weights) and of
+// the tiles (biases, output layer), each in order; the last block finishes the loss
+__global__ void __launch_bounds__(256) k_ml_grad(const float *__restrict__ wpart, int slices, const float *__restrict__ bpart,
+                                                 const double *__restrict__ lpart, int tiles, int n, float *__restrict__ grad,
+                                                 double *__restrict__ loss) {
+  if (blockIdx.x == gridDim.x - 1) {
+    __shared__ double sh[256];
+    double s = 0.0;
+    for (int t = threadIdx.x; t < tiles; t += 256) s += lpart[t];
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) *loss = sh[0] / n;
+    return;
+  }
+  // 32 parameters a block, eight threads each: short chains of loads, and the rounding of a
+  // few dozen additions in a row instead of a few hundred
+  __shared__ float red[8][32];
+  const int q = threadIdx.x >> 5, i = blockIdx.x * 32 + (threadIdx.x & 31);
+  const float *src = bpart;
+  int64_t step = kPartLen;
+  int cnt = i < kMlParams ? tiles : 0;
+  if (i < kMlOffB1) { src = wpart + i; step = kGradLen; cnt = slices; }
+  else if (i < kMlOffW2) src += i - kMlOffB1;
+  else if (i < kMlOffB2) { src = wpart + kMlIn * kMlW + (i - kMlOffW2); step = kGradLen; cnt = slices; }
+  else if (i < kMlOffW3) src += kMlW + (i - kMlOffB2);
+  else if (i < kMlOffB3) { src = wpart + kMlIn * kMlW + kMlW * kMlW + (i - kMlOffW3); step = kGradLen; cnt = slices; }
+  else if (i < kMlOffW4) src += 2 * kMlW + (i - kMlOffB3);
+  else src += 3 * kMlW + (i - kMlOffW4);
+  float s = 0.0f;
+#pragma unroll 8
+  for (int z = q; z < cnt; z += 8) s += src[z * step];
+  red[q][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (q == 0 && i < kMlParams) {
+    const int l = threadIdx.x;
+    grad[i] = ((red[0][l] + red[1][l]) + (red[2][l] + red[3][l])) + ((red[4][l] + red[5][l]) + (red[6][l] + red[7][l]));
+  }
+}
+
+// index of parameter i in the transposed weights, or -1 (biases, output layer)
+__device__ __forceinline__ int transposed_index(int i) {
+  if (i < kMlOffB1) return kPT1 + (i % kMlIn) * kMlW + i / kMlIn;
+  if (i >= kMlOffW2 && i < kMlOffB2) { const int x = i - kMlOffW2; return kPT2 + (x % kMlW) * kMlW + x / kMlW; }
+  if (i >= kMlOffW3 && i < kMlOffB3) { const int x = i - kMlOffW3; return kPT3 + (x % kMlW) * kMlW + x / kMlW; }
+  return -1;
+}
+__global__ void k_ml_transpose(const float *__restrict__ p, float *__restrict__ pT) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kMlParams) return;
+  const int t = transposed_index(i);
+  if (t >= 0) pT[t] = p[i];
+}
+
+__global__ void k_ml_adam(float *__restrict__ p, float *__restrict__ pT, float *__restrict__ m, float *__restrict__ v,
+                          const float *__restrict__ g, int n, float lr, float b1t, float b2t) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float gi = g[i];
@@ -302,15 +561,15 @@ __global__ void k_ml_adam(float *__restrict__ p, float *__restrict__ m, float *_
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / (1.0f - b1t)) / (sqrtf(vi / (1.0f - b2t)) + eps);
+    const float x = p[i] - lr * (mi / (1.0f - b1t)) / (sqrtf(vi / (1.0f - b2t)) + eps);
+    p[i] = x;
+    const int t = transposed_index(i);
+    if (t >= 0) pT[t] = x;
   }
 }
 
 __global__ void k_ml_scale(float *__restrict__ x, int64_t n, float s) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] *= s;
-}
-__global__ void k_ml_fill(float *__restrict__ x, int64_t n, float v) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) x[i] = v;
 }
 
 // ---------------------------------------------------------------- BF16 tensor-core inference
@@ -535,7 +794,9 @@ class Learner final : public ILearner {
     params_.alloc(kMlParams * 4);
     m_.alloc(kMlParams * 4);
     v_.alloc(kMlParams * 4);
-    grad_.alloc(kMlParams * 4);
+    grad_.alloc(kGradLoss + 8);
+    pT_.alloc(kPTLen * 4);
+    lck(cudaMallocHost(&host_grad_, kGradLoss + 8), "cudaMallocHost (learner)");
     wt_.alloc(kWBytes);
     err_.alloc(4);
     lck(cudaMemset(err_.p, 0, 4), "memset");
@@ -562,6 +823,7 @@ class Learner final : public ILearner {
   }
   ~Learner() override {
     if (st_) cudaStreamDestroy(st_);
+    if (host_grad_) cudaFreeHost(host_grad_);
   }
 
   void add_solution(const MLView &v, int stride) override {
@@ -659,8 +921,9 @@ class Learner final : public ILearner {
       forward_backward(Xs.as<float>() + off * kMlIn, ys.as<float>() + off, batch, lossd.as<double>() + s);
       ++t_;
       const float b1t = (float)std::pow(0.9, (double)t_), b2t = (float)std::pow(0.999, (double)t_);
-      k_ml_adam<<<(kMlParams + 255) / 256, 256, 0, st_>>>(params_.as<float>(), m_.as<float>(), v_.as<float>(),
-                                                           grad_.as<float>(), kMlParams, (float)lr, b1t, b2t);
+      k_ml_adam<<<(kMlParams + 255) / 256, 256, 0, st_>>>(params_.as<float>(), pT_.as<float>(), m_.as<float>(),
+                                                           v_.as<float>(), grad_.as<float>(), kMlParams, (float)lr, b1t,
+                                                           b2t);
     }
     // the output layer back in the targets' units (the Adam moments stay with the
     // standardised units of the next training)
@@ -695,6 +958,9 @@ class Learner final : public ILearner {
   }
   void set_params(const float *p) override {
     lck(cudaMemcpy(params_.p, p, kMlParams * 4, cudaMemcpyHostToDevice), "params");
+    k_ml_transpose<<<(kMlParams + 255) / 256, 256, 0, st_>>>(params_.as<float>(), pT_.as<float>());
+    lck(cudaGetLastError(), "params");
+    lck(cudaStreamSynchronize(st_), "params");
     folded_ = true;  // parameters from get_params: output layer in the targets' units
     lck(cudaMemset(m_.p, 0, kMlParams * 4), "adam");
     lck(cudaMemset(v_.p, 0, kMlParams * 4), "adam");
@@ -705,32 +971,29 @@ class Learner final : public ILearner {
   void loss_grad(const float *X, const float *y, int n, double *loss, float *grad) override {
     lck(cudaSetDevice(device_), "cudaSetDevice");
     if (n < 1) throw EngineError(1, "learner: empty batch");
-    LBuf dX, dy, dl;
-    dX.alloc((size_t)n * kMlIn * 4);
-    dy.alloc((size_t)n * 4);
-    dl.alloc(8);
-    lck(cudaMemcpy(dX.p, X, (size_t)n * kMlIn * 4, cudaMemcpyHostToDevice), "copy");
-    lck(cudaMemcpy(dy.p, y, (size_t)n * 4, cudaMemcpyHostToDevice), "copy");
     ensure_batch(n);
-    forward_backward(dX.as<float>(), dy.as<float>(), n, dl.as<double>());
+    ensure_io(n);
+    lck(cudaMemcpyAsync(ioX_.p, X, (size_t)n * kMlIn * 4, cudaMemcpyHostToDevice, st_), "copy");
+    lck(cudaMemcpyAsync(ioy_.p, y, (size_t)n * 4, cudaMemcpyHostToDevice, st_), "copy");
+    // the gradient and the loss behind it in one copy
+    forward_backward(ioX_.as<float>(), ioy_.as<float>(), n, (double *)(grad_.as<char>() + kGradLoss));
+    lck(cudaMemcpyAsync(host_grad_, grad_.p, kGradLoss + 8, cudaMemcpyDeviceToHost, st_), "copy");
     lck(cudaStreamSynchronize(st_), "loss_grad");
-    lck(cudaMemcpy(loss, dl.p, 8, cudaMemcpyDeviceToHost), "copy");
-    lck(cudaMemcpy(grad, grad_.p, kMlParams * 4, cudaMemcpyDeviceToHost), "copy");
+    std::memcpy(grad, host_grad_, kMlParams * 4);
+    std::memcpy(loss, host_grad_ + kGradLoss, 8);
   }
 
   void infer(const float *X, int n, float *out, int tensor_cores) override {
     lck(cudaSetDevice(device_), "cudaSetDevice");
     if (n < 1) return;
-    LBuf dX, dout;
-    dX.alloc((size_t)n * kMlIn * 4);
-    dout.alloc((size_t)n * 4);
-    lck(cudaMemcpy(dX.p, X, (size_t)n * kMlIn * 4, cudaMemcpyHostToDevice), "copy");
+    ensure_io(n);
+    lck(cudaMemcpyAsync(ioX_.p, X, (size_t)n * kMlIn * 4, cudaMemcpyHostToDevice, st_), "copy");
     if (tensor_cores) {
       upload_weight_tiles();
       InferArgs a{};
       a.use_view = 0;
-      a.X = dX.as<float>();
-      a.out = dout.as<float>();
+      a.X = ioX_.as<float>();
+      a.out = ioy_.as<float>();
       a.n = n;
       a.wt = wt_.as<uint8_t>();
       a.par = params_.as<float>();
@@ -738,12 +1001,17 @@ class Learner final : public ILearner {
       a.err = err_.as<int>();
       run_infer(a, st_);
     } else {
-      ensure_batch(n);
-      forward(dX.as<float>(), n);
-      lck(cudaMemcpyAsync(dout.p, out_.p, (size_t)n * 4, cudaMemcpyDeviceToDevice, st_), "copy");
+      PassArgs a{};
+      a.X = ioX_.as<float>();
+      a.n = n;
+      a.p = params_.as<float>();
+      a.pT = pT_.as<float>();
+      a.out = ioy_.as<float>();
+      run_pass(a);
     }
+    lck(cudaGetLastError(), "infer");
+    lck(cudaMemcpyAsync(out, ioy_.p, (size_t)n * 4, cudaMemcpyDeviceToHost, st_), "copy");
     lck(cudaStreamSynchronize(st_), "infer");
-    lck(cudaMemcpy(out, dout.p, (size_t)n * 4, cudaMemcpyDeviceToHost), "copy");
   }
 
  private:
@@ -762,73 +1030,60 @@ class Learner final : public ILearner {
     return c;
   }
 
+  // Workspaces grow to the largest batch seen and are freed with the learner.
   void ensure_batch(int b) {
     if (b <= cap_) return;
+    cap_ = 0;
+    for (LBuf *x : {&H1_, &H2_, &D1_, &D2_, &D3_}) x->alloc((size_t)b * kMlW * 4);
+    const int tiles = (b + PassTile<2>::kSamples - 1) / PassTile<2>::kSamples;
+    bpart_.alloc((size_t)tiles * kPartLen * 4);
+    lpart_.alloc((size_t)tiles * 8);
+    wpart_.alloc((size_t)kGradSlices * kGradLen * 4);
     cap_ = b;
-    for (LBuf *x : {&Z1_, &H1_, &Z2_, &H2_, &Z3_, &H3_, &dZ_, &dZb_}) x->alloc((size_t)b * kMlW * 4);
-    out_.alloc((size_t)b * 4);
-    dout_.alloc((size_t)b * 4);
-    ones_.alloc((size_t)b * 4);
-    k_ml_fill<<<256, 256, 0, st_>>>(ones_.as<float>(), b, 1.0f);
-    nsplit_max_ = (b + kSplitK - 1) / kSplitK;
-    part_.alloc((size_t)nsplit_max_ * kMlW * kMlW * 4);
-    lpart_.alloc(256 * 8);
-    lck(cudaGetLastError(), "learner buffers");
+  }
+  void ensure_io(int n) {
+    if (n <= io_cap_) return;
+    io_cap_ = 0;
+    ioX_.alloc((size_t)n * kMlIn * 4);
+    ioy_.alloc((size_t)n * 4);
+    io_cap_ = n;
   }
 
-  void sgemm(const float *A, int64_t sAm, int64_t sAk, const float *B, int64_t sBk, int64_t sBn, int M, int N, int K,
-             float *C, int64_t sCm, int64_t sCn, const float *bias, float *H, const float *Zp, int mode) {
-    SgArgs g{A, B, sAm, sAk, sBk, sBn, M, N, K, C, sCm, sCn, bias, H, Zp, mode, 0};
-    dim3 grid((M + 63) / 64, (N + 63) / 64, 1);
-    k_sgemm<<<grid, 256, 0, st_>>>(g);
+  // Tiles of 64 samples, or of 32 while that many leave SMs without one (a tile's time is
+  // latency and FMAs of one SM, so half the samples take half of it): 8192 samples 143 us a call in
+  // tiles of 64 and 169 of 32, 4096 samples 128 and 115.
+  int run_pass(const PassArgs &a) {
+    return a.n <= 152 * PassTile<2>::kSamples ? run_tiles<2>(a) : run_tiles<4>(a);
   }
-  // C (dense M x N, row-major) = sum over a long K with split-K partials
-  void sgemm_long(const float *A, int64_t sAm, int64_t sAk, const float *B, int64_t sBk, int64_t sBn, int M, int N, int K,
-                  float *C) {
-    const int nz = (K + kSplitK - 1) / kSplitK;
-    SgArgs g{A, B, sAm, sAk, sBk, sBn, M, N, K, part_.as<float>(), N, 1, nullptr, nullptr, nullptr, 0, kSplitK};
-    dim3 grid((M + 63) / 64, (N + 63) / 64, nz);
-    k_sgemm<<<grid, 256, 0, st_>>>(g);
-    k_ml_reduce<<<(M * N + 255) / 256, 256, 0, st_>>>(part_.as<float>(), nz, M * N, C);
-  }
-
-  void forward(const float *X, int n) {
-    const float *p = params_.as<float>();
-    sgemm(X, kMlIn, 1, p + kMlOffW1, 1, kMlIn, n, kMlW, kMlIn, Z1_.as<float>(), kMlW, 1, p + kMlOffB1, H1_.as<float>(),
-          nullptr, 1);
-    sgemm(H1_.as<float>(), kMlW, 1, p + kMlOffW2, 1, kMlW, n, kMlW, kMlW, Z2_.as<float>(), kMlW, 1, p + kMlOffB2,
-          H2_.as<float>(), nullptr, 1);
-    sgemm(H2_.as<float>(), kMlW, 1, p + kMlOffW3, 1, kMlW, n, kMlW, kMlW, Z3_.as<float>(), kMlW, 1, p + kMlOffB3,
-          H3_.as<float>(), nullptr, 1);
-    sgemm(H3_.as<float>(), kMlW, 1, p + kMlOffW4, 1, 0, n, 1, kMlW, out_.as<float>(), 1, 1, p + kMlOffB4, nullptr,
-          nullptr, 0);
+  template <int R>
+  int run_tiles(const PassArgs &a) {
+    const int tiles = (a.n + PassTile<R>::kSamples - 1) / PassTile<R>::kSamples;
+    lck(cudaFuncSetAttribute(k_ml_pass<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassTile<R>::kSmem),
+        "attribute");
+    k_ml_pass<R><<<tiles, kPassThreads, PassTile<R>::kSmem, st_>>>(a);
+    return tiles;
   }
 
   void forward_backward(const float *X, const float *y, int n, double *loss) {
-    const float *p = params_.as<float>();
-    float *gr = grad_.as<float>();
-    forward(X, n);
-    const int nb = std::min(256, (n + 255) / 256);
-    k_ml_dloss<<<nb, 256, 0, st_>>>(out_.as<float>(), y, n, dout_.as<float>(), lpart_.as<double>());
-    k_ml_loss_finish<<<1, 32, 0, st_>>>(lpart_.as<double>(), nb, n, loss);
-    // output layer: dw4 = H3^T dout, db4 = sum dout, dZ3 = (dout w4^T) * silu'(Z3)
-    sgemm_long(H3_.as<float>(), 1, kMlW, dout_.as<float>(), 1, 1, kMlW, 1, n, gr + kMlOffW4);
-    sgemm_long(dout_.as<float>(), 0, 1, ones_.as<float>(), 1, 1, 1, 1, n, gr + kMlOffB4);
-    sgemm(dout_.as<float>(), 1, 0, p + kMlOffW4, 0, 1, n, kMlW, 1, dZ_.as<float>(), kMlW, 1, nullptr, nullptr,
-          Z3_.as<float>(), 2);
-    // layer 3: dW3 = dZ3^T H2, db3, dZ2 = (dZ3 W3) * silu'(Z2)
-    sgemm_long(dZ_.as<float>(), 1, kMlW, H2_.as<float>(), kMlW, 1, kMlW, kMlW, n, gr + kMlOffW3);
-    sgemm_long(dZ_.as<float>(), 1, kMlW, ones_.as<float>(), 1, 1, kMlW, 1, n, gr + kMlOffB3);
-    sgemm(dZ_.as<float>(), kMlW, 1, p + kMlOffW3, kMlW, 1, n, kMlW, kMlW, dZb_.as<float>(), kMlW, 1, nullptr, nullptr,
-          Z2_.as<float>(), 2);
-    // layer 2
-    sgemm_long(dZb_.as<float>(), 1, kMlW, H1_.as<float>(), kMlW, 1, kMlW, kMlW, n, gr + kMlOffW2);
-    sgemm_long(dZb_.as<float>(), 1, kMlW, ones_.as<float>(), 1, 1, kMlW, 1, n, gr + kMlOffB2);
-    sgemm(dZb_.as<float>(), kMlW, 1, p + kMlOffW2, kMlW, 1, n, kMlW, kMlW, dZ_.as<float>(), kMlW, 1, nullptr, nullptr,
-          Z1_.as<float>(), 2);
-    // layer 1
-    sgemm_long(dZ_.as<float>(), 1, kMlW, X, kMlIn, 1, kMlW, kMlIn, n, gr + kMlOffW1);
-    sgemm_long(dZ_.as<float>(), 1, kMlW, ones_.as<float>(), 1, 1, kMlW, 1, n, gr + kMlOffB1);
+    PassArgs a{};
+    a.X = X;
+    a.y = y;
+    a.n = n;
+    a.p = params_.as<float>();
+    a.pT = pT_.as<float>();
+    a.H1 = H1_.as<float>(); a.H2 = H2_.as<float>();
+    a.D1 = D1_.as<float>(); a.D2 = D2_.as<float>(); a.D3 = D3_.as<float>();
+    a.part = bpart_.as<float>();
+    a.loss = lpart_.as<double>();
+    const int tiles = run_pass(a);
+    // as many slices as fill the SMs with the two large gradients, of at least 64 samples
+    const int want = std::max(1, std::min(kGradSlices, n / 64));
+    const int per = ((n + want - 1) / want + kGradK - 1) / kGradK * kGradK, slices = (n + per - 1) / per;
+    const WgradArgs w{X, a.H1, a.H2, a.D1, a.D2, a.D3, n, per, wpart_.as<float>()};
+    k_ml_wgrad<<<dim3(slices, 3), 256, 0, st_>>>(w);
+    k_ml_grad<<<(kMlParams + 31) / 32 + 1, 256, 0, st_>>>(wpart_.as<float>(), slices, bpart_.as<float>(),
+                                                            lpart_.as<double>(), tiles, n, grad_.as<float>(), loss);
+    lck(cudaGetLastError(), "training pass");
   }
 
   void upload_weight_tiles() {
@@ -867,12 +1122,14 @@ class Learner final : public ILearner {
     }
   }
 
-  static constexpr int kSplitK = 512;
+  static constexpr int kGradSlices = 76;
+  static constexpr size_t kGradLoss = (kMlParams * 4 + 7) / 8 * 8;  // byte offset of the loss behind the gradient
   int device_ = 0;
   cudaStream_t st_ = nullptr;
-  LBuf params_, m_, v_, grad_, wt_, err_;
-  LBuf Z1_, H1_, Z2_, H2_, Z3_, H3_, dZ_, dZb_, out_, dout_, ones_, part_, lpart_;
-  int cap_ = 0, nsplit_max_ = 0;
+  LBuf params_, pT_, m_, v_, grad_, wt_, err_;
+  LBuf H1_, H2_, D1_, D2_, D3_, bpart_, wpart_, lpart_, ioX_, ioy_;
+  char *host_grad_ = nullptr;  // page-locked: gradient and loss of loss_grad
+  int cap_ = 0, io_cap_ = 0;
   int64_t t_ = 0;
   bool weights_dirty_ = true;
   std::vector<Chunk> data_;
