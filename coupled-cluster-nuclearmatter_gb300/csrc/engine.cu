@@ -435,12 +435,12 @@ class Engine final : public IEngine {
       }
       case 2:
         check_ch(ch, L.fam[2].count());
-        if (!tr_) tr_ = make_triples<S>(*L_, D_, O_, device_);
+        if (!tr_) tr_ = make_triples<S>(*L_, O_, device_);
         tr_->set_hhhp(ch, v, st_);
         return;
       case 5:
         check_ch(ch, L.fam[5].count());
-        if (!tr_) tr_ = make_triples<S>(*L_, D_, O_, device_);
+        if (!tr_) tr_ = make_triples<S>(*L_, O_, device_);
         tr_->set_hppp(ch, v, st_);
         return;
       default:
@@ -750,7 +750,7 @@ class Engine final : public IEngine {
 
   void triples(double et[2]) override {
     require_ready();
-    if (!tr_) tr_ = make_triples<S>(*L_, D_, O_, device_);
+    if (!tr_) tr_ = make_triples<S>(*L_, O_, device_);
     if (!tr_->has_v()) {
       if (!generated_) throw EngineError(4, "(T) needs V_hhhp and V_hppp: set every HHHP and HPPP block, or generate the interaction");
       tr_->generate_v(pot_, st_);

@@ -25,10 +25,9 @@ class ITriples {
   // (n_t packed elements) and V; the |W|^2 / D accumulation is FP64 either way
   virtual void energy(const S *T, int64_t n_t, const S *fdiag, double et[2], cudaStream_t st, bool fp32) = 0;
   virtual int64_t launches() const = 0;
-  virtual int64_t count() const = 0;  // number of (abc, ijk) pairs
 };
 
 template <typename S>
-std::unique_ptr<ITriples<S>> make_triples(const Layout &L, const DevLayout &D, const DevOrbits &O, int device);
+std::unique_ptr<ITriples<S>> make_triples(const Layout &L, const DevOrbits &O, int device);
 
 }  // namespace ccx
