@@ -104,6 +104,10 @@ void upload(DBuf &d, const std::vector<T> &h, int64_t *counter) {
   if (!h.empty()) CK(cudaMemcpy(d.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
 }
 
+// Uploads and the zeroing of new buffers run on the legacy stream, which the engine's own
+// (non-blocking) streams do not wait for: set-up ends with this before they use the buffers.
+void settle() { CK(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 uint64_t splitmix(uint64_t &st) {
   uint64_t z = (st += 0x9e3779b97f4a7c15ULL);
   z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
@@ -206,6 +210,7 @@ class Engine final : public IEngine {
     // where each packed amplitude's one-body and ring terms come from (layout only)
     omap_.alloc(std::max<int64_t>(n_t_, 1) * sizeof(int4), &bytes_);
     rmap_.alloc(std::max<int64_t>(n_t_, 1) * sizeof(int4), &bytes_);
+    settle();
     launch_rinit_maps(D_, omap_.as<int4>(), rmap_.as<int4>(), st_);
     CK(cudaStreamSynchronize(st_));
   }
@@ -256,6 +261,7 @@ class Engine final : public IEngine {
     CK(cudaMemcpy(fdiag_.p, fd.data(), ns * sizeof(S), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(f6_.p, f6.data(), f6.size() * sizeof(S), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(f7_.p, f7.data(), f7.size() * sizeof(S), cudaMemcpyHostToDevice));
+    settle();
     e0_[0] = e0 ? e0[0] : 0.0;
     e0_[1] = e0 ? e0[1] : 0.0;
     have_fock_ = true;
@@ -515,6 +521,7 @@ class Engine final : public IEngine {
     }
     DBuf dp;
     upload(dp, pairs, nullptr);
+    settle();
     for (int ch = 0; ch < F.count(); ++ch) {
       const int n = F.side1[ch].size();
       if (n <= 0) continue;
@@ -559,6 +566,7 @@ class Engine final : public IEngine {
       DBuf dr, dc;
       upload(dr, r, nullptr);
       upload(dc, c, nullptr);
+      settle();
       launch_gen_ordered<S>(O_, pot_, dr.as<int2>(), dc.as<int2>(), nr, nc, kind == 5 ? 1 : 0, stage_.as<double>(), st_);
       ++launches_;
       CK(cudaMemcpyAsync(v, stage_.p, bytes, cudaMemcpyDeviceToHost, st_));
@@ -1261,6 +1269,7 @@ class Engine final : public IEngine {
     finalize_plan(P.ladder, bl);
     finalize_plan(P.x_i4, bx4);
     finalize_plan(P.ring_ladder, brl);
+    settle();
   }
 
   // Autotuner of the grouped FP64 GEMM: for each N bucket, time the residual's two product
@@ -2280,6 +2289,7 @@ class Engine final : public IEngine {
     finalize_oz(ozHH_, lhh);
     finalize_oz(ozI4_, l4);
     finalize_oz(ozRing_, lr);
+    settle();
     run_oz_split(ozsV_);
     CK(cudaStreamSynchronize(st_));
     oz_ready_ = true;
@@ -2447,6 +2457,7 @@ class Engine final : public IEngine {
       upload(gplan_.chunks, ch, &bytes_);
       upload(gplan_.jobs, gjobs, &bytes_);
       gplan_.nchunks = (int)ch.size();
+      settle();
       launch_tc_build_map(tc_kind_, (const TcMapJob *)mj.p, (const int4 *)gplan_.chunks.p, gplan_.nchunks, st_);
       CK(cudaStreamSynchronize(st_));  // the map job table goes out of scope
     }
@@ -2483,6 +2494,7 @@ class Engine final : public IEngine {
       finalize_plan(planHH_, bh);
     }
     commit();
+    settle();
     run_split(spStatic_);
     CK(cudaStreamSynchronize(st_));
     mixed_ready_ = true;

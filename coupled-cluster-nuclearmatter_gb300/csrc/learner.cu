@@ -799,7 +799,7 @@ class Learner final : public ILearner {
     lck(cudaMallocHost(&host_grad_, kGradLoss + 8), "cudaMallocHost (learner)");
     wt_.alloc(kWBytes);
     err_.alloc(4);
-    lck(cudaMemset(err_.p, 0, 4), "memset");
+    lck(cudaMemsetAsync(err_.p, 0, 4, st_), "memset");
     // Kaiming-uniform initial weights from splitmix64, zero biases, small output layer
     std::vector<float> p(kMlParams, 0.0f);
     uint64_t s = seed;
@@ -957,13 +957,15 @@ class Learner final : public ILearner {
     lck(cudaMemcpy(p, params_.p, kMlParams * 4, cudaMemcpyDeviceToHost), "params");
   }
   void set_params(const float *p) override {
-    lck(cudaMemcpy(params_.p, p, kMlParams * 4, cudaMemcpyHostToDevice), "params");
+    // on the learner's own stream, as all that reads them; waited for, since the engines' streams
+    // read them too
+    lck(cudaMemcpyAsync(params_.p, p, kMlParams * 4, cudaMemcpyHostToDevice, st_), "params");
+    lck(cudaMemsetAsync(m_.p, 0, kMlParams * 4, st_), "adam");
+    lck(cudaMemsetAsync(v_.p, 0, kMlParams * 4, st_), "adam");
     k_ml_transpose<<<(kMlParams + 255) / 256, 256, 0, st_>>>(params_.as<float>(), pT_.as<float>());
     lck(cudaGetLastError(), "params");
     lck(cudaStreamSynchronize(st_), "params");
     folded_ = true;  // parameters from get_params: output layer in the targets' units
-    lck(cudaMemset(m_.p, 0, kMlParams * 4), "adam");
-    lck(cudaMemset(v_.p, 0, kMlParams * 4), "adam");
     t_ = 0;
     weights_dirty_ = true;
   }
@@ -1102,7 +1104,8 @@ class Learner final : public ILearner {
         put(3 * kWTile, o, k, p[kMlOffW3 + o * kMlW + k]);
       }
     }
-    lck(cudaMemcpy(wt_.p, w.data(), kWBytes, cudaMemcpyHostToDevice), "weight tiles");
+    lck(cudaMemcpyAsync(wt_.p, w.data(), kWBytes, cudaMemcpyHostToDevice, st_), "weight tiles");
+    lck(cudaStreamSynchronize(st_), "weight tiles");  // read on the engine's stream
     weights_dirty_ = false;
   }
 
