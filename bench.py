@@ -237,7 +237,7 @@ def hbm_peak():
         return FALLBACK_HBM_GBS, "fallback 6.8 TB/s (of fallback)"
 
 
-def kernel_work(P, H, ring, precision, real=True):
+def kernel_work(P, H, ring, precision, real=True, planes=9):
     """Algorithmic work of one timed bracket per kernel slot: ('flop', F) or ('byte', B),
     and the bytes of the operand representation the kernel actually streams.
 
@@ -246,8 +246,8 @@ def kernel_work(P, H, ring, precision, real=True):
     below the BF16 ridge): their algorithmic bytes are the FP64 (or complex FP64)
     elements of every matrix the product reads, once, and of C written once, e = 8 (16)
     bytes per element.  The representation the kernel streams instead -- BF16 (TF32)
-    hi/lo halves or the 9 BF16 digit planes of the exact digit products -- is returned
-    beside it, so that the report can show both."""
+    hi/lo halves or the BF16 digit planes of the exact digit products (`planes` of them) --
+    is returned beside it, so that the report can show both."""
     e = 8.0 if real else 16.0
     nc = 1 if real else 2                     # real components per element
     mac = 2.0 if real else 8.0
@@ -274,16 +274,16 @@ def kernel_work(P, H, ring, precision, real=True):
     r_rg = nc * 2 * 2 * es * (PHr + HP2) + e * PHr
     # digit products at a re-base: A, B read once, C written once
     a_oz = e * (P2 + 2 * PH)
-    r_oz = nc * 9 * 2.0 * (P2 + PH) + e * PH
+    r_oz = nc * planes * 2.0 * (P2 + PH) + e * PH
     a_i4_oz = e * (2 * PHr + HP2)
-    r_i4_oz = nc * 9 * 2.0 * (2 * PHr) + e * HP2
+    r_i4_oz = nc * planes * 2.0 * (2 * PHr) + e * HP2
     a_rg_oz = e * (2 * PHr + HP2)
-    r_rg_oz = nc * 9 * 2.0 * (PHr + HP2) + e * PHr
+    r_rg_oz = nc * planes * 2.0 * (PHr + HP2) + e * PHr
     # X = V_hhpp'^T T' (H x H, K = P) and HH_b = T' I9' (P x H, K = H) at a re-base
     a_x_oz = e * (2 * PH + H2)
-    r_x_oz = nc * 9 * 2.0 * (2 * PH) + e * H2
+    r_x_oz = nc * planes * 2.0 * (2 * PH) + e * H2
     a_hh_oz = e * (2 * PH + H2)
-    r_hh_oz = nc * 9 * 2.0 * (PH + H2) + e * 2 * PH
+    r_hh_oz = nc * planes * 2.0 * (PH + H2) + e * 2 * PH
     return {"x_fp64": ("flop", x, None), "i4_fp64": ("flop", i4, None), "ring_fp64": ("flop", rg, None),
             "ladder_fp64": ("flop", pp + hh, None), "pp_rebase_fp64": ("flop", pp, None), "hh_fp64": ("flop", hh, None),
             "pp_tc": ("byte", a_pp, r_pp), "i4_tc": ("byte", a_i4, r_i4), "ring_tc": ("byte", a_rg, r_rg),
@@ -415,7 +415,7 @@ def run_ours(args, wl):
 
     # ---- roofline of the dominant kernel (largest device time in the profiled solves) ----
     timers, ktimers = breakdown(prec, args.steps)
-    work = kernel_work(P, H, ring, prec, real=real)
+    work = kernel_work(P, H, ring, prec, real=real, planes=7)
     dom = max((k for k in ktimers if k in work and ktimers[k][1] > 0), key=lambda k: ktimers[k][0])
     kms, kn = ktimers[dom]
     per_launch_ms = kms / kn
@@ -494,15 +494,7 @@ def run_ours(args, wl):
 # captures of `bench.py --steps 1 --warmup 1 --no-e2e --no-cpu-baseline` on the workload:
 # (workload, precision, kernel slot) -> bytes
 PROFILED_TRAFFIC = {
-    # profiles/k_oz_gemm_snm132n3.md: both phase launches of the pp re-base product
-    ("snm132n3", "bf16x3", "pp_rebase_digits"): 4.09e9,
-    # the same scaled to SNM 132 nmax=4 by the algorithmic bytes (12.0 GB / 1.51 GB)
-    ("snm132n4", "bf16x3", "pp_rebase_digits"): 32.6e9,
-    ("pnm66", "bf16x3", "x_fp64"): 32.0e6,
     ("pnm66", "bf16x3", "pp_tc"): 643.7e6,
-    ("pnm66", "bf16x3", "pp_rebase_digits"): 2426.5e6,
-    ("pnm66", "bf16x3", "i4_rebase_digits"): 506.5e6,
-    ("pnm66", "bf16x3", "ring_rebase_digits"): 505.4e6,
 }
 
 

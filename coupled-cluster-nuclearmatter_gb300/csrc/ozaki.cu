@@ -5,13 +5,14 @@
 //   warp 4 (one lane) streams the digit tiles with cp.async.bulk: per K tile, the
 //     kOzSlices B digit tiles into one of two B buffers, then the kOzSlices A digit
 //     tiles one by one through a ring of kOzStages stages;
-//   warp 5 (one lane) issues tcgen05.mma: A digit i times B digits j = 0 .. 8 - i into
+//   warp 5 (one lane) issues tcgen05.mma: A digit i times B digits j = 0 .. 6 - i into
 //     the tensor-memory accumulators of levels i + j, all j in one MMA over the stacked
-//     B digit tiles, and commits each stage back;
+//     B digit tiles, and commits each stage back; chunks alternate between two sets of
+//     accumulators;
 //   warps 0-3 drain the kOzLevels accumulators after every K chunk (kOzChunkTiles K
 //     tiles, short enough for every level sum to stay an exact FP32 integer) into two
-//     64-bit integer sums per row and column, and after the tile's last chunk convert
-//     them to FP64 once, scale by 2^(eA + eB) and add into C.
+//     64-bit integer sums per row and column, beside the next chunk's MMAs, and after the
+//     tile's last chunk convert them to FP64 once, scale by 2^(eA + eB) and add into C.
 // Every wait is bounded: on expiry the waiting thread records an error code and raises
 // a shared abort flag that ends every other wait at once; the producer lets its own
 // copies land before the CTA frees its tensor memory and exits.
@@ -28,12 +29,14 @@ namespace {
 
 using namespace tcptx;
 
-constexpr int kOzStages = 6;
+constexpr int kOzStages = 8;
 constexpr uint32_t kATile = 128u * 128u;                   // one A digit tile: 128 rows x 64 BF16
 constexpr uint32_t kBSlot = (uint32_t)kOzN * 128u;         // one B digit tile of kOzN rows
 constexpr uint32_t kBBuf = (uint32_t)kOzSlices * kBSlot;   // all B digits of one K tile
 constexpr uint32_t kBarOff = kOzStages * kATile + 2 * kBBuf;
-constexpr int kOzBars = 2 * kOzStages + 8;  // afull, aempty, bfull[2], bempty[2], done, drained, fin
+constexpr int kOzBars = 2 * kOzStages + 9;  // afull, aempty, bfull[2], bempty[2], done[2], drained[2], fin
+constexpr uint32_t kOzSet = kOzLevels * kOzN;  // tensor-memory columns of one set of accumulators
+static_assert(2 * kOzSet <= 512 && kOzSet <= 256, "two sets of accumulators, one MMA over all levels");
 constexpr size_t kOzSmem = kBarOff + kOzBars * 8 + 16;
 constexpr int kOzThreads = 192;
 
@@ -58,7 +61,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
   uint8_t *bbuf = smem + kOzStages * kATile;
   uint64_t *bars = (uint64_t *)(smem + kBarOff);
   uint64_t *afull = bars, *aempty = bars + kOzStages, *bfull = bars + 2 * kOzStages, *bempty = bfull + 2,
-           *done = bempty + 2, *drained = done + 1, *fin = done + 2;
+           *done = bempty + 2, *drained = done + 2, *fin = drained + 2;
   uint32_t *tmem_slot = (uint32_t *)(bars + kOzBars);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
@@ -74,9 +77,9 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&bfull[b]), 1);
       mbar_init(smem_u32(&bempty[b]), 1);
+      mbar_init(smem_u32(&done[b]), 1);
+      mbar_init(smem_u32(&drained[b]), 4);
     }
-    mbar_init(smem_u32(done), 1);
-    mbar_init(smem_u32(drained), 4);
     mbar_init(smem_u32(fin), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -158,8 +161,10 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
         const int nk = P.nk;
         const int nchunk = (nk + kOzChunkTiles - 1) / kOzChunkTiles;
         for (int c = 0; c < nchunk && ok; ++c, ++ck) {
-          if (ck > 0 && !wait(drained, (uint32_t)((ck - 1) & 1))) { ok = false; break; }
+          // the set's chunk before (two chunks back) is drained
+          if (ck >= 2 && !wait(&drained[ck & 1], (uint32_t)(((ck >> 1) - 1) & 1))) { ok = false; break; }
           tc_fence_after();
+          const uint32_t set = tmem + (uint32_t)(ck & 1) * kOzSet;
           const int k_beg = c * kOzChunkTiles, k_end = min(nk, k_beg + kOzChunkTiles);
           for (int kt = k_beg; kt < k_end && ok; ++kt, ++bk) {
             const int bb = bk & 1;
@@ -170,28 +175,23 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
               const int s = cnt % kOzStages;
               if (!wait(&afull[s], (uint32_t)((cnt / kOzStages) & 1))) { ok = false; break; }
               tc_fence_after();
-              // A digit i times B digits j = 0 .. 8 - i lands in levels i .. 8: the B digit
+              // A digit i times B digits j = 0 .. 6 - i lands in levels i .. 6: the B digit
               // tiles sit one after the other (kOzN rows each) and the level accumulators
-              // kOzN columns apart, so one MMA of N = kOzN (9 - i) covers them all (two
-              // when that exceeds 256 columns).  Columns beyond a narrow tile's nc come
-              // from stale B rows and are never drained.
-              const uint64_t da = smem_desc(smem_u32(abuf + s * kATile));
+              // kOzN columns apart, so one MMA of N = kOzN (7 - i) covers them all.  Columns
+              // beyond a narrow tile's nc come from stale B rows and are never drained.
+              const uint64_t da = smem_desc(smem_u32(abuf + s * kATile)), db = smem_desc(sb);
+              const uint32_t id = instr_desc<kTcBF16>(128, (kOzSlices - i) * kOzN);
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks) {
                 const uint32_t acc = (kt > k_beg || i > 0 || ks > 0) ? 1u : 0u;
-                for (int j0 = 0; j0 < kOzSlices - i; j0 += 256 / kOzN) {
-                  const int nj = min(kOzSlices - i - j0, 256 / kOzN);
-                  tc_mma<kTcBF16>(tmem + (uint32_t)((i + j0) * kOzN), da + (uint64_t)(ks * 16),
-                                  smem_desc(sb + (uint32_t)j0 * kBSlot) + (uint64_t)(ks * 16),
-                                  instr_desc<kTcBF16>(128, nj * kOzN), acc);
-                }
+                tc_mma<kTcBF16>(set + (uint32_t)(i * kOzN), da + (uint64_t)(ks * 16), db + (uint64_t)(ks * 16), id, acc);
               }
               tc_commit(smem_u32(&aempty[s]));
               ++cnt;
             }
             if (ok) tc_commit(smem_u32(&bempty[bb]));
           }
-          if (ok) tc_commit(smem_u32(done));
+          if (ok) tc_commit(smem_u32(&done[ck & 1]));
         }
       }
       if (!ok) atomicExch(err, 2);
@@ -214,17 +214,17 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       const bool live = m < P.M;
       // a warp none of whose rows is stored skips the drain
       const bool warp_live = tl.mt * 128 + warp * 32 < P.M;
-      // The tile's row sums so far as exact integers in units of 2^-30 (levels 0-3) and
-      // 2^-60 (levels 4-8, kept below 2^30 by carrying into the first): each chunk adds
-      // its level sums with integer operations only, so the accumulators are free for the
-      // next chunk's MMAs after a few integer operations per level and column, and the
+      // The tile's row sums so far as exact integers in units of 2^-38 (levels 0-3) and
+      // 2^-62 (levels 4-6, kept below 2^24 by carrying into the first): each chunk adds
+      // its level sums with integer operations only, so the accumulators are free again
+      // after a few integer operations per level and column, and the
       // FP64 work (conversion, scaling, the read-modify-write of C) runs once per tile,
       // beside the next tile's MMAs.
       long long ah[kOzN], al[kOzN];
 #pragma unroll
       for (int q = 0; q < kOzN; ++q) ah[q] = al[q] = 0;
       for (int c = 0; c < nchunk; ++c, ++ck) {
-        const bool got = __all_sync(0xffffffffu, wait(done, (uint32_t)(ck & 1)));
+        const bool got = __all_sync(0xffffffffu, wait(&done[ck & 1], (uint32_t)((ck >> 1) & 1)));
         if (!got) {
           if (lane == 0) atomicExch(err, 3);
           ok = false;
@@ -237,7 +237,8 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
           // all levels of 4 columns in flight at once, one wait
           uint32_t r[kOzLevels][4];
 #pragma unroll
-          for (int lv = 0; lv < kOzLevels; ++lv) tmem_ld4(tbase + (uint32_t)(lv * kOzN + cb), r[lv]);
+          for (int lv = 0; lv < kOzLevels; ++lv)
+            tmem_ld4(tbase + (uint32_t)(ck & 1) * kOzSet + (uint32_t)(lv * kOzN + cb), r[lv]);
           tmem_ld_wait();
 #pragma unroll
           for (int lv = 0; lv < kOzLevels; ++lv) {
@@ -246,19 +247,19 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
               // an exact integer below 2^24 in magnitude
               const long long x = (long long)__float2int_rz(__uint_as_float(r[lv][q]));
               if (lv < 4) ah[cb + q] += x * (1ll << (kOzBits * (3 - lv)));
-              else al[cb + q] += x * (1ll << (kOzBits * (8 - lv)));
+              else al[cb + q] += x * (1ll << (kOzBits * (6 - lv)));
             }
           }
         }
-        // the level accumulators are read: the next chunk's MMAs may start
+        // the set's accumulators are read: the chunk after the next may start
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(drained));
+        if (lane == 0) mbar_arrive(smem_u32(&drained[ck & 1]));
 #pragma unroll
         for (int q = 0; q < kOzN; ++q) {
-          const long long carry = al[q] >> 30;  // floor: al stays in [0, 2^30)
+          const long long carry = al[q] >> 24;  // floor: al stays in [0, 2^24)
           ah[q] += carry;
-          al[q] -= carry * (1ll << 30);
+          al[q] -= carry * (1ll << 24);
         }
       }
       if (ok && live) {
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
           for (int q = q0; q < q0 + 8; ++q) {
             const int n = tl.n0 + q;
             if (q < nc && n < P.N) {
-              const double z = fma((double)ah[q], 0x1p-30, (double)al[q] * 0x1p-60);
+              const double z = fma((double)ah[q], 0x1p-38, (double)al[q] * 0x1p-62);
               crow[(int64_t)n * P.sCn] = old[q - q0] + P.alpha * (z * pow2(eAm + P.eB[n]));
             }
           }
@@ -309,21 +310,23 @@ __global__ void k_oz_exps(const OzSplitJob *__restrict__ jobs, const int2 *__res
   if (lane == 0) J.exps[jr.y] = mx == 0 ? 0 : mx - 1022;
 }
 
-// kOzSlices signed 6-bit digits of x 2^-e (truncated after 54 bits), as BF16 bit patterns
+// The balanced 8-bit digits of x 2^-e rounded to 55 bits, as BF16 bit patterns: of
+// Y = x 2^(55 - e), each byte from the second on is lifted by 128, so that it is the digit
+// plus 128 with the borrow taken from the byte above; the top digit keeps the sign.
 __device__ __forceinline__ void oz_digits(double x, int e, uint32_t (&d)[kOzSlices]) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(x);
   const int ex = (int)((u >> 52) & 0x7ff);
   unsigned long long y = 0;
   if (ex != 0) {
     const unsigned long long mant = (u & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const int sh = ex - 1021 - e;  // y = |x| 2^(54 - e) = mant 2^sh < 2^54, sh <= 1
-    y = sh >= 0 ? (mant << sh) : (-sh >= 64 ? 0ull : (mant >> -sh));
+    const int sh = ex - 1020 - e;  // y = |x| 2^(55 - e) = mant 2^sh < 2^55, sh <= 2
+    y = sh >= 0 ? (mant << sh) : (-sh >= 64 ? 0ull : ((mant + (1ull << (-sh - 1))) >> -sh));
   }
-  const bool neg = (u >> 63) != 0;
+  const unsigned long long s = ((u >> 63) ? 0ull - y : y) + 0x80808080808080ull;
 #pragma unroll
   for (int i = 0; i < kOzSlices; ++i) {
-    const int v = (int)((y >> (kOzBits * (kOzSlices - 1 - i))) & 63);
-    d[i] = __float_as_uint((float)(neg ? -v : v)) >> 16;
+    const int v = (i == 0 ? (int)((long long)s >> 48) : (int)((s >> (kOzBits * (kOzSlices - 1 - i))) & 255)) - 128;
+    d[i] = __float_as_uint((float)v) >> 16;
   }
 }
 

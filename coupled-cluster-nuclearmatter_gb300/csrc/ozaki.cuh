@@ -3,15 +3,22 @@
 // matrix multiplication by using fast routines of matrix multiplication and its
 // applications", Numer. Algorithms 59 (2012)).
 //
-// Every row of A (every column of B) is scaled by a power of two 2^e so that its
-// entries lie in (-1, 1), and the scaled value is cut into kOzSlices signed digits of
-// kOzBits bits: x = 2^e sum_i d_i 2^(-kOzBits i), |d_i| <= 63, each exactly a BF16.
-// A digit product sum_k a_i(m,k) b_j(k,n) is an integer below 2^24 in magnitude when K
-// is cut into chunks of kOzChunkTiles K tiles, so the FP32 tensor-memory accumulator
-// holds it exactly; the digit pairs of one level l = i + j share an accumulator.
-// Levels up to kOzSlices + 1 are kept (45 digit products); the dropped tail is below
-// 2^-52 of K max|A(m,.)| max|B(.,n)|.  The levels of one chunk are combined in two
-// 64-bit integers and converted to FP64 once.
+// Every row of A (every column of B) is scaled by a power of two 2^e so that its entries lie
+// in (-1, 1), rounded to 55 bits and cut into kOzSlices balanced digits of kOzBits bits:
+// x = 2^e sum_i d_i 2^(-7 - kOzBits i), |d_i| <= 128, each exactly a BF16.  A digit product
+// sum_k a_i(m,k) b_j(k,n) summed over the at most seven pairs of one level l = i + j is an
+// integer below 2^24 in magnitude when K is cut into chunks of kOzChunkTiles K tiles, so the FP32
+// tensor-memory accumulator of the level holds it exactly.  Levels below kOzSlices are kept (28
+// digit products); the dropped tail is below 2^-53 of K max|A(m,.)| max|B(.,n)|.  The levels of a
+// chunk are added into two 64-bit integers, converted to FP64 once per tile.
+//
+// Digits of 8 bits and a sign, 28 products of which one MMA per K step covers a digit of A, do
+// the work of the nine 6-bit digits that an unsigned cut needs, 45 products in 10 MMAs (the
+// shared-memory reads of the operands bound the MMAs: 57 KB against 82 per K step).  They allow
+// chunks of two K tiles instead of seven, so the accumulators come in two sets and a chunk is
+// drained while the next one runs.  Against a long double product the error falls from 5e-15 to
+// 5e-16 of the largest element (the rounding is to nearest), and five ragged products up to 1000 x
+// 256 x 1500 take 64 instead of 115 us; the SNM 132 nmax=4 solve 285 to 261 ms.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -21,11 +28,12 @@
 
 namespace ccx {
 
-constexpr int kOzSlices = 9;       // digits per operand
-constexpr int kOzBits = 6;         // bits per digit
-constexpr int kOzLevels = kOzSlices;  // levels 2 .. kOzSlices + 1
+constexpr int kOzSlices = 7;       // digits per operand
+constexpr int kOzBits = 8;         // bits per digit
+constexpr int kOzLevels = kOzSlices;  // levels 0 .. kOzSlices - 1
 constexpr int kOzN = 32;           // columns per CTA: kOzLevels accumulators at 32-column offsets
-constexpr int kOzChunkTiles = 7;   // K tiles (64 each) per exact accumulation chunk
+constexpr int kOzChunkTiles = 2;   // K tiles (64 each) per exact accumulation chunk
+static_assert((long long)kOzLevels * kOzChunkTiles * 64 * 128 * 128 < (1ll << 24), "level sums are exact in FP32");
 
 // Digit planes of one operand in the canonical K-major tiling of the split-precision
 // kernel (A: 128-row tiles, B: npad-row tiles), plane p at planes + p * plane_elems.

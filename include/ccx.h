@@ -281,7 +281,7 @@ typedef struct {
                                 has fallen by this factor since the last one (0: the default 1e-4) */
 } ccx_iter_opts;
 #define CCX_REBASE_FP64 0      /* products of a re-base on the FP64 FMA pipe */
-#define CCX_REBASE_DIGITS 1    /* the pp-ladder, I4 and ring products of a re-base as exact 6-bit digit
+#define CCX_REBASE_DIGITS 1    /* the pp-ladder, I4 and ring products of a re-base as exact digit
                                   products on the BF16 tensor cores (Ozaki scheme), FP64-accurate */
 
 typedef struct {
