@@ -348,7 +348,7 @@ __global__ void k_i7dots(DevLayout L, const S *__restrict__ V, const S *__restri
       const int ch = s1.x, P = L.P[ch];
       const S *v = V + L.t_off[ch] + (int64_t)P * sidx(s1.y);
       const S *u = T + L.t_off[ch] + (int64_t)P * sidx(s2.y);
-      for (int k = lane; k < P; k += 32) acc += v[k] * u[k];
+      for (int k = lane; k < P; k += 32) acc = madd(v[k], u[k], acc);
       acc = (ssign(s1.y) * ssign(s2.y)) * from2<S>(warp_sum2(to2(acc)));
     }
   }
@@ -448,9 +448,9 @@ __global__ void k_i6_rows(DevLayout L, const int2 *__restrict__ rowtile, const S
   for (int k = part; k < H; k += kI6Parts) {
     const int64_t o = (int64_t)P * k;
     const S t = tc[o + rho];
-    d0 += t * vc[o + rho];
-    if (i1 >= 0) d1 += t * vc[o + i1];
-    if (i2 >= 0) d2 += t * vc[o + i2];
+    d0 = madd(t, vc[o + rho], d0);
+    if (i1 >= 0) d1 = madd(t, vc[o + i1], d1);
+    if (i2 >= 0) d2 = madd(t, vc[o + i2], d2);
   }
   // the kI6Parts interleaved k partials of a row, summed in part order
   red[part][r][0] = d0;
@@ -584,9 +584,16 @@ void launch_rinit_maps(const DevLayout &L, int4 *omap, int4 *rmap, cudaStream_t 
   if (L.nttile) k_rinit_maps<<<L.nttile, 256, 0, st>>>(L, omap, rmap);
 }
 
+// x with its sign flipped when neg: the sign bits on the integer pipe (a subtraction from zero
+// costs as much of the FP64 pipe as a multiply-add)
+__device__ __forceinline__ double flip_sign(double x, bool neg) {
+  return __longlong_as_double(__double_as_longlong(x) ^ (neg ? (long long)(1ull << 63) : 0ll));
+}
+__device__ __forceinline__ cplx flip_sign(cplx x, bool neg) { return cplx(flip_sign(x.re, neg), flip_sign(x.im, neg)); }
+// T at signed position m, negated when neg
 template <typename S>
-__device__ __forceinline__ S signed_at(const S *__restrict__ T, int m) {
-  return m > 0 ? T[m - 1] : S(0.0) - T[-m - 1];
+__device__ __forceinline__ S signed_at(const S *__restrict__ T, int m, bool neg) {
+  return flip_sign(T[abs(m) - 1], (m < 0) != neg);
 }
 template <typename S>
 __device__ __forceinline__ S at_or_zero(const S *__restrict__ X, int m) {
@@ -613,14 +620,14 @@ __global__ void k_rinit(DevLayout L, const int4 *__restrict__ omap, const int4 *
     if (o.x | o.y) {
       const int ab = e % P;
       const int2 po = L.pp_orb[L.pp_off[ch] + ab];
-      if (o.x) r += i6off[po.y - A] * signed_at(T, o.x);
-      if (o.y) r -= i6off[po.x - A] * signed_at(T, o.y);
+      if (o.x) r = madd(i6off[po.y - A], signed_at(T, o.x, false), r);
+      if (o.y) r = madd(i6off[po.x - A], signed_at(T, o.y, true), r);
     }
     if (o.z | o.w) {
       const int ij = e / P;
       const int2 ho = L.hh_orb[L.hh_off[ch] + ij];
-      if (o.z) r -= i7off[ho.y] * signed_at(T, o.z);
-      if (o.w) r += i7off[ho.x] * signed_at(T, o.w);
+      if (o.z) r = madd(i7off[ho.y], signed_at(T, o.z, true), r);
+      if (o.w) r = madd(i7off[ho.x], signed_at(T, o.w, false), r);
     }
     const S ring = at_or_zero(Rph, m.x) - at_or_zero(Rph, m.y) - at_or_zero(Rph, m.z) + at_or_zero(Rph, m.w);
     if (ring_out) ring_out[base + e] = ring;  // the ring term of this R_ph, kept per amplitude
@@ -808,14 +815,14 @@ __global__ void __launch_bounds__(256) k_update_std(DevLayout L, const S *__rest
       const int ij = el / P, ab = el - ij * P;
       const int2 po = pporb[ab];
       const S D = (sdij[ij - ij0] - d2ab[po.x - A]) - d2ab[po.y - A];
-      const S q = r - D * t;
+      const S q = madd(flip_sign(D, true), t, r);
       const E step = upd_step(q, D, r2);
       hist_t[g] = add_step(t, step);
       hist_e[g] = step;
       if constexpr (ScalarOf<S>::complex) {
-        const S pr = t * vij;
-        e_re += real_(pr);
-        e_im += imag_(pr);
+        const cplx en = madd(t, vij, cplx(e_re, e_im));
+        e_re = en.re;
+        e_im = en.im;
       } else {
         e_re = fma(t, vij, e_re);
       }
@@ -902,12 +909,45 @@ template <typename S>
 __global__ void k_combine(int64_t n, PtrPack<S> xs, CoefPack<S> c, int m, S *y) {
   for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     S acc = S(0.0);
-    for (int i = 0; i < m; ++i) acc += make_scalar<S>(c.re[i], c.im[i]) * xs.p[i][x];
+    for (int i = 0; i < m; ++i) acc = madd(make_scalar<S>(c.re[i], c.im[i]), xs.p[i][x], acc);
     y[x] = acc;
   }
 }
+// Real coefficients (the standard mode's, and every real engine's): a complex vector is twice
+// as many real entries, one FP64 operation for each of them and term where a complex product takes
+// four.  With the general form the FP64 pipe bounded it: 0.92 ms for the 8 vectors of SNM 132
+// nmax=4, now 0.38, close to the time of reading them.  M terms, all their loads in flight together.
+template <int M>
+__global__ void __launch_bounds__(256) k_combine_real(int64_t n, PtrPack<double> xs, CoefPack<double> c, double *y) {
+  for (int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
+    double v[M], acc = 0.0;
+#pragma unroll
+    for (int i = 0; i < M; ++i) v[i] = xs.p[i][x];
+#pragma unroll
+    for (int i = 0; i < M; ++i) acc = fma(c.re[i], v[i], acc);
+    y[x] = acc;
+  }
+}
+template <int M = kMaxDots>
+void combine_real(int64_t n, const PtrPack<double> &xs, const CoefPack<double> &c, int m, double *y, cudaStream_t st) {
+  if (m == M) k_combine_real<M><<<(int)std::min<int64_t>((n + 255) / 256, 2432), 256, 0, st>>>(n, xs, c, y);
+  else if constexpr (M > 1) combine_real<M - 1>(n, xs, c, m, y, st);
+}
 template <typename S>
 void launch_combine(int64_t n, const S *const *xs, const double *coef, int m, S *y, cudaStream_t st) {
+  if (n <= 0 || m < 1) return;
+  bool real = m <= kMaxDots;
+  for (int k = 0; k < m; ++k) real = real && coef[2 * k + 1] == 0.0;
+  if (real) {
+    PtrPack<double> pk{};
+    CoefPack<double> c{};
+    for (int k = 0; k < m; ++k) {
+      pk.p[k] = reinterpret_cast<const double *>(xs[k]);
+      c.re[k] = coef[2 * k];
+    }
+    combine_real(n * (ScalarOf<S>::complex ? 2 : 1), pk, c, m, reinterpret_cast<double *>(y), st);
+    return;
+  }
   PtrPack<S> pk{};
   CoefPack<S> c{};
   for (int k = 0; k < m && k < kMaxDots; ++k) {
