@@ -1968,39 +1968,6 @@ class Engine final : public IEngine {
       gj.push_back(g);
     }
   }
-  // C (S units, strides sCm, sCn) += alpha A B with A (M x K) in tile buffer a at ao and
-  // B (N x K) in b at bo.  N beyond one accumulator (256 columns) runs as column blocks
-  // of at most 256 that step through the whole B operand's K tiles.
-  void add_tc(TcList &l, TileBuf &a, int64_t ao, TileBuf &b, int64_t bo, int M, int N, int K, S *C, int64_t sCm,
-              int64_t sCn, double alpha) {
-    const size_t es = tc_kind_ == kTcBF16 ? 2 : 4;
-    const int tk = tc_tile_k(tc_kind_);
-    const int npad_all = (N + 15) / 16 * 16;
-    auto one = [&](int ca, int cb, int cc, double al, int ph) {
-      for (int n0 = 0; n0 < N; n0 += 256) {
-        const int nb = std::min(256, N - n0);
-        TcProb p{};
-        p.Ahi = (char *)a.hi.p + (ao + ca * a.n) * es;
-        p.Alo = (char *)a.lo.p + (ao + ca * a.n) * es;
-        p.Bhi = (char *)b.hi.p + (bo + cb * b.n) * es + (size_t)n0 * 128;
-        p.Blo = (char *)b.lo.p + (bo + cb * b.n) * es + (size_t)n0 * 128;
-        p.M = M; p.N = nb; p.nk = (K + tk - 1) / tk; p.npad = (nb + 15) / 16 * 16;
-        p.bstride = npad_all > 256 ? (int64_t)npad_all * 128 : 0;
-        p.C = (double *)C + cc + (int64_t)n0 * sCn * kNComp; p.sCm = sCm * kNComp; p.sCn = sCn * kNComp; p.alpha = al;
-        for (int mt = 0; mt < (M + 127) / 128; ++mt) l.tiles.push_back(TcTile{(int)l.probs.size(), mt});
-        l.probs.push_back(p);
-        l.phase.push_back(ph);
-      }
-    };
-    if (kNComp == 1) {
-      one(0, 0, 0, alpha, 0);
-    } else {
-      one(0, 0, 0, alpha, 0);
-      one(0, 1, 1, alpha, 0);
-      one(1, 1, 0, -alpha, 1);
-      one(1, 0, 1, alpha, 1);
-    }
-  }
   // Up to three products accumulated into one output tile and written once:
   // C = (overwrite ? 0 : C) + C0 + alpha sum_op A_op B_op, every op with the same M, N.
   struct TcOp {

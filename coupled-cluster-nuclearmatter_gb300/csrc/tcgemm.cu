@@ -33,23 +33,29 @@ constexpr int kTcThreads = 320;   // warps 0-7 epilogue, warp 8 producer, warp 9
 constexpr int kTcHalfCols = 256;  // tensor-memory columns of one accumulator half
 constexpr int kTcMaxStages = 8;
 
-// FP32 bit pattern -> the same value as FP64, exactly, with integer operations only (a
-// float-to-double conversion would run on this GPU's narrow FP64 pipe)
-__device__ __forceinline__ double f32_bits_to_f64(uint32_t u) {
+// FP32 bit pattern -> the same value as FP64 times 2^ash, exactly, with integer operations
+// only (a float-to-double conversion would run on this GPU's narrow FP64 pipe); |ash| small
+__device__ __forceinline__ double f32_bits_to_f64(uint32_t u, int ash) {
   const unsigned long long sign = (unsigned long long)(u >> 31) << 63;
   const uint32_t e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
   unsigned long long bits;
   if (e == 0xffu) {  // infinities and NaNs
     bits = sign | (0x7ffull << 52) | ((unsigned long long)m << 29);
   } else if (e != 0) {  // normal: exponent rebiased from 127 to 1023
-    bits = sign | ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)m << 29);
+    bits = sign | ((unsigned long long)(e + 896u + (uint32_t)ash) << 52) | ((unsigned long long)m << 29);
   } else if (m == 0) {
     bits = sign;
   } else {  // subnormal m 2^-149, normalised on its leading bit p
     const int p = 31 - __clz((int)m);
-    bits = sign | ((unsigned long long)(p - 149 + 1023) << 52) | (((unsigned long long)m << (52 - p)) & 0xFFFFFFFFFFFFFull);
+    bits = sign | ((unsigned long long)(p - 149 + 1023 + ash) << 52) | (((unsigned long long)m << (52 - p)) & 0xFFFFFFFFFFFFFull);
   }
   return __longlong_as_double((long long)bits);
+}
+// hi + lo += x, the rounding of the addition kept in lo (Knuth's two-sum)
+__device__ __forceinline__ void pair_add(float &hi, float &lo, float x) {
+  const float s = __fadd_rn(hi, x), t = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(x, t)));
+  hi = s;
 }
 
 // K tiles of segment e of a problem (e = 0: the problem's own operands)
@@ -75,7 +81,7 @@ __device__ __forceinline__ TcGeom tc_geom(const TcProb *__restrict__ pp, int npa
   // one FP32 accumulator per segment while they fit in half of the tensor memory (the
   // other half holds the next tile's accumulators); a segment beyond that adds into the
   // last one.  Each product then keeps the rounding of its own accumulation, and the
-  // epilogue sums them in FP64.
+  // epilogue sums them in pairs of FP32 numbers.
   g.nacc = g.nseg;
   while (g.nacc > 1 && g.nacc * g.ncols > kTcHalfCols) --g.nacc;
   return g;
@@ -268,7 +274,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
       const double *C0 = pp->C0;
       const double *__restrict__ c0row = C0 ? C0 + (int64_t)m * sCm : nullptr;
       const bool keep = pp->overwrite == 0;
-      const double alpha = pp->alpha;
+      // alpha (1 or 1/2) is an exponent, not a multiplication
+      const int ash = (int)((__double_as_longlong(pp->alpha) >> 52) & 0x7ff) - 1023;
       const int nvalid = pp->N;
       const bool live = m < pp->M;
       if (tl.mt * 128 + quad * 32 >= pp->M) {  // no row of this warp's lanes is stored
@@ -277,49 +284,67 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
         continue;
       }
       const uint32_t accb = lane_base + (uint32_t)(b * kTcHalfCols);
-      // 32 columns per read (npad rounded up to 32 stays inside each accumulator)
-      for (int c0 = 0; c0 < G.npad; c0 += 32) {
+      // 16 columns at a time: the registers of 32 would spill
+      for (int c0 = 0; c0 < G.npad; c0 += 16) {
         // the C and C0 loads go first, so that their latency overlaps the tensor-memory
         // reads; the mode is uniform over the tile, so the branches sit outside the
-        // unrolled loops and the 32 loads of a row issue back to back
-        double v[32];
+        // unrolled loops and the 16 loads of a row issue back to back
+        double v[16];
         if (live && keep) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = (c0 + j < nvalid) ? crow[(int64_t)(c0 + j) * sCn] : 0.0;
+          for (int j = 0; j < 16; ++j) v[j] = (c0 + j < nvalid) ? crow[(int64_t)(c0 + j) * sCn] : 0.0;
         } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = 0.0;
+          for (int j = 0; j < 16; ++j) v[j] = 0.0;
         }
         if (live && c0row) {
-          double add[32];
+          double add[16];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) add[j] = (c0 + j < nvalid) ? c0row[(int64_t)(c0 + j) * sCn] : 0.0;
+          for (int j = 0; j < 16; ++j) add[j] = (c0 + j < nvalid) ? c0row[(int64_t)(c0 + j) * sCn] : 0.0;
           if (keep) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] += add[j];
+            for (int j = 0; j < 16; ++j) v[j] += add[j];
           } else {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = add[j];
+            for (int j = 0; j < 16; ++j) v[j] = add[j];
           }
         }
-        // one FP64 multiply-add per accumulator and element: the FP32 values widen on
-        // the integer pipe
+        // The accumulators are summed as pairs of FP32 numbers (48 bits, against the 24 of each
+        // accumulator) and widen on the integer pipe: one FP64 addition an element, none for a
+        // single accumulator that is only stored.  A multiply-add in FP64 for each of them bound
+        // the ring's launch: 1.16 ms for dR_ph of SNM 132 nmax=4 (four accumulators), now 1.00; dI4
+        // (two) stays at 1.0 ms.  Reading two accumulators for each wait costs 1 % of the solve.
+        float hi[16], lo[16];
         for (int a = 0; a < G.nacc; ++a) {
-          uint32_t r[32];
-          tmem_ld32(accb + (uint32_t)(a * G.ncols + c0), r);
+          uint32_t r[16];
+          tmem_ld16(accb + (uint32_t)(a * G.ncols + c0), r);
           tmem_ld_wait();
+          if (a == 0) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = fma(alpha, f32_bits_to_f64(r[j]), v[j]);
+            for (int j = 0; j < 16; ++j) { hi[j] = __uint_as_float(r[j]); lo[j] = 0.0f; }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) pair_add(hi[j], lo[j], __uint_as_float(r[j]));
+          }
         }
-        if (c0 + 32 >= G.npad) {
+        if (c0 + 16 >= G.npad) {
           // the accumulators of this half are read: hand it back to the MMA issuer
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&tempty[b]));
         }
+        const bool onto = keep || c0row;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const uint32_t h = __float_as_uint(hi[j]);
+          double x = f32_bits_to_f64(h, ash);
+          // (a pair that overflowed has no lo part: infinities stay infinities)
+          if (G.nacc > 1 && (h & 0x7f800000u) != 0x7f800000u) x += f32_bits_to_f64(__float_as_uint(lo[j]), ash);
+          v[j] = onto ? v[j] + x : x;
+        }
         if (live) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
+          for (int j = 0; j < 16; ++j)
             if (c0 + j < nvalid) crow[(int64_t)(c0 + j) * sCn] = v[j];
         }
       }

@@ -34,7 +34,7 @@ struct TcProb {
   int M, N, nk, npad;     // rows, columns, K tiles, padded columns (multiple of 16, <= 256)
   double *C;              // C(m, n) at C[m * sCm + n * sCn]
   int64_t sCm, sCn;
-  double alpha;
+  double alpha;           // a positive power of two: the epilogue adds its exponent
   int64_t bstride;        // bytes between B K tiles (0: npad * 128, the whole B operand); a
                           // column block of a wider B points Bhi/Blo at its first row and
                           // steps by the full operand's K-tile size
