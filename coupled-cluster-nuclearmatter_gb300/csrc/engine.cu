@@ -1945,28 +1945,27 @@ class Engine final : public IEngine {
       js.push_back(j);
     }
   }
-  // Map and gather jobs filling tile region (b, off) from the packed split of T - T_b:
+  // Map and gather job filling tile region (b, off) from the packed split of T - T_b:
   // element (r, k) is packed entry ind ? ind[base + r sr + k sk] : base + r sr + k sk
-  // (scalar elements), one job per scalar component
+  // (in elements of S)
   void add_gather(std::vector<TcMapJob> &mj, std::vector<TcGatherJob> &gj, int64_t base, const int32_t *ind,
                   int64_t sr, int64_t sk, int rows, int cols, int tile_rows, int rows_pad, TileBuf &b, DBuf &map,
                   int64_t off) {
     const size_t es = tc_kind_ == kTcBF16 ? 2 : 4;
     const int tk = tc_tile_k(tc_kind_);
-    for (int c = 0; c < kNComp; ++c) {
-      TcMapJob m{};
-      m.base = base; m.sr = sr; m.sk = sk;
-      m.rows = rows; m.cols = cols; m.tile_rows = tile_rows; m.nk = (cols + tk - 1) / tk; m.rows_pad = rows_pad;
-      m.ind = ind;
-      m.map = map.as<int32_t>() + off + c * b.n;
-      mj.push_back(m);
-      TcGatherJob g{};
-      g.map = m.map;
-      g.phl = (const char *)phl_.p + (size_t)c * n_t_ * 2 * es;
-      g.hi = (char *)b.hi.p + (off + c * b.n) * es;
-      g.lo = (char *)b.lo.p + (off + c * b.n) * es;
-      gj.push_back(g);
-    }
+    TcMapJob m{};
+    m.base = base; m.sr = sr; m.sk = sk;
+    m.rows = rows; m.cols = cols; m.tile_rows = tile_rows; m.nk = (cols + tk - 1) / tk; m.rows_pad = rows_pad;
+    m.ind = ind;
+    m.map = map.as<int32_t>() + off;
+    mj.push_back(m);
+    TcGatherJob g{};
+    g.map = m.map;
+    g.phl = phl_.p;
+    g.cs = b.n * (int64_t)es / 16;
+    g.hi = (char *)b.hi.p + off * es;
+    g.lo = (char *)b.lo.p + off * es;
+    gj.push_back(g);
   }
   // Up to three products accumulated into one output tile and written once:
   // C = (overwrite ? 0 : C) + C0 + alpha sum_op A_op B_op, every op with the same M, N.
@@ -2343,7 +2342,7 @@ class Engine final : public IEngine {
     launch_tph_map(D_, tphmap_.as<int32_t>(), st_);
     for (auto pr : {std::make_pair(&mD_, &tD_), std::make_pair(&mDA_, &tDA_), std::make_pair(&mDphB_, &tDphB_),
                     std::make_pair(&mDphA_, &tDphA_)})
-      pr.first->alloc((size_t)pr.second->n * kNComp * sizeof(int32_t), &bytes_);
+      pr.first->alloc((size_t)pr.second->n * sizeof(int32_t), &bytes_);
     std::vector<TcMapJob> mjobs;
     std::vector<TcGatherJob> gjobs;
     TcList pp, p4, pr1;
@@ -2587,11 +2586,9 @@ class Engine final : public IEngine {
     kbegin(kKSplit);
     // dT' = T' - T_b' split once; dT' (B and A) and dT_ph (B and A) gathered from it
     // (T_ph itself is not needed in FP64 between re-bases)
-    for (int c = 0; c < kNComp; ++c)
-      launch_tc_split_packed(tc_kind_, (const double *)T_.p + c, (const double *)Tb_.p + c, n_t_, kNComp,
-                             (char *)phl_.p + (size_t)c * n_t_ * (tc_kind_ == kTcBF16 ? 4 : 8), st_);
-    launch_tc_gather(tc_kind_, (const TcGatherJob *)gplan_.jobs.p, (const int4 *)gplan_.chunks.p, gplan_.nchunks, st_);
-    launches_ += kNComp + 1;
+    launch_tc_split_packed(tc_kind_, (const double *)T_.p, (const double *)Tb_.p, n_t_ * kNComp, phl_.p, st_);
+    launch_tc_gather(tc_kind_, kNComp, (const TcGatherJob *)gplan_.jobs.p, (const int4 *)gplan_.chunks.p, gplan_.nchunks, st_);
+    launches_ += 2;
     kend();
     mark(1);
     // X in FP64: it feeds the dressed hole denominators of every amplitude through I7

@@ -570,15 +570,15 @@ __global__ void __launch_bounds__(256) k_tc_build_map(const TcMapJob *__restrict
   }
 }
 
-// the hi and lo bit patterns of packed entry |m| - 1 (hi and lo interleaved in one word:
-// BF16 hi | lo << 16, TF32 hi | lo << 32), sign flipped for m < 0
-template <int KIND>
-__device__ __forceinline__ void gather_one(const void *phl, int32_t m, uint32_t &h, uint32_t &l) {
+// the hi and lo bit patterns of component c of packed entry |m| - 1 (hi and lo interleaved in
+// one word: BF16 hi | lo << 16, TF32 hi | lo << 32), sign flipped for m < 0
+template <int KIND, int NC>
+__device__ __forceinline__ void gather_one(const void *phl, int32_t m, int c, uint32_t &h, uint32_t &l) {
   if (m == 0) {
     h = l = 0;
     return;
   }
-  const int64_t i = (m > 0 ? m : -m) - 1;
+  const int64_t i = (int64_t)((m > 0 ? m : -m) - 1) * NC + c;
   if (KIND == kTcBF16) {
     const uint32_t w = ((const uint32_t *)phl)[i] ^ (m < 0 ? 0x80008000u : 0u);
     h = w & 0xFFFFu;
@@ -590,13 +590,17 @@ __device__ __forceinline__ void gather_one(const void *phl, int32_t m, uint32_t 
   }
 }
 
-template <int KIND>
+// Bound by the random reads of the packed pairs.  Adjacent lanes take the two components of a
+// complex operand's unit, which lie in one sector of the packed array and share the map entry; a
+// job for each component read both twice.  SNM 132 nmax=4: 621 to 498 us.
+template <int KIND, int NC>
 __global__ void __launch_bounds__(256) k_tc_gather(const TcGatherJob *__restrict__ jobs, const int4 *__restrict__ chunks) {
   constexpr int cme = Half<KIND>::per16;
   const int4 ck = chunks[blockIdx.x];
   const TcGatherJob J = jobs[ck.x];
-  uint4 *hi = (uint4 *)J.hi, *lo = (uint4 *)J.lo;
-  for (int u = ck.y + threadIdx.x; u < ck.z; u += blockDim.x) {
+  const int c = threadIdx.x % NC;
+  uint4 *hi = (uint4 *)J.hi + c * J.cs, *lo = (uint4 *)J.lo + c * J.cs;
+  for (int u = ck.y + (int)threadIdx.x / NC; u < ck.z; u += (int)blockDim.x / NC) {
     int32_t m[cme];
     const int4 *mp = (const int4 *)J.map + (int64_t)u * (cme / 4);  // the unit's map entries
 #pragma unroll
@@ -609,7 +613,7 @@ __global__ void __launch_bounds__(256) k_tc_gather(const TcGatherJob *__restrict
     }
     uint32_t h[cme], l[cme];
 #pragma unroll
-    for (int j = 0; j < cme; ++j) gather_one<KIND>(J.phl, m[j], h[j], l[j]);
+    for (int j = 0; j < cme; ++j) gather_one<KIND, NC>(J.phl, m[j], c, h[j], l[j]);
     uint32_t hw[4], lw[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -628,12 +632,12 @@ __global__ void __launch_bounds__(256) k_tc_gather(const TcGatherJob *__restrict
 
 template <int KIND>
 __global__ void __launch_bounds__(256) k_tc_split_packed(const double *__restrict__ src, const double *__restrict__ sub,
-                                                         int64_t n, int stride, void *phl) {
+                                                         int64_t n, void *phl) {
   using B = BitSplit<Half<KIND>::nb>;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     uint32_t h, l;
-    if (sub) B::split_diff(src[i * stride], sub[i * stride], h, l);
-    else B::split(src[i * stride], h, l);
+    if (sub) B::split_diff(src[i], sub[i], h, l);
+    else B::split(src[i], h, l);
     if (KIND == kTcBF16) ((uint32_t *)phl)[i] = (h >> 16) | (l & 0xFFFF0000u);
     else ((unsigned long long *)phl)[i] = (unsigned long long)h | ((unsigned long long)l << 32);
   }
@@ -646,17 +650,17 @@ void launch_tc_build_map(int kind, const TcMapJob *jobs, const int4 *chunks, int
   if (kind == kTcBF16) k_tc_build_map<kTcBF16><<<nchunks, 256, 0, st>>>(jobs, chunks);
   else k_tc_build_map<kTcTF32><<<nchunks, 256, 0, st>>>(jobs, chunks);
 }
-void launch_tc_gather(int kind, const TcGatherJob *jobs, const int4 *chunks, int nchunks, cudaStream_t st) {
+void launch_tc_gather(int kind, int comps, const TcGatherJob *jobs, const int4 *chunks, int nchunks, cudaStream_t st) {
   if (nchunks <= 0) return;
-  if (kind == kTcBF16) k_tc_gather<kTcBF16><<<nchunks, 256, 0, st>>>(jobs, chunks);
-  else k_tc_gather<kTcTF32><<<nchunks, 256, 0, st>>>(jobs, chunks);
+  auto k = kind == kTcBF16 ? (comps == 2 ? k_tc_gather<kTcBF16, 2> : k_tc_gather<kTcBF16, 1>)
+                           : (comps == 2 ? k_tc_gather<kTcTF32, 2> : k_tc_gather<kTcTF32, 1>);
+  k<<<nchunks, 256, 0, st>>>(jobs, chunks);
 }
-void launch_tc_split_packed(int kind, const double *src, const double *sub, int64_t n, int stride, void *phl,
-                            cudaStream_t st) {
+void launch_tc_split_packed(int kind, const double *src, const double *sub, int64_t n, void *phl, cudaStream_t st) {
   if (n <= 0) return;
   const int grid = (int)std::min<int64_t>((n + 255) / 256, 4096);
-  if (kind == kTcBF16) k_tc_split_packed<kTcBF16><<<grid, 256, 0, st>>>(src, sub, n, stride, phl);
-  else k_tc_split_packed<kTcTF32><<<grid, 256, 0, st>>>(src, sub, n, stride, phl);
+  if (kind == kTcBF16) k_tc_split_packed<kTcBF16><<<grid, 256, 0, st>>>(src, sub, n, phl);
+  else k_tc_split_packed<kTcTF32><<<grid, 256, 0, st>>>(src, sub, n, phl);
 }
 
 int tc_stages(int npad_max) {

@@ -96,16 +96,17 @@ struct TcMapJob {
   int32_t *map;  // parallel to the tile region: element j of unit u at map[u * per16 + j]
 };
 void launch_tc_build_map(int kind, const TcMapJob *jobs, const int4 *chunks, int nchunks, cudaStream_t st);
-// the gather: unit u of job j from its map and the packed arrays of its scalar component
+// the gather: unit u of job j from its map and the packed array; comps = 2: both scalar
+// components of a complex operand, whose tiles lie cs units apart, through one map
 struct TcGatherJob {
   const int32_t *map;
-  const void *phl;  // packed hi/lo pairs: BF16 hi | lo << 16 (32 bits), TF32 hi | lo << 32 (64 bits)
+  const void *phl;  // packed hi/lo pairs: BF16 hi | lo << 16 (32 bits), TF32 hi | lo << 32 (64 bits);
+                    // component c of entry i is pair i comps + c
   void *hi, *lo;    // tile region
+  int64_t cs;
 };
-void launch_tc_gather(int kind, const TcGatherJob *jobs, const int4 *chunks, int nchunks, cudaStream_t st);
-// packed split of src - sub, n entries at a stride of `stride` doubles (the scalar
-// components of complex data are split as separate vectors by their offsets)
-void launch_tc_split_packed(int kind, const double *src, const double *sub, int64_t n, int stride, void *phl,
-                            cudaStream_t st);
+void launch_tc_gather(int kind, int comps, const TcGatherJob *jobs, const int4 *chunks, int nchunks, cudaStream_t st);
+// packed split of src - sub, n doubles (two per entry of a complex vector)
+void launch_tc_split_packed(int kind, const double *src, const double *sub, int64_t n, void *phl, cudaStream_t st);
 
 }  // namespace ccx
