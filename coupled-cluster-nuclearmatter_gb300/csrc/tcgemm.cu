@@ -33,9 +33,8 @@ constexpr int kTcThreads = 320;   // warps 0-7 epilogue, warp 8 producer, warp 9
 constexpr int kTcHalfCols = 256;  // tensor-memory columns of one accumulator half
 constexpr int kTcMaxStages = 8;
 
-// FP32 bit pattern -> the same value as FP64 times 2^ash, exactly, with integer operations
-// only (a float-to-double conversion would run on this GPU's narrow FP64 pipe); |ash| small
-__device__ __forceinline__ double f32_bits_to_f64(uint32_t u, int ash) {
+// FP32 bit pattern -> the same value as FP64 times 2^ash, exactly: any number, with branches
+__device__ __noinline__ double f32_bits_to_f64(uint32_t u, int ash) {
   const unsigned long long sign = (unsigned long long)(u >> 31) << 63;
   const uint32_t e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
   unsigned long long bits;
@@ -50,6 +49,29 @@ __device__ __forceinline__ double f32_bits_to_f64(uint32_t u, int ash) {
     bits = sign | ((unsigned long long)(p - 149 + 1023 + ash) << 52) | (((unsigned long long)m << (52 - p)) & 0xFFFFFFFFFFFFFull);
   }
   return __longlong_as_double((long long)bits);
+}
+// the same of zeros and normal numbers, without branches; odd: any other number
+__device__ __forceinline__ unsigned long long f32_widen(uint32_t u, int ash, bool &odd) {
+  const uint32_t a = u & 0x7fffffffu;
+  odd |= a - 1u < 0x7fffffu || a >= 0x7f800000u;
+  const uint32_t hi = a ? (a >> 3) + ((uint32_t)(896 + ash) << 20) : 0u;
+  return ((unsigned long long)hi << 32) | (u << 29);
+}
+// (hi + lo) 2^ash rounded to FP64, hi + lo = hi in FP32.  lo counts in units of the last place of
+// the FP64 number that hi widens to, and is added to it as an integer.
+__device__ __forceinline__ double pair_widen(float hi, float lo, int ash, bool &odd) {
+  const uint32_t u = __float_as_uint(hi), v = __float_as_uint(lo);
+  const uint32_t el = (v >> 23) & 0xffu, ml = v & 0x7fffffu;
+  odd |= el == 0 && ml != 0;
+  const unsigned long long w = f32_widen(u, ash, odd);
+  // (lo != 0: the shift is not negative, |lo| being at most half an ulp of hi)
+  const int sh = max(0, min(31, (int)((u >> 23) & 0xffu) - (int)el - 24));
+  uint32_t t = el ? ((ml | 0x800000u) << 5) : 0u;
+  t = (t + ((1u << sh) >> 1)) >> sh;
+  const bool down = (int)(u ^ v) < 0;
+  if (down && (u & 0x7fffffu) == 0) t <<= 1;  // towards the binade below, whose unit is half
+  const unsigned long long x = down ? w - t : w + t;
+  return __longlong_as_double((long long)(x | ((unsigned long long)(u & 0x80000000u) << 32)));
 }
 // hi + lo += x, the rounding of the addition kept in lo (Knuth's two-sum)
 __device__ __forceinline__ void pair_add(float &hi, float &lo, float x) {
@@ -310,10 +332,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
           }
         }
         // The accumulators are summed as pairs of FP32 numbers (48 bits, against the 24 of each
-        // accumulator) and widen on the integer pipe: one FP64 addition an element, none for a
-        // single accumulator that is only stored.  A multiply-add in FP64 for each of them bound
-        // the ring's launch: 1.16 ms for dR_ph of SNM 132 nmax=4 (four accumulators), now 1.00; dI4
-        // (two) stays at 1.0 ms.  Reading two accumulators for each wait costs 1 % of the solve.
+        // accumulator) and rounded to FP64 as integers without branches: one FP64 addition an
+        // element where it is added onto something, else none.  The drain warps bound the
+        // launches on the particle-hole channels: a multiply-add in FP64 for each accumulator
+        // took 1.16 ms for dR_ph of SNM 132 nmax=4 (four accumulators) and 1.03 for dI4 (two),
+        // pairs with a branching conversion and an FP64 addition 1.00 and 1.03, now 0.77 and
+        // 0.81; PNM 66 nmax=4 140 and 93, 136 and 96, now 95 and 69 us.  Reading two accumulators
+        // for each wait costs 1 % of a solve.
         float hi[16], lo[16];
         for (int a = 0; a < G.nacc; ++a) {
           uint32_t r[16];
@@ -334,14 +359,33 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
           if (lane == 0) mbar_arrive(smem_u32(&tempty[b]));
         }
         const bool onto = keep || c0row;
+        bool odd = false;
+        double x[16];
+        if (G.nacc > 1) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const uint32_t h = __float_as_uint(hi[j]);
-          double x = f32_bits_to_f64(h, ash);
-          // (a pair that overflowed has no lo part: infinities stay infinities)
-          if (G.nacc > 1 && (h & 0x7f800000u) != 0x7f800000u) x += f32_bits_to_f64(__float_as_uint(lo[j]), ash);
-          v[j] = onto ? v[j] + x : x;
+          for (int j = 0; j < 16; ++j) {
+            // the pair's own sum first; infinities stay infinities
+            const float l = fabsf(hi[j]) < __int_as_float(0x7f800000) ? lo[j] : 0.0f;
+            lo[j] = 0.0f;
+            pair_add(hi[j], lo[j], l);
+            x[j] = pair_widen(hi[j], lo[j], ash, odd);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const uint32_t u = __float_as_uint(hi[j]);
+            x[j] = __longlong_as_double((long long)(f32_widen(u, ash, odd) | ((unsigned long long)(u & 0x80000000u) << 32)));
+          }
         }
+        if (__any_sync(0xffffffffu, odd && live)) {  // a subnormal, an infinity or a NaN
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            x[j] = f32_bits_to_f64(__float_as_uint(hi[j]), ash);
+            if (isfinite(hi[j])) x[j] += f32_bits_to_f64(__float_as_uint(lo[j]), ash);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = onto ? v[j] + x[j] : x[j];
         if (live) {
 #pragma unroll
           for (int j = 0; j < 16; ++j)
