@@ -1,18 +1,19 @@
 // FP64-accurate GEMM by exact digit products on the BF16 tensor cores (sm_103a).
 //
 // Persistent: one CTA per SM walks the (128-row tile, up to kOzN columns) tiles of the
-// problem list; six warps:
-//   warp 4 (one lane) streams the digit tiles with cp.async.bulk: per K tile, the
+// problem list; ten warps:
+//   warp 8 (one lane) streams the digit tiles with cp.async.bulk: per K tile, the
 //     kOzSlices B digit tiles into one of two B buffers, then the kOzSlices A digit
 //     tiles one by one through a ring of kOzStages stages;
-//   warp 5 (one lane) issues tcgen05.mma: A digit i times B digits j = 0 .. 6 - i into
+//   warp 9 (one lane) issues tcgen05.mma: A digit i times B digits j = 0 .. 6 - i into
 //     the tensor-memory accumulators of levels i + j, all j in one MMA over the stacked
 //     B digit tiles, and commits each stage back; chunks alternate between two sets of
 //     accumulators;
-//   warps 0-3 drain the kOzLevels accumulators after every K chunk (kOzChunkTiles K
+//   warps 0-7 drain the kOzLevels accumulators after every K chunk (kOzChunkTiles K
 //     tiles, short enough for every level sum to stay an exact FP32 integer) into two
 //     64-bit integer sums per row and column, beside the next chunk's MMAs, and after the
-//     tile's last chunk convert them to FP64 once, scale by 2^(eA + eB) and add into C.
+//     tile's last chunk round them to FP64 once, scale by 2^(eA + eB) and add into C; half of
+//     the columns in warps 0-3, the other half in warps 4-7.
 // Every wait is bounded: on expiry the waiting thread records an error code and raises
 // a shared abort flag that ends every other wait at once; the producer lets its own
 // copies land before the CTA frees its tensor memory and exits.
@@ -38,11 +39,35 @@ constexpr int kOzBars = 2 * kOzStages + 9;  // afull, aempty, bfull[2], bempty[2
 constexpr uint32_t kOzSet = kOzLevels * kOzN;  // tensor-memory columns of one set of accumulators
 static_assert(2 * kOzSet <= 512 && kOzSet <= 256, "two sets of accumulators, one MMA over all levels");
 constexpr size_t kOzSmem = kBarOff + kOzBars * 8 + 16;
-constexpr int kOzThreads = 192;
+constexpr int kOzThreads = 320;
+constexpr int kOzDrain = kOzN / 2;  // columns of a drain warp
 
-__device__ __forceinline__ double pow2(int e) {
-  e = max(-1022, min(1023, e));
-  return __longlong_as_double((long long)(e + 1023) << 52);
+// |ah 2^-38 + al 2^-62| 2^es (0 <= al < 2^24), rounded to FP64 once, to nearest even, as a bit
+// pattern without the sign.  Integers and no branches: converting and adding the two sums and
+// scaling took seven operations an element on the narrow FP64 pipe, 18000 cycles a tile, longer
+// than the MMAs of twenty K steps.  far: the sum is below 2^-46 or not a normal number.  (|ah| <
+// 2^55, up to 2^17 terms, leaves room for eight more bits.)
+// With eight drain warps in the place of four, a launch on the particle-hole channels of SNM 132
+// nmax=4 takes 1.85 instead of 2.99 ms and of PNM 66 nmax=4 0.17 instead of 0.34.
+__device__ __forceinline__ unsigned long long oz_round(long long ah, long long al, int es, bool &far) {
+  const bool neg = ah < 0;
+  const uint32_t l = neg ? (0u - (uint32_t)al) & 0xffffffu : (uint32_t)al;  // the magnitude of the pair
+  const unsigned long long h = ((neg ? ~(unsigned long long)ah + (l == 0) : (unsigned long long)ah) << 8) | (l >> 16);
+  const int z = __clzll((long long)h) & 63;
+  const unsigned long long low = (unsigned long long)l << 48;  // what follows the last bit of h
+  const unsigned long long n = (h << z) | (low >> 1 >> (63 - z));  // bits from the leading one on
+  const unsigned long long q = n >> 11;
+  // the remainder's ties go up when anything was left below or the last bit is odd
+  const bool up_tie = (low << z) != 0 || (q & 1);
+  const unsigned long long up = ((n & 0x7ffull) + (up_tie ? 0x400ull : 0x3ffull)) >> 11;
+  const int be = es + 1022 + 63 - 46 - z;  // biased exponent, less the one that q's leading bit adds
+  far |= (h == 0 && (l & 0xffffu) != 0) || (h != 0 && (unsigned)be > 2044u);
+  return h == 0 ? 0ull : ((unsigned long long)be << 52) + q + up;
+}
+// the same for any sum
+__device__ __noinline__ double oz_any(long long ah, long long al, int es) {
+  const double z = fma((double)ah, 0x1p-38, (double)al * 0x1p-62);
+  return ldexp(z, es);
 }
 
 __device__ __forceinline__ bool oz_tile_ok(const OzProb &P, const OzTile &tl) {
@@ -78,7 +103,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       mbar_init(smem_u32(&bfull[b]), 1);
       mbar_init(smem_u32(&bempty[b]), 1);
       mbar_init(smem_u32(&done[b]), 1);
-      mbar_init(smem_u32(&drained[b]), 4);
+      mbar_init(smem_u32(&drained[b]), 8);
     }
     mbar_init(smem_u32(fin), 1);
     *abort_flag = 0;
@@ -103,7 +128,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
     return true;
   };
 
-  if (warp == 4) {
+  if (warp == 8) {
     if (lane == 0) {  // producer
       int na[kOzStages] = {}, nb[2] = {0, 0};
       int cnt = 0, bk = 0;
@@ -147,7 +172,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       for (int b = 0; b < 2; ++b)
         if (nb[b]) mbar_wait(smem_u32(&bfull[b]), (uint32_t)((nb[b] - 1) & 1));
     }
-  } else if (warp == 5) {
+  } else if (warp == 9) {
     if (lane == 0) {  // MMA issuer
       int cnt = 0, bk = 0, ck = 0;
       bool ok = true;
@@ -199,30 +224,30 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       tc_commit(smem_u32(fin));
       mbar_wait(smem_u32(fin), 0);
     }
-  } else {  // warps 0-3: drain the level accumulators of every chunk, C once per tile
-    const int row = warp * 32 + lane;
-    const uint32_t tbase = tmem + ((uint32_t)(warp * 32) << 16);
+  } else {  // warps 0-7: drain the level accumulators of every chunk, C once per tile
+    const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * kOzDrain;
+    const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
     int ck = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
       const OzTile tl = tiles[t];
       const OzProb P = probs[tl.prob];
       if (!oz_tile_ok(P, tl)) continue;
-      const int nc = min(kOzN, P.npad - tl.n0), nk = P.nk;
+      const int nc = min(kOzN, P.npad - tl.n0) - c0, nk = P.nk;  // columns from c0 on
       const int nchunk = (nk + kOzChunkTiles - 1) / kOzChunkTiles;
       const int m = tl.mt * 128 + row;
       const bool live = m < P.M;
-      // a warp none of whose rows is stored skips the drain
-      const bool warp_live = tl.mt * 128 + warp * 32 < P.M;
+      // a warp none of whose rows or columns is stored skips the drain
+      const bool warp_live = tl.mt * 128 + (warp & 3) * 32 < P.M && nc > 0;
       // The tile's row sums so far as exact integers in units of 2^-38 (levels 0-3) and
       // 2^-62 (levels 4-6, kept below 2^24 by carrying into the first): each chunk adds
       // its level sums with integer operations only, so the accumulators are free again
       // after a few integer operations per level and column, and the
       // FP64 work (conversion, scaling, the read-modify-write of C) runs once per tile,
       // beside the next tile's MMAs.
-      long long ah[kOzN], al[kOzN];
+      long long ah[kOzDrain], al[kOzDrain];
 #pragma unroll
-      for (int q = 0; q < kOzN; ++q) ah[q] = al[q] = 0;
+      for (int q = 0; q < kOzDrain; ++q) ah[q] = al[q] = 0;
       for (int c = 0; c < nchunk; ++c, ++ck) {
         const bool got = __all_sync(0xffffffffu, wait(&done[ck & 1], (uint32_t)((ck >> 1) & 1)));
         if (!got) {
@@ -232,7 +257,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
         }
         tc_fence_after();
 #pragma unroll
-        for (int cb = 0; cb < kOzN; cb += 4) {
+        for (int cb = 0; cb < kOzDrain; cb += 4) {
           if (!warp_live || cb >= nc) break;
           // all levels of 4 columns in flight at once, one wait
           uint32_t r[kOzLevels][4];
@@ -256,32 +281,46 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&drained[ck & 1]));
 #pragma unroll
-        for (int q = 0; q < kOzN; ++q) {
+        for (int q = 0; q < kOzDrain; ++q) {
           const long long carry = al[q] >> 24;  // floor: al stays in [0, 2^24)
           ah[q] += carry;
           al[q] -= carry * (1ll << 24);
         }
       }
-      if (ok && live) {
-        const int eAm = P.eA[m];
-        double *crow = P.C + (int64_t)m * P.sCm;
+      if (ok && warp_live) {
+        // alpha is a sign and an exponent
+        const unsigned long long ab = (unsigned long long)__double_as_longlong(P.alpha);
+        const int eAm = (live ? P.eA[m] : 0) + (int)((ab >> 52) & 0x7ff) - 1023;
+        double *crow = P.C + (int64_t)m * P.sCm + (int64_t)(tl.n0 + c0) * P.sCn;
+        const int ncol = live ? min(nc, P.N - tl.n0 - c0) : 0;
+        const int *eB = P.eB + tl.n0 + c0;
         // 8 columns at a time: their loads of C in flight together, then the stores
 #pragma unroll
-        for (int q0 = 0; q0 < kOzN; q0 += 8) {
-          double old[8];
+        for (int q0 = 0; q0 < kOzDrain; q0 += 8) {
+          double old[8], x[8];
+          int es[8];
 #pragma unroll
-          for (int q = q0; q < q0 + 8; ++q) {
-            const int n = tl.n0 + q;
-            old[q - q0] = (q < nc && n < P.N) ? crow[(int64_t)n * P.sCn] : 0.0;
+          for (int q = 0; q < 8; ++q) {
+            old[q] = q0 + q < ncol ? crow[(int64_t)(q0 + q) * P.sCn] : 0.0;
+            es[q] = q0 + q < ncol ? eAm + eB[q0 + q] : 0;
           }
+          bool far = false;
 #pragma unroll
-          for (int q = q0; q < q0 + 8; ++q) {
-            const int n = tl.n0 + q;
-            if (q < nc && n < P.N) {
-              const double z = fma((double)ah[q], 0x1p-38, (double)al[q] * 0x1p-62);
-              crow[(int64_t)n * P.sCn] = old[q - q0] + P.alpha * (z * pow2(eAm + P.eB[n]));
+          for (int q = 0; q < 8; ++q) {
+            const long long h = q0 + q < ncol ? ah[q0 + q] : 0, l = q0 + q < ncol ? al[q0 + q] : 0;
+            const unsigned long long sign = ((unsigned long long)h ^ ab) & (1ull << 63);
+            x[q] = __longlong_as_double((long long)(oz_round(h, l, es[q], far) | sign));
+          }
+          if (__any_sync(0xffffffffu, far)) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const double y = oz_any(ah[q0 + q], al[q0 + q], es[q]);
+              x[q] = (ab >> 63) ? -y : y;
             }
           }
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (q0 + q < ncol) crow[(int64_t)(q0 + q) * P.sCn] = old[q] + x[q];
         }
       }
     }

@@ -46,7 +46,7 @@ struct OzProb {
   int M, N, nk, npad;
   double *C;           // C(m, n) += alpha * (A B)(m, n) at C[m * sCm + n * sCn]
   int64_t sCm, sCn;
-  double alpha;
+  double alpha;        // a power of two, of either sign
 };
 struct OzTile {
   int prob, mt, n0;    // 128-row tile mt, columns n0 .. n0 + min(kOzN, npad - n0)
