@@ -467,6 +467,21 @@ struct BitSplit {
     ex = e - 1075;
   }
   __device__ static void split(double x, uint32_t &hi, uint32_t &lo) {
+    if constexpr (NB == 8) {  // with 32-bit operations
+      const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+      const uint32_t w = (uint32_t)(u >> 32), v = (uint32_t)u, sign = w & 0x80000000u;
+      const int e = (int)((w >> 20) & 0x7ffu) - 896;
+      // |x| cut to the 24 bits of a float and the 29 bits below; hi from the float, whose bit 8
+      // decides the rounding; the remainder of hi is exact, and takes the lower bits rounded to 24
+      uint32_t f = ((w << 3) & 0x7ffff8u) | (v >> 29) | ((uint32_t)e << 23);
+      f = e <= 0 ? 0u : e >= 255 ? 0x7f800000u : f;  // below the float range; beyond it or not finite
+      const uint32_t h = (f + 0x8000u) & 0xffff0000u;
+      const float tail = __uint2float_rn(v & 0x1fffffffu) * 0x1p-52f, unit = __uint_as_float(f & 0x7f800000u);
+      const float rem = __fmaf_rn(tail, unit, __fsub_rn(__uint_as_float(f), __uint_as_float(h)));
+      hi = h | sign;
+      lo = ((__float_as_uint(rem) + 0x8000u) & 0xffff0000u) ^ sign;
+      return;
+    }
     uint32_t sign;
     unsigned long long sig;
     int ex;
