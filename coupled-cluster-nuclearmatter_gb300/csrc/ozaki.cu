@@ -1,19 +1,19 @@
 // FP64-accurate GEMM by exact digit products on the BF16 tensor cores (sm_103a).
 //
 // Persistent: one CTA per SM walks the (128-row tile, up to kOzN columns) tiles of the
-// problem list; ten warps:
-//   warp 8 (one lane) streams the digit tiles with cp.async.bulk: per K tile, the
+// problem list; eighteen warps:
+//   warp 16 (one lane) streams the digit tiles with cp.async.bulk: per K tile, the
 //     kOzSlices B digit tiles into one of two B buffers, then the kOzSlices A digit
 //     tiles one by one through a ring of kOzStages stages;
-//   warp 9 (one lane) issues tcgen05.mma: A digit i times B digits j = 0 .. 6 - i into
+//   warp 17 (one lane) issues tcgen05.mma: A digit i times B digits j = 0 .. 6 - i into
 //     the tensor-memory accumulators of levels i + j, all j in one MMA over the stacked
 //     B digit tiles, and commits each stage back; chunks alternate between two sets of
 //     accumulators;
-//   warps 0-7 drain the kOzLevels accumulators after every K chunk (kOzChunkTiles K
+//   warps 0-15 drain the kOzLevels accumulators after every K chunk (kOzChunkTiles K
 //     tiles, short enough for every level sum to stay an exact FP32 integer) into two
 //     64-bit integer sums per row and column, beside the next chunk's MMAs, and after the
-//     tile's last chunk round them to FP64 once, scale by 2^(eA + eB) and add into C; half of
-//     the columns in warps 0-3, the other half in warps 4-7.
+//     tile's last chunk round them to FP64 once, scale by 2^(eA + eB) and add into C; four
+//     warps for each eight columns.
 // Every wait is bounded: on expiry the waiting thread records an error code and raises
 // a shared abort flag that ends every other wait at once; the producer lets its own
 // copies land before the CTA frees its tensor memory and exits.
@@ -39,16 +39,17 @@ constexpr int kOzBars = 2 * kOzStages + 9;  // afull, aempty, bfull[2], bempty[2
 constexpr uint32_t kOzSet = kOzLevels * kOzN;  // tensor-memory columns of one set of accumulators
 static_assert(2 * kOzSet <= 512 && kOzSet <= 256, "two sets of accumulators, one MMA over all levels");
 constexpr size_t kOzSmem = kBarOff + kOzBars * 8 + 16;
-constexpr int kOzThreads = 320;
-constexpr int kOzDrain = kOzN / 2;  // columns of a drain warp
+constexpr int kOzThreads = 576;
+constexpr int kOzDrain = kOzN / 4;  // columns of a drain warp
 
 // |ah 2^-38 + al 2^-62| 2^es (0 <= al < 2^24), rounded to FP64 once, to nearest even, as a bit
 // pattern without the sign.  Integers and no branches: converting and adding the two sums and
 // scaling took seven operations an element on the narrow FP64 pipe, 18000 cycles a tile, longer
 // than the MMAs of twenty K steps.  far: the sum is below 2^-46 or not a normal number.  (|ah| <
 // 2^55, up to 2^17 terms, leaves room for eight more bits.)
-// With eight drain warps in the place of four, a launch on the particle-hole channels of SNM 132
-// nmax=4 takes 1.85 instead of 2.99 ms and of PNM 66 nmax=4 0.17 instead of 0.34.
+// With sixteen drain warps in the place of four, whose instructions wait for one another, a launch
+// on the particle-hole channels of PNM 66 nmax=4 takes 0.15 instead of 0.34 ms (eight: 0.17), of
+// SNM 132 nmax=4 1.87 instead of 2.99 (eight: 1.85).
 __device__ __forceinline__ unsigned long long oz_round(long long ah, long long al, int es, bool &far) {
   const bool neg = ah < 0;
   const uint32_t l = neg ? (0u - (uint32_t)al) & 0xffffffu : (uint32_t)al;  // the magnitude of the pair
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       mbar_init(smem_u32(&bfull[b]), 1);
       mbar_init(smem_u32(&bempty[b]), 1);
       mbar_init(smem_u32(&done[b]), 1);
-      mbar_init(smem_u32(&drained[b]), 8);
+      mbar_init(smem_u32(&drained[b]), 16);
     }
     mbar_init(smem_u32(fin), 1);
     *abort_flag = 0;
@@ -128,7 +129,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
     return true;
   };
 
-  if (warp == 8) {
+  if (warp == 16) {
     if (lane == 0) {  // producer
       int na[kOzStages] = {}, nb[2] = {0, 0};
       int cnt = 0, bk = 0;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       for (int b = 0; b < 2; ++b)
         if (nb[b]) mbar_wait(smem_u32(&bfull[b]), (uint32_t)((nb[b] - 1) & 1));
     }
-  } else if (warp == 9) {
+  } else if (warp == 17) {
     if (lane == 0) {  // MMA issuer
       int cnt = 0, bk = 0, ck = 0;
       bool ok = true;
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       tc_commit(smem_u32(fin));
       mbar_wait(smem_u32(fin), 0);
     }
-  } else {  // warps 0-7: drain the level accumulators of every chunk, C once per tile
+  } else {  // warps 0-15: drain the level accumulators of every chunk, C once per tile
     const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * kOzDrain;
     const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
     int ck = 0;
@@ -245,6 +246,17 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       // after a few integer operations per level and column, and the
       // FP64 work (conversion, scaling, the read-modify-write of C) runs once per tile,
       // beside the next tile's MMAs.
+      const int eAm = live && nc > 0 ? P.eA[m] : 0;
+      double *crow = P.C + (int64_t)m * P.sCm + (int64_t)(tl.n0 + c0) * P.sCn;
+      const int ncol = live ? min(nc, P.N - tl.n0 - c0) : 0;
+      // C and the exponents are read while the tile's products run
+      double old[kOzDrain];
+      int es[kOzDrain];
+#pragma unroll
+      for (int q = 0; q < kOzDrain; ++q) {
+        old[q] = q < ncol ? crow[(int64_t)q * P.sCn] : 0.0;
+        es[q] = q < ncol ? P.eB[tl.n0 + c0 + q] : 0;
+      }
       long long ah[kOzDrain], al[kOzDrain];
 #pragma unroll
       for (int q = 0; q < kOzDrain; ++q) ah[q] = al[q] = 0;
@@ -290,38 +302,25 @@ __global__ void __launch_bounds__(kOzThreads, 1) k_oz_gemm(const OzProb *__restr
       if (ok && warp_live) {
         // alpha is a sign and an exponent
         const unsigned long long ab = (unsigned long long)__double_as_longlong(P.alpha);
-        const int eAm = (live ? P.eA[m] : 0) + (int)((ab >> 52) & 0x7ff) - 1023;
-        double *crow = P.C + (int64_t)m * P.sCm + (int64_t)(tl.n0 + c0) * P.sCn;
-        const int ncol = live ? min(nc, P.N - tl.n0 - c0) : 0;
-        const int *eB = P.eB + tl.n0 + c0;
-        // 8 columns at a time: their loads of C in flight together, then the stores
+        const int eal = eAm + (int)((ab >> 52) & 0x7ff) - 1023;
+        double x[kOzDrain];
+        bool far = false;
 #pragma unroll
-        for (int q0 = 0; q0 < kOzDrain; q0 += 8) {
-          double old[8], x[8];
-          int es[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            old[q] = q0 + q < ncol ? crow[(int64_t)(q0 + q) * P.sCn] : 0.0;
-            es[q] = q0 + q < ncol ? eAm + eB[q0 + q] : 0;
-          }
-          bool far = false;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const long long h = q0 + q < ncol ? ah[q0 + q] : 0, l = q0 + q < ncol ? al[q0 + q] : 0;
-            const unsigned long long sign = ((unsigned long long)h ^ ab) & (1ull << 63);
-            x[q] = __longlong_as_double((long long)(oz_round(h, l, es[q], far) | sign));
-          }
-          if (__any_sync(0xffffffffu, far)) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const double y = oz_any(ah[q0 + q], al[q0 + q], es[q]);
-              x[q] = (ab >> 63) ? -y : y;
-            }
-          }
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            if (q0 + q < ncol) crow[(int64_t)(q0 + q) * P.sCn] = old[q] + x[q];
+        for (int q = 0; q < kOzDrain; ++q) {
+          const long long h = q < ncol ? ah[q] : 0, l = q < ncol ? al[q] : 0;
+          const unsigned long long sign = ((unsigned long long)h ^ ab) & (1ull << 63);
+          x[q] = __longlong_as_double((long long)(oz_round(h, l, eal + es[q], far) | sign));
         }
+        if (__any_sync(0xffffffffu, far)) {
+#pragma unroll
+          for (int q = 0; q < kOzDrain; ++q) {
+            const double y = oz_any(ah[q], al[q], eal + es[q]);
+            x[q] = (ab >> 63) ? -y : y;
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < kOzDrain; ++q)
+          if (q < ncol) crow[(int64_t)q * P.sCn] = old[q] + x[q];
       }
     }
   }

@@ -5,12 +5,12 @@
 // Persistent: one CTA per SM walks the tile list (a tile = 128 rows of one problem, all N
 // <= 256 columns); a tile may sum up to six products with the same M, N (segments), each
 // added or subtracted.
-// Lane 0 of warp 8 streams the pre-tiled K tiles of A and B into a ring of shared-memory
+// Lane 0 of warp 16 streams the pre-tiled K tiles of A and B into a ring of shared-memory
 // stages with cp.async.bulk (one contiguous copy per operand tile, completion on an
-// mbarrier); the ring runs on across tiles.  Lane 0 of warp 9 issues the MMAs into one
+// mbarrier); the ring runs on across tiles.  Lane 0 of warp 17 issues the MMAs into one
 // of two tensor-memory halves, alternating by tile, and tcgen05.commit hands each stage
-// back.  Warps 0-3 drain the tiles of half 0 and warps 4-7 those of half 1: each reads
-// its 32 TMEM lanes (rows) with tcgen05.ld and adds into C while the next tile
+// back.  Eight warps drain the tiles of either half: each reads 32 TMEM lanes (rows) and
+// every other group of columns with tcgen05.ld and adds into C while the next tile
 // accumulates in the other half.
 // Every mbarrier wait is bounded by a clock budget: on expiry the kernel records an
 // error code, lets its own copies land, frees its TMEM and returns.
@@ -29,7 +29,8 @@ namespace {
 
 using namespace tcptx;
 
-constexpr int kTcThreads = 320;   // warps 0-7 epilogue, warp 8 producer, warp 9 MMA issuer
+constexpr int kTcThreads = 576;   // warps 0-15 epilogue, warp 16 producer, warp 17 MMA issuer
+constexpr int kTcCols = 8;        // columns that an epilogue warp reads at a time
 constexpr int kTcHalfCols = 256;  // tensor-memory columns of one accumulator half
 constexpr int kTcMaxStages = 8;
 
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&tfull[b]), 1);
-      mbar_init(smem_u32(&tempty[b]), 4);  // the four warps of drain group b
+      mbar_init(smem_u32(&tempty[b]), 8);  // the eight warps of drain group b
     }
     mbar_init(smem_u32(fin), 1);
     *abort_flag = 0;
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
     return true;
   };
 
-  if (warp == 8) {
+  if (warp == 16) {
     if (lane == 0) {
       // producer: one bulk copy per operand tile into the stage ring, which runs on
       // across tiles; a stage is refilled once the MMAs that read it have completed
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
         if (n_s > 0) mbar_wait(smem_u32(&full[s]), (uint32_t)((n_s - 1) & 1));
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == 17) {
     if (lane == 0) {
       // MMA issuer: the K tiles of every segment of a tile into its accumulators in
       // tensor-memory half b = (local tile) & 1, then tcgen05.commit to tfull[b]
@@ -268,9 +269,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
       mbar_wait(smem_u32(fin), 0);
     }
   } else {
-    // warps 0-7: two groups of four, group g draining the tiles of tensor-memory half g,
-    // so two tiles' C updates are in flight; warp w reads lanes 32 (w % 4) .. + 31
-    const int grp = warp >> 2, quad = warp & 3;
+    // warps 0-15: two groups of eight, group g draining the tiles of tensor-memory half g,
+    // so two tiles' C updates are in flight; warp w reads lanes 32 (w % 4) .. + 31, and two
+    // warps share the columns of each
+    const int grp = (warp >> 2) & 1, quad = warp & 3, sub = warp >> 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
     int lt = 0;
@@ -306,64 +308,58 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
         continue;
       }
       const uint32_t accb = lane_base + (uint32_t)(b * kTcHalfCols);
-      // 16 columns at a time: the registers of 32 would spill
-      for (int c0 = 0; c0 < G.npad; c0 += 16) {
+      for (int c0 = sub * kTcCols; c0 < G.npad; c0 += 2 * kTcCols) {
         // the C and C0 loads go first, so that their latency overlaps the tensor-memory
         // reads; the mode is uniform over the tile, so the branches sit outside the
-        // unrolled loops and the 16 loads of a row issue back to back
-        double v[16];
+        // unrolled loops and the loads of a row issue back to back
+        double v[kTcCols];
         if (live && keep) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = (c0 + j < nvalid) ? crow[(int64_t)(c0 + j) * sCn] : 0.0;
+          for (int j = 0; j < kTcCols; ++j) v[j] = (c0 + j < nvalid) ? crow[(int64_t)(c0 + j) * sCn] : 0.0;
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0.0;
+          for (int j = 0; j < kTcCols; ++j) v[j] = 0.0;
         }
+        double add[kTcCols];
         if (live && c0row) {
-          double add[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) add[j] = (c0 + j < nvalid) ? c0row[(int64_t)(c0 + j) * sCn] : 0.0;
-          if (keep) {
+          for (int j = 0; j < kTcCols; ++j) add[j] = (c0 + j < nvalid) ? c0row[(int64_t)(c0 + j) * sCn] : 0.0;
+        } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] += add[j];
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = add[j];
-          }
+          for (int j = 0; j < kTcCols; ++j) add[j] = 0.0;
         }
         // The accumulators are summed as pairs of FP32 numbers (48 bits, against the 24 of each
         // accumulator) and rounded to FP64 as integers without branches: one FP64 addition an
         // element where it is added onto something, else none.  The drain warps bound the
         // launches on the particle-hole channels: a multiply-add in FP64 for each accumulator
         // took 1.16 ms for dR_ph of SNM 132 nmax=4 (four accumulators) and 1.03 for dI4 (two),
-        // pairs with a branching conversion and an FP64 addition 1.00 and 1.03, now 0.77 and
-        // 0.81; PNM 66 nmax=4 140 and 93, 136 and 96, now 95 and 69 us.  Reading two accumulators
-        // for each wait costs 1 % of a solve.
-        float hi[16], lo[16];
+        // integers 0.77 and 0.81 in eight warps of 16 columns at a time, now 0.73 and 0.76;
+        // PNM 66 nmax=4 140 and 93, 95 and 69, now 79 and 55 us.  Sixteen warps, because the
+        // instructions of a warp wait for one another.
+        float hi[kTcCols], lo[kTcCols];
         for (int a = 0; a < G.nacc; ++a) {
-          uint32_t r[16];
-          tmem_ld16(accb + (uint32_t)(a * G.ncols + c0), r);
+          uint32_t r[kTcCols];
+          tmem_ld8(accb + (uint32_t)(a * G.ncols + c0), r);
           tmem_ld_wait();
           if (a == 0) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) { hi[j] = __uint_as_float(r[j]); lo[j] = 0.0f; }
+            for (int j = 0; j < kTcCols; ++j) { hi[j] = __uint_as_float(r[j]); lo[j] = 0.0f; }
           } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) pair_add(hi[j], lo[j], __uint_as_float(r[j]));
+            for (int j = 0; j < kTcCols; ++j) pair_add(hi[j], lo[j], __uint_as_float(r[j]));
           }
         }
-        if (c0 + 16 >= G.npad) {
+        if (c0 + 2 * kTcCols >= G.npad) {
           // the accumulators of this half are read: hand it back to the MMA issuer
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&tempty[b]));
         }
-        const bool onto = keep || c0row;
         bool odd = false;
-        double x[16];
+        double x[kTcCols];
         if (G.nacc > 1) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
+          for (int j = 0; j < kTcCols; ++j) {
             // the pair's own sum first; infinities stay infinities
             const float l = fabsf(hi[j]) < __int_as_float(0x7f800000) ? lo[j] : 0.0f;
             lo[j] = 0.0f;
@@ -372,23 +368,31 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
+          for (int j = 0; j < kTcCols; ++j) {
             const uint32_t u = __float_as_uint(hi[j]);
             x[j] = __longlong_as_double((long long)(f32_widen(u, ash, odd) | ((unsigned long long)(u & 0x80000000u) << 32)));
           }
         }
         if (__any_sync(0xffffffffu, odd && live)) {  // a subnormal, an infinity or a NaN
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
+          for (int j = 0; j < kTcCols; ++j) {
             x[j] = f32_bits_to_f64(__float_as_uint(hi[j]), ash);
             if (isfinite(hi[j])) x[j] += f32_bits_to_f64(__float_as_uint(lo[j]), ash);
           }
         }
+        if (keep && c0row) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = onto ? v[j] + x[j] : x[j];
+          for (int j = 0; j < kTcCols; ++j) v[j] = (v[j] + add[j]) + x[j];
+        } else if (keep || c0row) {
+#pragma unroll
+          for (int j = 0; j < kTcCols; ++j) v[j] = (keep ? v[j] : add[j]) + x[j];
+        } else {
+#pragma unroll
+          for (int j = 0; j < kTcCols; ++j) v[j] = x[j];
+        }
         if (live) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j)
+          for (int j = 0; j < kTcCols; ++j)
             if (c0 + j < nvalid) crow[(int64_t)(c0 + j) * sCn] = v[j];
         }
       }
