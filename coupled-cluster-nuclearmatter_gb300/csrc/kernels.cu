@@ -600,20 +600,24 @@ __device__ __forceinline__ S at_or_zero(const S *__restrict__ X, int m) {
   return m ? X[m - 1] : S(0.0);
 }
 
-// R' = conj(V) + the one-body I6 / I7 terms + the ring scatter, through the maps
+// R' = conj(V) + the one-body I6 / I7 terms + the ring scatter, through the maps.  A block takes a
+// quarter of a tile, one element a thread: four elements one after the other were four chains of
+// dependent reads.  PNM 14 nmax=1 15 to 7.2 us, a twist of SNM 76 nmax=2 39 to 28; SNM 132 nmax=4
+// (630 us) is bound by the sectors of its eight random reads either way.
+constexpr int kTileParts = kTileElems / 256;
 template <typename S>
 __global__ void k_rinit(DevLayout L, const int4 *__restrict__ omap, const int4 *__restrict__ rmap, const S *__restrict__ T,
                         const S *__restrict__ Vhp, const S *__restrict__ Rph, const S *__restrict__ i6off,
                         const S *__restrict__ i7off, const S *__restrict__ ring_base, S *__restrict__ ring_out,
                         int add, S *__restrict__ R) {
-  const int2 tl = L.ttile[blockIdx.x];
+  const int2 tl = L.ttile[blockIdx.x / kTileParts];
   const int ch = tl.x;
   const int P = L.P[ch], H = L.H[ch];
   const int n = P * H;  // < 2^31 per channel
-  const int end = min(tl.y + kTileElems, n);
   const int A = L.A;
   const int64_t base = L.t_off[ch];
-  for (int e = tl.y + threadIdx.x; e < end; e += blockDim.x) {
+  const int e = tl.y + blockIdx.x % kTileParts * 256 + threadIdx.x;
+  if (e < n) {
     const int4 o = omap[base + e];
     const int4 m = rmap[base + e];
     S r = conj_(Vhp[base + e]);
@@ -639,7 +643,7 @@ template <typename S>
 void launch_rinit(const DevLayout &L, const int4 *omap, const int4 *rmap, const S *T, const S *Vhp, const S *Rph,
                   const S *i6off, const S *i7off, const S *ring_base, S *ring_out, bool add, S *R, cudaStream_t st) {
   if (L.nttile)
-    k_rinit<S><<<L.nttile, 256, 0, st>>>(L, omap, rmap, T, Vhp, Rph, i6off, i7off, ring_base, ring_out, add, R);
+    k_rinit<S><<<L.nttile * kTileParts, 256, 0, st>>>(L, omap, rmap, T, Vhp, Rph, i6off, i7off, ring_base, ring_out, add, R);
 }
 
 // ============================================================================
@@ -786,7 +790,7 @@ __global__ void __launch_bounds__(256) k_update_std(DevLayout L, const S *__rest
                                                     const S *__restrict__ d2ab, S *__restrict__ hist_t,
                                                     typename StepOf<S>::type *__restrict__ hist_e,
                                                     PtrPack<typename StepOf<S>::type> es, int nb, int self,
-                                                    const int *err, double *partial) {
+                                                    const int *err, int parts, double *partial) {
   using E = typename StepOf<S>::type;
   __shared__ S sdij[kTileElems];  // hole-pair sums of one tile (at most kTileElems rows)
   __shared__ double red[kUpdStdNV][8];
@@ -795,11 +799,14 @@ __global__ void __launch_bounds__(256) k_update_std(DevLayout L, const S *__rest
 #pragma unroll
   for (int k = 0; k < kMaxDots; ++k) f[k] = 0.0f;
   const int A = L.A;
-  for (int tix = blockIdx.x; tix < L.nttile; tix += gridDim.x) {
-    const int2 tl = L.ttile[tix];
+  const int span = kTileElems / parts;
+  for (int tix = blockIdx.x; tix < L.nttile * parts; tix += gridDim.x) {
+    int2 tl = L.ttile[tix / parts];
     const int ch = tl.x;
     const int P = L.P[ch];
-    const int end = min(tl.y + kTileElems, P * L.H[ch]);
+    tl.y += tix % parts * span;
+    const int end = min(tl.y + span, P * L.H[ch]);
+    if (tl.y >= end) continue;  // (uniform over the block)
     const int ij0 = tl.y / P, nij = (end - 1) / P - ij0 + 1;
     __syncthreads();  // the previous tile's sums are no longer read
     for (int i = threadIdx.x; i < nij; i += blockDim.x) {
@@ -861,8 +868,11 @@ void launch_update_std(const DevLayout &L, const S *T, const S *R, const S *Vhp,
   if (!L.nttile) return;
   PtrPack<typename StepOf<S>::type> pk{};
   for (int k = 0; k < nb; ++k) pk.p[k] = es[k];
-  const int blocks = std::min(L.nttile, kUpdStdBlocks);
-  k_update_std<S><<<blocks, 256, 0, st>>>(L, T, R, Vhp, d2ij, d2ab, hist_t, hist_e, pk, nb, self, err, partial);
+  // quarters of a tile, one element a thread, while a block has no more than one of them: PNM 14
+  // nmax=1 20 to 11 us; at 400 tiles (SNM 76 nmax=2) 39 us whole and 40 in quarters
+  const int parts = L.nttile * kTileParts <= kUpdStdBlocks ? kTileParts : 1;
+  const int blocks = std::min(L.nttile * parts, kUpdStdBlocks);
+  k_update_std<S><<<blocks, 256, 0, st>>>(L, T, R, Vhp, d2ij, d2ab, hist_t, hist_e, pk, nb, self, err, parts, partial);
   finish(partial, blocks, kUpdStdNV, out, st);
 }
 
