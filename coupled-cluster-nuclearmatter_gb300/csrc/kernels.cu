@@ -602,7 +602,7 @@ __device__ __forceinline__ S at_or_zero(const S *__restrict__ X, int m) {
 
 // R' = conj(V) + the one-body I6 / I7 terms + the ring scatter, through the maps.  A block takes a
 // quarter of a tile, one element a thread: four elements one after the other were four chains of
-// dependent reads.  PNM 14 nmax=1 15 to 7.2 us, a twist of SNM 76 nmax=2 39 to 28; SNM 132 nmax=4
+// dependent reads.  PNM 14 nmax=2 15 to 7.2 us, a twist of SNM 76 nmax=2 39 to 28; SNM 132 nmax=4
 // (630 us) is bound by the sectors of its eight random reads either way.
 constexpr int kTileParts = kTileElems / 256;
 template <typename S>
@@ -869,7 +869,7 @@ void launch_update_std(const DevLayout &L, const S *T, const S *R, const S *Vhp,
   PtrPack<typename StepOf<S>::type> pk{};
   for (int k = 0; k < nb; ++k) pk.p[k] = es[k];
   // quarters of a tile, one element a thread, while a block has no more than one of them: PNM 14
-  // nmax=1 20 to 11 us; at 400 tiles (SNM 76 nmax=2) 39 us whole and 40 in quarters
+  // nmax=2 20 to 11 us; at 400 tiles (SNM 76 nmax=2) 39 us whole and 40 in quarters
   const int parts = L.nttile * kTileParts <= kUpdStdBlocks ? kTileParts : 1;
   const int blocks = std::min(L.nttile * parts, kUpdStdBlocks);
   k_update_std<S><<<blocks, 256, 0, st>>>(L, T, R, Vhp, d2ij, d2ab, hist_t, hist_e, pk, nb, self, err, parts, partial);
