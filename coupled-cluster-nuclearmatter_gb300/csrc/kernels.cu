@@ -760,7 +760,10 @@ void launch_dots(int64_t n, const S *a, const S *const *bs, int nb, int conj_a, 
 // Re(conj(step) hist_e[j]) in FP32 per thread (FP64 across warps and blocks).  One pass,
 // one launch and one host copy per iteration instead of an update and a dots pass.  The
 // FP32 step vanishes with the residual, so the fixed point is the FP64 one.
-constexpr int kUpdStdBlocks = 608;
+// The blocks that run at once: the registers allow five an SM for real engines and four for complex
+// ones.  A tile is a chain of dependent reads, so blocks in flight count: PNM 66 nmax=4 (2064 tiles)
+// 79 us with four an SM, 66 with five; six, with 40 registers, 66.
+template <typename S> constexpr int kUpdStdBlocks = (ScalarOf<S>::complex ? 4 : 5) * 152;
 constexpr int kUpdStdNV = 4 + kMaxDots;  // E re, E im, |q|^2, error word, Gram row
 __device__ inline float warp_sum_f(float x) {
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -870,8 +873,8 @@ void launch_update_std(const DevLayout &L, const S *T, const S *R, const S *Vhp,
   for (int k = 0; k < nb; ++k) pk.p[k] = es[k];
   // quarters of a tile, one element a thread, while a block has no more than one of them: PNM 14
   // nmax=2 20 to 11 us; at 400 tiles (SNM 76 nmax=2) 39 us whole and 40 in quarters
-  const int parts = L.nttile * kTileParts <= kUpdStdBlocks ? kTileParts : 1;
-  const int blocks = std::min(L.nttile * parts, kUpdStdBlocks);
+  const int parts = L.nttile * kTileParts <= kUpdStdBlocks<S> ? kTileParts : 1;
+  const int blocks = std::min(L.nttile * parts, kUpdStdBlocks<S>);
   k_update_std<S><<<blocks, 256, 0, st>>>(L, T, R, Vhp, d2ij, d2ab, hist_t, hist_e, pk, nb, self, err, parts, partial);
   finish(partial, blocks, kUpdStdNV, out, st);
 }

@@ -104,7 +104,7 @@ void launch_dots(int64_t n, const S *a, const S *const *bs, int nb, int conj_a, 
 // mode-1 update and the Gram row of its step in one pass:
 // out[0] = E (re), out[1] = E (im, 0 for real engines), out[2] = |R - D T|^2, out[3] = *err (0 when err is null),
 // out[4 + j] = Re(conj(step) . es[j]) for j < nb (1 <= nb <= 16); es[self] is hist_e, the step
-// this pass writes.  partial holds 20 doubles for each of up to 608 blocks.
+// this pass writes.  partial holds 20 doubles for each of up to 760 blocks.
 template <typename S>
 void launch_update_std(const DevLayout &L, const S *T, const S *R, const S *Vhp, const S *d2ij, const S *d2ab, S *hist_t,
                        typename StepOf<S>::type *hist_e, const typename StepOf<S>::type *const *es, int nb, int self,
