@@ -103,8 +103,11 @@ __device__ __forceinline__ double wnorm2(cplx w) { return w.re * w.re + w.im * w
 // FP32 contractions the ratio is formed in FP32 (its rounding, 6e-8 of the term, is far below the
 // FP32 contractions' own) from a denominator that keeps FP64's accuracy to there, and the sum
 // has FP64's: both as pairs of FP32 numbers, since an FP64 operation costs 64 FP32 ones on this
-// GPU and a pair needs six of them.
+// GPU and a pair needs six of them.  A pair holds at most 64 terms a round (kFlush steps) and is
+// then added to an FP64 sum: over a whole lattice it would lose the many terms below 2^-48 of it,
+// all of one sign (SNM 132 nmax=3, 3.4e10 terms: 6e-9 of the sum).
 template <typename S, typename W> struct TripleSum;
+constexpr int kFlush = 16;  // a power of two; the additions cost 1.5 % of the sum's time at 16
 // n1 / d1 + n2 / d2 as one fraction: an FP64 division costs some ten operations of the FP64
 // pipe, three multiplications and an addition are cheaper
 __device__ __forceinline__ void add_fractions(double n1, double d1, double n2, double d2, double &n, double &d) {
@@ -128,6 +131,7 @@ template <> struct TripleSum<double, double> {
     add_fractions(n2[0], d2[0], n2[1], d2[1], nn, dd);
     re += nn / dd;
   }
+  __device__ __forceinline__ void flush() {}
   __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = re; v[1] = 0.0; }
 };
 template <> struct TripleSum<cplx, cplx> {
@@ -144,6 +148,7 @@ template <> struct TripleSum<cplx, cplx> {
         s.im = fma(-r, d.im, s.im);
       }
   }
+  __device__ __forceinline__ void flush() {}
   __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = s.re; v[1] = s.im; }
 };
 __device__ __forceinline__ float2 two_floats(double x) {
@@ -165,17 +170,23 @@ __device__ __forceinline__ float two_sub(float2 h, float2 p) {
 template <> struct TripleSum<double, float> {
   using Fock = float2;
   float hi = 0.0f, lo = 0.0f;
+  double re = 0.0;
   static __device__ __forceinline__ Fock fock(double f) { return two_floats(f); }
   __device__ __forceinline__ void add(const float (&w)[4], const Fock (&h)[4], const Fock (&p)[4], const bool (&live)[4]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (live[q]) two_add(hi, lo, (w[q] * w[q]) / two_sub(h[q], p[q]));
   }
-  __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = (double)hi + (double)lo; v[1] = 0.0; }
+  __device__ __forceinline__ void flush() {
+    re += (double)hi + (double)lo;
+    hi = lo = 0.0f;
+  }
+  __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = re; v[1] = 0.0; }
 };
 template <> struct TripleSum<cplx, cplxf> {
   using Fock = float4;
   float hr = 0.0f, lr = 0.0f, hi = 0.0f, li = 0.0f;
+  double re = 0.0, im = 0.0;
   static __device__ __forceinline__ Fock fock(cplx f) {
     const float2 a = two_floats(f.re), b = two_floats(f.im);
     return make_float4(a.x, a.y, b.x, b.y);
@@ -194,10 +205,12 @@ template <> struct TripleSum<cplx, cplxf> {
         two_add(hi, li, -s * di);
       }
   }
-  __device__ __forceinline__ void total(double (&v)[2]) const {
-    v[0] = (double)hr + (double)lr;
-    v[1] = (double)hi + (double)li;
+  __device__ __forceinline__ void flush() {
+    re += (double)hr + (double)lr;
+    im += (double)hi + (double)li;
+    hr = lr = hi = li = 0.0f;
   }
+  __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = re; v[1] = im; }
 };
 
 // FP32 copy of an FP64 array
@@ -241,7 +254,7 @@ constexpr unsigned long long kTermOrder = 0x596A84210ull;
 // Gathering the factors pair by pair through slot tables, 36 gathers of some ten dependent
 // loads each, kept the integer pipe and L1 busy and the FP32 pipe idle.  ms before and now, FP32
 // / FP64 contractions: PNM 14 nmax=2 0.32 to 0.21 / 0.36 to 0.34, PNM 54 nmax=2 8.5 to 2.0 / 9.0
-// to 4.2, SNM 28 nmax=2 6.8 to 1.5 / 12.8 to 10.2, SNM 76 nmax=2 (6.3e8 pairs) 88.5 to 10.5 /
+// to 4.2, SNM 28 nmax=2 6.8 to 1.5 / 12.8 to 10.2, SNM 76 nmax=2 (6.3e8 pairs) 88.5 to 10.6 /
 // 171 to 83.5.  FP32 issues 2 of 4 instructions a clock, the rest is the latency of the gathers and
 // barriers; FP64 is bound by its pipe.
 template <typename W> struct alignas(2 * sizeof(W)) SpinPair {
@@ -548,12 +561,14 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
 #pragma unroll
         for (int r = 0; r < Sh::kRounds; ++r)
           pairs(mine[r], st, st % 3, tab + (Sh::kBuffers == 2 ? (size_t)(st & 1) * KB * 36 * CU : 0));
+        if ((st & (kFlush - 1)) == kFlush - 1) sum.flush();
         __syncthreads();
         if (Sh::kBuffers == 1 && st + 1 < steps) {
           build(st + 1, (st + 1) % 3, tab);
           __syncthreads();
         }
       }
+      sum.flush();
     }
   }
   double acc[2];
