@@ -1318,14 +1318,14 @@ class Engine final : public IEngine {
     for (int p = 0; p < 3; ++p) {
       double t[2];
       for (int v = 0; v < 2; ++v) {
-        plans[p]->merged[0] = plans[p]->merged[1] = v;
+        plans[p]->merged = v;
         float best = 1e30f;
         for (int rep = 0; rep < 3; ++rep) best = std::min(best, ev.time(st_, [&] { run_tc(*plans[p]); }));
         t[v] = best;
         ms[2 * p + v] = best;
       }
       const int pick = t[1] <= t[0] ? 1 : 0;
-      plans[p]->merged[0] = plans[p]->merged[1] = pick;
+      plans[p]->merged = pick;
       tc_choice_[p] = pick;
       merged[p] = pick;
     }
@@ -1816,11 +1816,11 @@ class Engine final : public IEngine {
   }
 
   // ================================================================== mixed precision
-  // Tensor-core products on FP64 data of either scalar kind.  A real product is one
-  // problem.  A complex product C += a A B becomes four real ones on the re / im parts
-  // of the interleaved operands, in two launch phases so that no two CTAs update the
-  // same C entries at once: phase 0 C_re += a Are Bre, C_im += a Are Bim; phase 1
-  // C_re -= a Aim Bim, C_im += a Aim Bre.
+  // Tensor-core products on FP64 data of either scalar kind.  A real product is one problem.
+  // A complex correction is one problem for each component of C, with the products that are
+  // subtracted marked so.  A complex digit product becomes four real ones in two launch phases, so
+  // that no two CTAs update the same C entries at once: phase 0 C_re += a Are Bre, C_im += a Are
+  // Bim; phase 1 C_re -= a Aim Bim, C_im += a Aim Bre.
   static constexpr int kNComp = ScalarOf<S>::complex ? 2 : 1;
   // Tiles bucketed by padded N, so that small problems run with small shared-memory
   // stages (and more CTAs per SM) instead of the largest problem's footprint.
@@ -1831,10 +1831,10 @@ class Engine final : public IEngine {
   // launch form per phase: one launch by default; the tensor-core autotuner times both.
   struct TcPlan {
     DBuf probs;
-    DBuf tiles[2][kTcBuckets], tiles_m[2];
-    int ntiles[2][kTcBuckets] = {}, npad_max[2][kTcBuckets] = {}, max_nk[2][kTcBuckets] = {};
-    int ntiles_m[2] = {0, 0}, npad_m[2] = {16, 16}, nk_m[2] = {1, 1};
-    int merged[2] = {0, 0};
+    DBuf tiles[kTcBuckets], tiles_m;
+    int ntiles[kTcBuckets] = {}, npad_max[kTcBuckets] = {}, max_nk[kTcBuckets] = {};
+    int ntiles_m = 0, npad_m = 16, nk_m = 1;
+    int merged = 0;
   };
   struct SplitPlan {
     DBuf jobs, chunks;
@@ -1844,54 +1844,47 @@ class Engine final : public IEngine {
     DBuf hi, lo;
     int64_t n = 0;  // elements of one scalar component; the buffer holds kNComp of them
   };
-  // problems, their launch phase and their row tiles, built on the host
+  // problems and their row tiles, built on the host
   struct TcList {
     std::vector<TcProb> probs;
-    std::vector<int> phase;
     std::vector<TcTile> tiles;
   };
   void finalize_tc(TcPlan &pl, const TcList &l, int choice = -1) {
     upload(pl.probs, l.probs, &bytes_);
-    std::vector<TcTile> b[2][kTcBuckets], m[2];
-    for (int ph = 0; ph < 2; ++ph)
-      for (int k = 0; k < kTcBuckets; ++k) { pl.npad_max[ph][k] = 16; pl.max_nk[ph][k] = 1; }
-    for (const TcTile &t : l.tiles) {
-      const TcProb &p = l.probs[t.prob];
-      const int ph = l.phase[t.prob];
-      const int k = p.npad <= 32 ? 0 : p.npad <= 64 ? 1 : p.npad <= 128 ? 2 : 3;
-      b[ph][k].push_back(t);
-      m[ph].push_back(t);
-      int nk = p.nk;
-      for (int e = 0; e < p.next; ++e) nk += p.ext[e].nk;
-      pl.npad_max[ph][k] = std::max(pl.npad_max[ph][k], p.npad);
-      pl.max_nk[ph][k] = std::max(pl.max_nk[ph][k], nk);
-    }
-    // longest tiles first: the persistent CTAs take tiles in strides of the grid
+    std::vector<TcTile> b[kTcBuckets], m;
+    for (int k = 0; k < kTcBuckets; ++k) { pl.npad_max[k] = 16; pl.max_nk[k] = 1; }
     auto work = [&](const TcTile &t) {
       const TcProb &p = l.probs[t.prob];
       int nk = p.nk;
       for (int e = 0; e < p.next; ++e) nk += p.ext[e].nk;
       return nk;
     };
-    auto by_work = [&](const TcTile &x, const TcTile &y) { return work(x) > work(y); };
-    for (int ph = 0; ph < 2; ++ph) {
-      int np = 16, nk = 1;
-      for (int k = 0; k < kTcBuckets; ++k) {
-        std::stable_sort(b[ph][k].begin(), b[ph][k].end(), by_work);
-        upload(pl.tiles[ph][k], b[ph][k], &bytes_);
-        pl.ntiles[ph][k] = (int)b[ph][k].size();
-        if (!b[ph][k].empty()) { np = std::max(np, pl.npad_max[ph][k]); nk = std::max(nk, pl.max_nk[ph][k]); }
-      }
-      std::stable_sort(m[ph].begin(), m[ph].end(), by_work);
-      upload(pl.tiles_m[ph], m[ph], &bytes_);
-      pl.ntiles_m[ph] = (int)m[ph].size();
-      pl.npad_m[ph] = np;
-      pl.nk_m[ph] = nk;
-      // one launch unless the autotuner found the bucket launches faster: the persistent
-      // grid then has no tail per bucket, and on every lattice measured it won even where
-      // the widest tile leaves the kernel only two shared-memory stages
-      pl.merged[ph] = choice >= 0 ? choice : 1;
+    for (const TcTile &t : l.tiles) {
+      const TcProb &p = l.probs[t.prob];
+      const int k = p.npad <= 32 ? 0 : p.npad <= 64 ? 1 : p.npad <= 128 ? 2 : 3;
+      b[k].push_back(t);
+      m.push_back(t);
+      pl.npad_max[k] = std::max(pl.npad_max[k], p.npad);
+      pl.max_nk[k] = std::max(pl.max_nk[k], work(t));
     }
+    // longest tiles first: the persistent CTAs take tiles in strides of the grid
+    auto by_work = [&](const TcTile &x, const TcTile &y) { return work(x) > work(y); };
+    int np = 16, nk = 1;
+    for (int k = 0; k < kTcBuckets; ++k) {
+      std::stable_sort(b[k].begin(), b[k].end(), by_work);
+      upload(pl.tiles[k], b[k], &bytes_);
+      pl.ntiles[k] = (int)b[k].size();
+      if (!b[k].empty()) { np = std::max(np, pl.npad_max[k]); nk = std::max(nk, pl.max_nk[k]); }
+    }
+    std::stable_sort(m.begin(), m.end(), by_work);
+    upload(pl.tiles_m, m, &bytes_);
+    pl.ntiles_m = (int)m.size();
+    pl.npad_m = np;
+    pl.nk_m = nk;
+    // one launch unless the autotuner found the bucket launches faster: the persistent
+    // grid then has no tail per bucket, and on every lattice measured it won even where
+    // the widest tile leaves the kernel only two shared-memory stages
+    pl.merged = choice >= 0 ? choice : 1;
   }
   void finalize_split(SplitPlan &pl, const std::vector<TcSplitJob> &jobs) {
     upload(pl.jobs, jobs, &bytes_);
@@ -1900,20 +1893,18 @@ class Engine final : public IEngine {
     pl.nchunks = (int)ch.size();
   }
   void run_tc(const TcPlan &pl) {
-    for (int ph = 0; ph < 2; ++ph) {
-      if (pl.merged[ph]) {
-        if (!pl.ntiles_m[ph]) continue;
-        launch_tc_gemm(tc_kind_, (const TcProb *)pl.probs.p, (const TcTile *)pl.tiles_m[ph].p, pl.ntiles_m[ph],
-                       pl.npad_m[ph], pl.nk_m[ph], tcerr_.as<int>(), st_);
-        ++launches_;
-        continue;
-      }
-      for (int k = 0; k < kTcBuckets; ++k) {
-        if (!pl.ntiles[ph][k]) continue;
-        launch_tc_gemm(tc_kind_, (const TcProb *)pl.probs.p, (const TcTile *)pl.tiles[ph][k].p, pl.ntiles[ph][k],
-                       pl.npad_max[ph][k], pl.max_nk[ph][k], tcerr_.as<int>(), st_);
-        ++launches_;
-      }
+    if (pl.merged) {
+      if (!pl.ntiles_m) return;
+      launch_tc_gemm(tc_kind_, (const TcProb *)pl.probs.p, (const TcTile *)pl.tiles_m.p, pl.ntiles_m, pl.npad_m, pl.nk_m,
+                     tcerr_.as<int>(), st_);
+      ++launches_;
+      return;
+    }
+    for (int k = 0; k < kTcBuckets; ++k) {
+      if (!pl.ntiles[k]) continue;
+      launch_tc_gemm(tc_kind_, (const TcProb *)pl.probs.p, (const TcTile *)pl.tiles[k].p, pl.ntiles[k], pl.npad_max[k],
+                     pl.max_nk[k], tcerr_.as<int>(), st_);
+      ++launches_;
     }
   }
   void run_split(const SplitPlan &pl, cudaStream_t s = nullptr) {
@@ -2018,7 +2009,6 @@ class Engine final : public IEngine {
         p.overwrite = overwrite;
         for (int mt = 0; mt < (M + 127) / 128; ++mt) l.tiles.push_back(TcTile{(int)l.probs.size(), mt});
         l.probs.push_back(p);
-        l.phase.push_back(0);
       }
     };
     if (kNComp == 1) {
