@@ -275,7 +275,9 @@ class Engine final : public IEngine {
   }
   // blocks in device-addressable host memory, packed in place on the compute stream: one
   // launch for all of them (a channel given twice starts a new one, so that the last block
-  // given stays the one that counts)
+  // given stays the one that counts).  The blocks before an invalid channel count, as one by
+  // one, and each block raises the version before it is packed: a call that ends in an error
+  // leaves no copy of V taken for the present one.
   void set_vblocks_direct(int kind, int n, const int *chs, double *const *src) {
     const Layout &L = *L_;
     S *dst = kind == 3 ? Vhp_.as<S>() : kind == 6 ? Vpp_.as<S>() : Vhh_.as<S>();
@@ -293,11 +295,16 @@ class Engine final : public IEngine {
       std::fill(seen.begin(), seen.end(), 0);
       units = 0;
     };
+    const int nch = L.fam[kind == 1 ? 1 : 3].count();
     for (int i = 0; i < n; ++i) {
       const int ch = chs[i];
-      check_ch(ch, L.fam[kind == 1 ? 1 : 3].count());
+      if (ch < 0 || ch >= nch) flush();
+      check_ch(ch, nch);
       const int target = kind == 1 ? hhhh_to_hhpp_[ch] : ch;
       if (target < 0) continue;  // an hhhh channel without an hhpp partner is not used by CCD
+      dirty_ = true;
+      user_set_ |= 1u << kind;
+      ++v_version_;
       const auto &pk = L.pk[target];
       if (seen[target]) flush();
       seen[target] = 1;
@@ -314,9 +321,6 @@ class Engine final : public IEngine {
       jobs.push_back(j);
     }
     flush();
-    dirty_ = true;
-    user_set_ |= 1u << kind;
-    ++v_version_;
   }
   // HPHP blocks in device-addressable host memory: one batched copy launch
   void set_v4_direct(int n, const int *chs, double *const *src) {
