@@ -958,7 +958,9 @@ class Learner final : public ILearner {
   }
   void set_params(const float *p) override {
     // on the learner's own stream, as all that reads them; waited for, since the engines' streams
-    // read them too
+    // read them too.  Marked first: a failure half-way leaves no inference tiles of the old ones.
+    lck(cudaSetDevice(device_), "cudaSetDevice");
+    weights_dirty_ = true;
     lck(cudaMemcpyAsync(params_.p, p, kMlParams * 4, cudaMemcpyHostToDevice, st_), "params");
     lck(cudaMemsetAsync(m_.p, 0, kMlParams * 4, st_), "adam");
     lck(cudaMemsetAsync(v_.p, 0, kMlParams * 4, st_), "adam");
@@ -967,7 +969,6 @@ class Learner final : public ILearner {
     lck(cudaStreamSynchronize(st_), "params");
     folded_ = true;  // parameters from get_params: output layer in the targets' units
     t_ = 0;
-    weights_dirty_ = true;
   }
 
   void loss_grad(const float *X, const float *y, int n, double *loss, float *grad) override {
