@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <string>
 #include <vector>
@@ -973,6 +974,7 @@ class Learner final : public ILearner {
 
   void loss_grad(const float *X, const float *y, int n, double *loss, float *grad) override {
     lck(cudaSetDevice(device_), "cudaSetDevice");
+    std::lock_guard<std::mutex> hold(io_mutex_);
     if (n < 1) throw EngineError(1, "learner: empty batch");
     ensure_batch(n);
     ensure_io(n);
@@ -988,6 +990,7 @@ class Learner final : public ILearner {
 
   void infer(const float *X, int n, float *out, int tensor_cores) override {
     lck(cudaSetDevice(device_), "cudaSetDevice");
+    std::lock_guard<std::mutex> hold(io_mutex_);
     if (n < 1) return;
     ensure_io(n);
     lck(cudaMemcpyAsync(ioX_.p, X, (size_t)n * kMlIn * 4, cudaMemcpyHostToDevice, st_), "copy");
@@ -1134,6 +1137,7 @@ class Learner final : public ILearner {
   LBuf H1_, H2_, D1_, D2_, D3_, bpart_, wpart_, lpart_, ioX_, ioy_;
   char *host_grad_ = nullptr;  // page-locked: gradient and loss of loss_grad
   int cap_ = 0, io_cap_ = 0;
+  std::mutex io_mutex_;  // loss_grad and infer share ioX_, ioy_ and host_grad_: one call at a time
   int64_t t_ = 0;
   bool weights_dirty_ = true;
   std::vector<Chunk> data_;
