@@ -284,11 +284,12 @@ __constant__ const unsigned char kIso[20] = {0x00, 0x09, 0x0a, 0x0c, 0x11, 0x12,
 template <typename S, typename W, int G>
 __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>::kMinBlocks)
     k_triples(TriplesDev D, const W *__restrict__ T, const W *__restrict__ V5, const W *__restrict__ V2,
-              const S *__restrict__ fd, int seg, int nseg, double *partial) {
+              const S *__restrict__ fd, int seg, int nseg, int stride, double *partial) {
   using Sh = TripleShape<W, G>;
   using Sum = TripleSum<S, W>;
   using Fock = typename Sum::Fock;
   constexpr int NT = Sh::kThreads, KB = Sh::kKets, CU = Sh::kCube, CAP = 2 * NT;
+  constexpr bool kSort = std::is_same<S, W>::value, kOne = kSort && G == 4;
   extern __shared__ __align__(32) unsigned char tsm[];
   SpinPair<W> *tab = reinterpret_cast<SpinPair<W> *>(tsm);  // [buffer][ket][table U, Q, X, Y][term][states]
   __shared__ Fock eh[CU], ep[3][KB][CU];
@@ -307,10 +308,13 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
   // this thread's ket of a step and its states of it: bit s of spin (and 2 t of isospin)
   struct Item {
     int kb, iso, sa, sb, si, sj;
+    bool bc;     // a state of c in order behind b's
+    int cs, ks;  // the one spin of c and k of a single pair
   };
   Item mine[Sh::kRounds];
   auto state = [](int iso, int pos, int s) { return G == 4 ? ((iso >> (5 - pos)) & 1) * 2 + s : s; };
   int last_bra = -1, nket = 0;
+  bool one = false;
   int3 hm = make_int3(0, 0, 0);
   unsigned qn = 0;
   // closing momenta of the kets of step st
@@ -422,17 +426,21 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
     }
   };
   // the pairs of the kets of step st
-  auto pairs = [&](const Item &I, int st, int m, const SpinPair<W> *from) {
+  auto pairs = [&](const Item &I, int st, int m, const SpinPair<W> *from, auto single) {
+    constexpr int NS = decltype(single)::value ? 1 : 2;  // spins of c and of k
     const int kb = I.kb, sa = I.sa, sb = I.sb, si = I.si, sj = I.sj;
     if (kb >= KB || st * KB + kb >= nket) return;
     const SpinPair<W> *tb = from + (size_t)kb * 36 * CU;
     const int2 kt = kets[st * KB + kb];
     const int pa = kt.x & 0xffff, pb = (int)((unsigned)kt.x >> 16), pc = kt.y;
-    W w[2][2];
+    // each triple once: states in order where momenta coincide, and all of them present
+    const int(*o)[4] = op[m][kb];
+    if ((pa == pb && sa >= sb) || (kSort && pb == pc && !I.bc) || (o[0][sa] | o[1][sb]) < 0) return;
+    W w[NS][NS];
 #pragma unroll
-    for (int cs = 0; cs < 2; ++cs)
+    for (int cs = 0; cs < NS; ++cs)
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) w[cs][ks] = wzero<W>();
+      for (int ks = 0; ks < NS; ++ks) w[cs][ks] = wzero<W>();
     auto cube = [](int p, int q, int r) { return (p * G + q) * G + r; };
 #pragma unroll
     for (int half = 0; half < 2; ++half)  // the terms in pert_triples2's order
@@ -442,10 +450,10 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
         if (close[st & 3][kb][9 * half + 3 * pp + hp] < 0) continue;
         const SpinPair<W> *first = tb + (18 * half + 3 * pp + hp) * CU, *second = first + 9 * CU;
 #pragma unroll
-        for (int cs = 0; cs < 2; ++cs)
+        for (int cs = 0; cs < NS; ++cs)
 #pragma unroll
-          for (int ks = 0; ks < 2; ++ks) {
-            const int sc = state(I.iso, 2, cs), sk = state(I.iso, 5, ks);
+          for (int ks = 0; ks < NS; ++ks) {
+            const int sc = state(I.iso, 2, NS == 1 ? I.cs : cs), sk = state(I.iso, 5, NS == 1 ? I.ks : ks);
             int f, g;
             if (half == 0) {
               f = cube(pp == 0 ? sa : pp == 1 ? sb : sc, hp == 1 ? sk : si, hp == 2 ? sk : sj);
@@ -459,19 +467,20 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
             w[cs][ks] = madd_conj(y.v[1], x.v[1], w[cs][ks]);
           }
       }
-    // each triple once: states in order where momenta coincide, and all of them present
-    const int(*o)[4] = op[m][kb];
-    const bool there = (pa != pb || sa < sb) && (o[0][sa] | o[1][sb]) >= 0;
     W wv[4];
     Fock hv[4], pv[4];
     bool on[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int sc = state(I.iso, 2, q >> 1), sk = state(I.iso, 5, q & 1);
-      wv[q] = w[q >> 1][q & 1];
+      on[q] = q < NS * NS;
+      wv[q] = wzero<W>();
+      hv[q] = pv[q] = Fock{};
+      if (!on[q]) continue;
+      const int sc = state(I.iso, 2, NS == 1 ? I.cs : q >> 1), sk = state(I.iso, 5, NS == 1 ? I.ks : q & 1);
+      wv[q] = w[NS == 1 ? 0 : q >> 1][NS == 1 ? 0 : q & 1];
       hv[q] = eh[cube(si, sj, sk)];
       pv[q] = ep[m][kb][cube(sa, sb, sc)];
-      on[q] = there && (o[2][sc] | oh[2][sk]) >= 0 && (pb != pc || sb < sc) && (hm.y != hm.z || sj < sk);
+      on[q] = (o[2][sc] | oh[2][sk]) >= 0 && (pb != pc || sb < sc) && (hm.y != hm.z || sj < sk);
     }
     sum.add(wv, hv, pv, on);
   };
@@ -494,42 +503,56 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
         const int i = oh[0][x / (G * G)], j = oh[1][x / G % G], k = oh[2][x % G];
         eh[x] = Sum::fock(i >= 0 && j >= 0 && k >= 0 ? fd[i] + fd[j] + fd[k] : S(0.0));
       }
-      // The states (a, b, i, j) of this block whose i and j exist and come in order, spread
-      // over the threads without gaps: where i and j share a momentum they are 6 of 16.
+      // The states (a, b, i, j) of this block whose i and j exist and come in order, with a k behind
+      // them, spread over the threads without gaps.  FP64 contractions, which are bound by their pipe,
+      // take those first that kets of coinciding momenta need (a < b, and a c behind b), so that
+      // whole warps have nothing to do there; and single pairs where all of i, j, k share a momentum
+      // (96 pairs, in 36 of the 320 states).  FP32 ones keep neighbouring states in neighbouring
+      // lanes, which the shared-memory reads want.
+      one = kOne && hm.x == hm.z;
       if (wid == 0) {
         int n = 0;
-        for (int x0 = 0; x0 < Sh::kItems; x0 += 32) {
-          const int x = x0 + lane;
-          bool ok = false;
-          if (x < Sh::kItems) {
-            const int iso = G == 4 ? kIso[x >> 4] : 0;
-            const int i = state(iso, 3, (x >> 1) & 1), j = state(iso, 4, x & 1);
-            ok = (oh[0][i] | oh[1][j]) >= 0 && (hm.x != hm.y || i < j);
+        for (int y = 0; y < (kSort ? 4 : 1) * (one ? 4 : 1); ++y)
+          for (int x0 = 0; x0 < Sh::kItems; x0 += 32) {
+            const int x = x0 + lane, order = one ? y >> 2 : y, cs = one ? y >> 1 & 1 : 1;
+            bool ok = false;
+            if (x < Sh::kItems) {
+              const int iso = G == 4 ? kIso[x >> 4] : 0;
+              const int a = state(iso, 0, (x >> 3) & 1), b = state(iso, 1, (x >> 2) & 1);
+              const int i = state(iso, 3, (x >> 1) & 1), j = state(iso, 4, x & 1);
+              bool k = false;
+              for (int s = one ? y & 1 : 0; s < (one ? (y & 1) + 1 : 2); ++s)
+                k |= oh[2][state(iso, 5, s)] >= 0 && (hm.y != hm.z || j < state(iso, 5, s));
+              ok = (oh[0][i] | oh[1][j]) >= 0 && (hm.x != hm.y || i < j) && k &&
+                   (!kSort || (a < b ? 0 : 2) + (b < state(iso, 2, cs) ? 0 : 1) == order);
+            }
+            const unsigned vote = __ballot_sync(0xffffffffu, ok);
+            if (ok) items[n + __popc(vote & ((1u << lane) - 1u))] = (unsigned short)(x | (y & 3) << 9);
+            n += __popc(vote);
           }
-          const unsigned vote = __ballot_sync(0xffffffffu, ok);
-          if (ok) items[n + __popc(vote & ((1u << lane) - 1u))] = (unsigned short)x;
-          n += __popc(vote);
-        }
         if (lane == 0) nkets_warp[NT / 32] = n;
       }
       __syncthreads();
       const int nitem = nkets_warp[NT / 32];
 #pragma unroll
       for (int r = 0; r < Sh::kRounds; ++r) {
-        const int y = tid + r * NT, x = nitem > 0 ? items[y % nitem] : 0, iso = G == 4 ? kIso[x >> 4] : 0;
+        const int y = tid + r * NT, z = nitem > 0 ? items[y % nitem] : 0, x = z & 511, iso = G == 4 ? kIso[x >> 4] : 0;
         mine[r] = Item{nitem > 0 ? y / nitem : KB, iso, state(iso, 0, (x >> 3) & 1), state(iso, 1, (x >> 2) & 1),
-                       state(iso, 3, (x >> 1) & 1), state(iso, 4, x & 1)};
+                       state(iso, 3, (x >> 1) & 1), state(iso, 4, x & 1), false, z >> 10 & 1, z >> 9 & 1};
+        mine[r].bc = mine[r].sb < state(iso, 2, one ? mine[r].cs : 1);
       }
     }
-    int t0 = sg * seg;
-    const int t1 = min(tests, t0 + seg);
+    // test x of the segment: (p1, p2) number first + x * stride
+    const int first = stride == 1 ? sg * seg : sg;
+    const int t1 = min(seg, (tests - first + stride - 1) / stride);
+    int t0 = 0;
     while (t0 < t1) {
       // the ket momenta p1 <= p2 <= p3 of this total, in the order of (p1, p2)
       nket = 0;
       for (; t0 < t1 && nket + NT <= CAP; t0 += NT) {
-        const int t = t0 + tid, p1 = t / D.npm, p2 = t - p1 * D.npm;
+        const int x = t0 + tid, t = x < t1 ? first + x * stride : 0, p1 = t / D.npm, p2 = t - p1 * D.npm;
         int p3 = -1;
-        if (t < t1 && p2 >= p1)
+        if (x < t1 && p2 >= p1)
           p3 = t_momentum(D, __vsub4(__vadd4(__vsub4(qn, D.pmom[p1]), 2 * kQBias * 0x010101u), D.pmom[p2])).y;
         const bool live = p3 >= 0 && p3 >= p2;
         const unsigned vote = __ballot_sync(0xffffffffu, live);
@@ -540,7 +563,11 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
           if (w < wid) before += nkets_warp[w];
           all += nkets_warp[w];
         }
-        if (live) kets[before + __popc(vote & ((1u << lane) - 1u))] = make_int2(p1 | p2 << 16, p3);
+        // (FP64: two that coincide first, as in the order of the bras)
+        const bool turn = kSort && p2 == p3;
+        if (live)
+          kets[before + __popc(vote & ((1u << lane) - 1u))] =
+              turn ? make_int2(p2 | p3 << 16, p1) : make_int2(p1 | p2 << 16, p3);
         nket += all;
         __syncthreads();
       }
@@ -558,9 +585,14 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
         if (st + 3 < steps) closing(st + 3);
         if (st + 2 < steps) meta(st + 2, (st + 2) % 3);
         if (Sh::kBuffers == 2 && st + 1 < steps) build(st + 1, (st + 1) % 3, tab + (size_t)((st + 1) & 1) * KB * 36 * CU);
+        const SpinPair<W> *from = tab + (Sh::kBuffers == 2 ? (size_t)(st & 1) * KB * 36 * CU : 0);
+        if (kOne && one) {
 #pragma unroll
-        for (int r = 0; r < Sh::kRounds; ++r)
-          pairs(mine[r], st, st % 3, tab + (Sh::kBuffers == 2 ? (size_t)(st & 1) * KB * 36 * CU : 0));
+          for (int r = 0; r < Sh::kRounds; ++r) pairs(mine[r], st, st % 3, from, std::true_type{});
+        } else {
+#pragma unroll
+          for (int r = 0; r < Sh::kRounds; ++r) pairs(mine[r], st, st % 3, from, std::false_type{});
+        }
         if ((st & (kFlush - 1)) == kFlush - 1) sum.flush();
         __syncthreads();
         if (Sh::kBuffers == 1 && st + 1 < steps) {
@@ -818,20 +850,34 @@ class Triples final : public ITriples<S> {
     using Sh = TripleShape<W, G>;
     const auto kernel = k_triples<S, W, G>;
     TD_.bra = std::is_same<S, W>::value ? bra64_.as<int3>() : bra_.as<int3>();
-    tck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::table_bytes()), "(T) attribute");
-    int per_sm = 0, sms = 0, dev = 0;
-    tck(cudaGetDevice(&dev), "(T) device");
-    tck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "(T) attribute");
-    tck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, Sh::kThreads, Sh::table_bytes()), "(T) occupancy");
+    int64_t &want = want_[std::is_same<S, W>::value];  // blocks that the device holds at once
+    if (!want) {
+      tck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Sh::table_bytes()), "(T) attribute");
+      int per_sm = 0, sms = 0, dev = 0;
+      tck(cudaGetDevice(&dev), "(T) device");
+      tck(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "(T) attribute");
+      tck(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, Sh::kThreads, Sh::table_bytes()), "(T) occupancy");
+      want = std::min<int64_t>(kMaxBlocks, std::max(1, per_sm * sms));
+    }
     // Items of work: a block of hole triples and a segment of its (p1, p2) tests, some 64 a thread
-    // block where the lattice has enough for a few steps of kets in each.  Thread blocks take them in strides, segment by
-    // segment: the first segments hold most of the kets, so each block must get some of all.
-    const int64_t tests = (int64_t)TD_.npm * TD_.npm, want = (int64_t)std::max(1, per_sm * sms);
-    const int64_t seg64 = std::max<int64_t>(48 * Sh::kKets, (int64_t)TD_.nbra * tests / (64 * want));
-    const int seg = (int)std::min<int64_t>(tests, (seg64 + Sh::kThreads - 1) / Sh::kThreads * Sh::kThreads);
-    const int nseg = (int)((tests + seg - 1) / seg);
-    const int blocks = (int)std::min<int64_t>((int64_t)TD_.nbra * nseg, std::min<int64_t>(kMaxBlocks, want));
-    kernel<<<blocks, Sh::kThreads, Sh::table_bytes(), st>>>(TD_, T, V5, V2, fdiag, seg, nseg, partial_.as<double>());
+    // block where the lattice has enough for a few steps of kets in each.  Thread blocks take them in
+    // strides, segment by segment: the first segments hold most of the kets, so each block must get
+    // some of all.  A lattice with fewer than two such items a block (a step of kets takes some 5 us,
+    // and an item three to get going) gives every block one, every nseg-th test of its triples: SNM 4
+    // nmax=2 1280 to 139 us with FP64 contractions and 563 to 78 with FP32, SNM 28 nmax=1 503 to 327
+    // and 118 to 79, with the states and their order above.
+    const int64_t tests = (int64_t)TD_.npm * TD_.npm;
+    int64_t seg = std::max<int64_t>(48 * Sh::kKets, (int64_t)TD_.nbra * tests / (64 * want));
+    seg = std::min(tests, (seg + Sh::kThreads - 1) / Sh::kThreads * Sh::kThreads);
+    int64_t nseg = (tests + seg - 1) / seg, stride = 1;
+    if (nseg * TD_.nbra < 2 * want) {
+      nseg = std::min(tests, std::max<int64_t>(1, want / TD_.nbra));
+      seg = (tests + nseg - 1) / nseg;
+      stride = nseg;
+    }
+    const int blocks = (int)std::min<int64_t>((int64_t)TD_.nbra * nseg, want);
+    kernel<<<blocks, Sh::kThreads, Sh::table_bytes(), st>>>(TD_, T, V5, V2, fdiag, (int)seg, (int)nseg, (int)stride,
+                                                            partial_.as<double>());
     return blocks;
   }
 
@@ -893,6 +939,15 @@ class Triples final : public ITriples<S> {
           bra.push_back(make_int3(a, b, c));
           bra64.push_back(b == c && a != b ? make_int3(b, c, a) : make_int3(a, b, c));
         }
+    // The longest first (distinct momenta, two that coincide, three), but for FP64 contractions only
+    // where thread blocks get one item each: SNM 28 nmax=1 361 to 327 us, nmax=2 9.8 to 10.3 ms (FP32
+    // 1.50 to 1.45).
+    auto spread = [](const int3 &b) { return (b.x != b.y) + (b.y != b.z) + (b.x != b.z); };
+    auto longest = [&](std::vector<int3> &v) {
+      std::stable_sort(v.begin(), v.end(), [&](const int3 &x, const int3 &y) { return spread(x) > spread(y); });
+    };
+    longest(bra);
+    if ((int64_t)bra.size() * TD_.npm * TD_.npm < 1 << 18) longest(bra64);
     TD_.nbra = (int)bra.size();
     hmom_.put(q[0]); pmom_.put(q[1]); mom_of_.put(mom); bra_.put(bra); bra64_.put(bra64);
     horb_.put(orb[0]); porb_.put(orb[1]);
@@ -913,6 +968,7 @@ class Triples final : public ITriples<S> {
   std::vector<int64_t> off5_h_, off2_h_;
   std::vector<int> nr5_h_, nc5_h_, nr2_h_, nc2_h_;
   int64_t n_v5_ = 0, n_v2_ = 0, launches_ = 0;
+  int64_t want_[2] = {0, 0};  // thread blocks of a launch with FP32 and FP64 contractions
   bool have5_ = false, have2_ = false;
 };
 
