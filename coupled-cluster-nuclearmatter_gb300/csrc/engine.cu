@@ -507,6 +507,7 @@ class Engine final : public IEngine {
     dirty_ = true;
     ++v_version_;
     vph_ready_ = false;
+    if (tr_ && tr_->generated()) tr_->generate_v(pot_, st_);  // (T) reads the new interaction as well
     commit();
   }
   // The first caller HPHP block on a generated engine: W is rebuilt from the stored

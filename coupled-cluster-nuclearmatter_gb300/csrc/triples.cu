@@ -771,6 +771,7 @@ class Triples final : public ITriples<S> {
   }
 
   bool has_v() const override { return have5_ && have2_; }
+  bool generated() const override { return generated_; }
   int64_t launches() const override { return launches_; }
 
   void set_hhhp(int ch, const double *v, cudaStream_t st) override {
@@ -799,7 +800,7 @@ class Triples final : public ITriples<S> {
     else gen(k_gen_block<S, false>);
     launches_ += 2;
     tck(cudaGetLastError(), "V_hppp/V_hhhp generation");
-    have5_ = have2_ = true;
+    have5_ = have2_ = generated_ = true;
     low_ready_ = false;
   }
   void energy(const S *T, int64_t n_t, const S *fdiag, double et[2], cudaStream_t st, bool fp32) override {
@@ -969,7 +970,7 @@ class Triples final : public ITriples<S> {
   std::vector<int> nr5_h_, nc5_h_, nr2_h_, nc2_h_;
   int64_t n_v5_ = 0, n_v2_ = 0, launches_ = 0;
   int64_t want_[2] = {0, 0};  // thread blocks of a launch with FP32 and FP64 contractions
-  bool have5_ = false, have2_ = false;
+  bool have5_ = false, have2_ = false, generated_ = false;
 };
 
 template <typename S>

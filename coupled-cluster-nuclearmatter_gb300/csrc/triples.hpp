@@ -17,6 +17,7 @@ class ITriples {
  public:
   virtual ~ITriples() = default;
   virtual bool has_v() const = 0;
+  virtual bool generated() const = 0;  // V_hppp and V_hhhp come from generate_v
   // vnn_hhhp(ch)%val (n_hh x n_hp) / vnn_hppp(ch)%val (n_hp x n_pp), ordered, complex interleaved
   virtual void set_hhhp(int ch, const double *v, cudaStream_t st) = 0;
   virtual void set_hppp(int ch, const double *v, cudaStream_t st) = 0;
