@@ -99,15 +99,15 @@ __device__ __forceinline__ cplxf madd_conj(cplxf v, cplxf t, cplxf acc) {
 __device__ __forceinline__ double wnorm2(double w) { return w * w; }
 __device__ __forceinline__ double wnorm2(cplx w) { return w.re * w.re + w.im * w.im; }
 
-// Sum of |W|^2 / D, and the denominators it needs.  With FP64 contractions all in FP64.  With
-// FP32 contractions the ratio is formed in FP32 (its rounding, 6e-8 of the term, is far below the
-// FP32 contractions' own) from a denominator that keeps FP64's accuracy to there, and the sum
-// has FP64's: both as pairs of FP32 numbers, since an FP64 operation costs 64 FP32 ones on this
-// GPU and a pair needs six of them.  A pair holds at most 64 terms a round (kFlush steps) and is
-// then added to an FP64 sum: over a whole lattice it would lose the many terms below 2^-48 of it,
-// all of one sign (SNM 132 nmax=3, 3.4e10 terms: 6e-9 of the sum).
+// Sum of |W|^2 / D, in FP64 term by term, and the denominators it needs.  With FP64 contractions the
+// ratio is FP64 as well, with FP32 ones FP32 (its rounding, 6e-8 of the term, is far below the
+// contractions' own), from FP64 denominators in real engines.  Complex ones, with two FP64
+// differences a pair beside the two additions of the sum, take the denominators' differences from
+// pairs of FP32 numbers, which hold the Fock sums to 2^-49: an FP64 operation costs 64 FP32 ones on
+// this GPU (SNM 76 nmax=2 16.1 ms with FP64 differences, 11.6 so; PNM 54 nmax=2 1.97 with FP64, 2.00
+// with pairs).  The sum in pairs, added to an FP64 one every 64 terms, would save another tenth of
+// the complex time (10.4 ms), but holds 48 bits and turns an infinite term into a NaN.
 template <typename S, typename W> struct TripleSum;
-constexpr int kFlush = 16;  // a power of two; the additions cost 1.5 % of the sum's time at 16
 // n1 / d1 + n2 / d2 as one fraction: an FP64 division costs some ten operations of the FP64
 // pipe, three multiplications and an addition are cheaper
 __device__ __forceinline__ void add_fractions(double n1, double d1, double n2, double d2, double &n, double &d) {
@@ -131,7 +131,6 @@ template <> struct TripleSum<double, double> {
     add_fractions(n2[0], d2[0], n2[1], d2[1], nn, dd);
     re += nn / dd;
   }
-  __device__ __forceinline__ void flush() {}
   __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = re; v[1] = 0.0; }
 };
 template <> struct TripleSum<cplx, cplx> {
@@ -148,44 +147,31 @@ template <> struct TripleSum<cplx, cplx> {
         s.im = fma(-r, d.im, s.im);
       }
   }
-  __device__ __forceinline__ void flush() {}
   __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = s.re; v[1] = s.im; }
 };
 __device__ __forceinline__ float2 two_floats(double x) {
   const float h = __double2float_rn(x);
   return make_float2(h, __double2float_rn(x - (double)h));
 }
-// a + b of pairs of floats where b's low part is dropped into the sum's (Knuth's two-sum)
-__device__ __forceinline__ void two_add(float &hi, float &lo, float x) {
-  const float s = __fadd_rn(hi, x), bb = __fsub_rn(s, hi);
-  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bb)), __fsub_rn(x, bb)));
-  hi = s;
-}
-// (h - p) of two pairs, to FP32
+// (h - p) of two pairs, to FP32: Knuth's two-sum of the high parts, and what it leaves
 __device__ __forceinline__ float two_sub(float2 h, float2 p) {
-  float hi = h.x, lo = 0.0f;
-  two_add(hi, lo, -p.x);
-  return __fadd_rn(hi, __fadd_rn(lo, __fsub_rn(h.y, p.y)));
+  const float s = __fsub_rn(h.x, p.x), bb = __fsub_rn(s, h.x);
+  const float rest = __fsub_rn(__fsub_rn(h.x, __fsub_rn(s, bb)), __fadd_rn(p.x, bb));
+  return __fadd_rn(s, __fadd_rn(rest, __fsub_rn(h.y, p.y)));
 }
 template <> struct TripleSum<double, float> {
-  using Fock = float2;
-  float hi = 0.0f, lo = 0.0f;
+  using Fock = double;
   double re = 0.0;
-  static __device__ __forceinline__ Fock fock(double f) { return two_floats(f); }
+  static __device__ __forceinline__ Fock fock(double f) { return f; }
   __device__ __forceinline__ void add(const float (&w)[4], const Fock (&h)[4], const Fock (&p)[4], const bool (&live)[4]) {
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-      if (live[q]) two_add(hi, lo, (w[q] * w[q]) / two_sub(h[q], p[q]));
-  }
-  __device__ __forceinline__ void flush() {
-    re += (double)hi + (double)lo;
-    hi = lo = 0.0f;
+      if (live[q]) re += (double)((w[q] * w[q]) / (float)(h[q] - p[q]));
   }
   __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = re; v[1] = 0.0; }
 };
 template <> struct TripleSum<cplx, cplxf> {
   using Fock = float4;
-  float hr = 0.0f, lr = 0.0f, hi = 0.0f, li = 0.0f;
   double re = 0.0, im = 0.0;
   static __device__ __forceinline__ Fock fock(cplx f) {
     const float2 a = two_floats(f.re), b = two_floats(f.im);
@@ -201,14 +187,9 @@ template <> struct TripleSum<cplx, cplxf> {
         const float dr = two_sub(make_float2(h[q].x, h[q].y), make_float2(p[q].x, p[q].y));
         const float di = two_sub(make_float2(h[q].z, h[q].w), make_float2(p[q].z, p[q].w));
         const float s = n / (dr * dr + di * di);  // |W|^2 / D = |W|^2 conj(D) / |D|^2
-        two_add(hr, lr, s * dr);
-        two_add(hi, li, -s * di);
+        re += (double)(s * dr);
+        im += (double)(-s * di);
       }
-  }
-  __device__ __forceinline__ void flush() {
-    re += (double)hr + (double)lr;
-    im += (double)hi + (double)li;
-    hr = lr = hi = li = 0.0f;
   }
   __device__ __forceinline__ void total(double (&v)[2]) const { v[0] = re; v[1] = im; }
 };
@@ -593,14 +574,12 @@ __global__ void __launch_bounds__(TripleShape<W, G>::kThreads, TripleShape<W, G>
 #pragma unroll
           for (int r = 0; r < Sh::kRounds; ++r) pairs(mine[r], st, st % 3, from, std::false_type{});
         }
-        if ((st & (kFlush - 1)) == kFlush - 1) sum.flush();
         __syncthreads();
         if (Sh::kBuffers == 1 && st + 1 < steps) {
           build(st + 1, (st + 1) % 3, tab);
           __syncthreads();
         }
       }
-      sum.flush();
     }
   }
   double acc[2];
