@@ -145,6 +145,7 @@ def lib():
         "ccx_engine_stream": ([vp, C.POINTER(vp)], C.c_int),
         "ccx_device_fp64_peak": ([i32, C.POINTER(dbl)], C.c_int),
         "ccx_selftest_tc_gemm": ([i32, i32, i32, vp, vp, vp, i32, C.c_uint64, C.POINTER(dbl), C.POINTER(dbl)], C.c_int),
+        "ccx_selftest_tc_product": ([i32, i32, i32, i32, i32, i32, vp, vp, vp], C.c_int),
         "ccx_ccd_energy_noalloc": ([i32, vp, vp, vp, vp, vp], C.c_int),
         "ccx_selftest_tc_wait": ([i32, C.c_int64, C.POINTER(i32)], C.c_int),
         "ccx_engine_prepare": ([vp, C.POINTER(_IterOpts)], C.c_int),
@@ -214,6 +215,16 @@ def selftest_tc_gemm(shapes, kind: int = 0, use_alo: bool = True, seed: int = 1,
     _check(lib().ccx_selftest_tc_gemm(device, kind, len(shapes), _ptr(M), _ptr(N), _ptr(K), int(use_alo) | (2 if segments else 0), seed,
                                       C.byref(err), C.byref(ms)))
     return err.value, ms.value
+
+
+def selftest_tc_product(A, B, kind: int = 0, use_alo: bool = True, segments: bool = False, device: int = 0) -> np.ndarray:
+    """1/2 A B by the tensor-core kernels of selftest_tc_gemm, on the caller's operands."""
+    a = np.ascontiguousarray(A, np.float64)
+    b = np.asfortranarray(B, np.float64)
+    c = np.zeros((a.shape[0], b.shape[1]), order="F")
+    _check(lib().ccx_selftest_tc_product(device, kind, a.shape[0], b.shape[1], a.shape[1],
+                                         int(use_alo) | (2 if segments else 0), _ptr(a), _ptr(b), _ptr(c)))
+    return c
 
 
 class HostBuffer:

@@ -607,6 +607,15 @@ int ccx_selftest_tc_gemm(int32_t device, int32_t kind, int32_t nprob, const int3
     return fail(CCX_EINVAL, "bad selftest arguments");
   return guard([&] { ccx::tc_selftest(device, kind, nprob, M, N, K, use_alo, seed, max_rel_err, ms); });
 }
+int ccx_selftest_tc_product(int32_t device, int32_t kind, int32_t M, int32_t N, int32_t K, int32_t use_alo, const double *A,
+                            const double *B, double *C) {
+  if (!A || !B || !C || kind < 0 || kind > 2) return fail(CCX_EINVAL, "bad selftest arguments");
+  return guard([&] {
+    const ccx::TcGiven given{A, B, C};
+    double rel = 0.0, ms = 0.0;
+    ccx::tc_selftest(device, kind, 1, &M, &N, &K, use_alo, 1, &rel, &ms, 0, nullptr, &given);
+  });
+}
 int ccx_host_alloc(int64_t bytes, void **ptr) {
   if (!ptr || bytes <= 0) return fail(CCX_EINVAL, "bad host allocation arguments");
   *ptr = nullptr;

@@ -136,9 +136,13 @@ void draw_lecs(uint64_t seed, double out[9]);
 double fp64_peak(int device);
 // message returned by ccx_last_error() on the calling thread
 void set_last_error(const std::string &msg);
-// tensor-core split GEMM self-test (tc_selftest.cu)
+// tensor-core split GEMM self-test (tc_selftest.cu), on random operands or on the caller's
+struct TcGiven {
+  const double *A, *B;  // M x K row-major, K x N column-major
+  double *C;            // out: 1/2 A B, M x N column-major
+};
 void tc_selftest(int device, int kind, int nprob, const int *Ms, const int *Ns, const int *Ks, int use_alo, uint64_t seed,
                  double *max_rel, double *ms,
-                 long long wait_budget = 0, int *kernel_err = nullptr);
+                 long long wait_budget = 0, int *kernel_err = nullptr, const TcGiven *given = nullptr);
 
 }  // namespace ccx

@@ -26,10 +26,17 @@ struct Dev {
   explicit Dev(size_t b) : bytes(std::max<size_t>(b, 16)) { sck(cudaMalloc(&p, bytes), "cudaMalloc"); }
   ~Dev() { cudaFree(p); }
 };
+// the caller's operands in the place of random ones, onto C = 0
+void take(const TcGiven &g, std::vector<double> &A, std::vector<double> &B, std::vector<double> &C) {
+  std::copy(g.A, g.A + A.size(), A.begin());
+  std::copy(g.B, g.B + B.size(), B.begin());
+  std::fill(C.begin(), C.end(), 0.0);
+}
 }  // namespace
 
 // Ozaki digit-product GEMM on the same kind of problems; reference in long double.
-static void oz_selftest(int nprob, const int *Ms, const int *Ns, const int *Ks, uint64_t seed, double *max_rel, double *ms) {
+static void oz_selftest(int nprob, const int *Ms, const int *Ns, const int *Ks, uint64_t seed, double *max_rel, double *ms,
+                        const TcGiven *given) {
   std::mt19937_64 rng(seed);
   std::uniform_real_distribution<double> U(-1.0, 1.0);
   struct Host {
@@ -51,6 +58,7 @@ static void oz_selftest(int nprob, const int *Ms, const int *Ns, const int *Ks, 
     for (double &v : x.A) v = U(rng) * std::pow(10.0, -3.0 * std::fabs(U(rng)));
     for (double &v : x.B) v = U(rng) * std::pow(10.0, -3.0 * std::fabs(U(rng)));
     for (double &v : x.C) v = U(rng);
+    if (given) take(*given, x.A, x.B, x.C);
     fa += x.A.size(); fb += x.B.size(); fc += x.C.size();
     pa += (size_t)x.mpad * x.nk * 64;
     pb += (size_t)x.npad * x.nk * 64;
@@ -125,6 +133,10 @@ static void oz_selftest(int nprob, const int *Ms, const int *Ns, const int *Ks, 
   for (auto &x : h) {
     std::vector<double> c(x.C.size());
     sck(cudaMemcpy(c.data(), (double *)dC.p + oc, c.size() * 8, cudaMemcpyDeviceToHost), "copy C back");
+    if (given) {
+      std::copy(c.begin(), c.end(), given->C);
+      return;
+    }
     long double scale = 0.0L, diff = 0.0L;
     for (int n = 0; n < x.N; ++n)
       for (int m = 0; m < x.M; ++m) {
@@ -145,12 +157,12 @@ static void oz_selftest(int nprob, const int *Ms, const int *Ns, const int *Ks, 
 // problems and the kernel time (ms).  kind 2: the Ozaki digit-product GEMM.
 // wait_budget > 0: the clock-cycle budget of the kernel's pipeline waits; kernel_err
 // non-null: the kernel's error word is returned there instead of raised, and the product
-// is checked only when it is 0.
+// is checked only when it is 0.  given: one problem on the caller's operands, returned unchecked.
 void tc_selftest(int device, int kind, int nprob, const int *Ms, const int *Ns, const int *Ks, int use_alo, uint64_t seed,
-                 double *max_rel, double *ms, long long wait_budget, int *kernel_err) {
+                 double *max_rel, double *ms, long long wait_budget, int *kernel_err, const TcGiven *given) {
   sck(cudaSetDevice(device), "cudaSetDevice");
   if (kind == 2) {
-    oz_selftest(nprob, Ms, Ns, Ks, seed, max_rel, ms);
+    oz_selftest(nprob, Ms, Ns, Ks, seed, max_rel, ms, given);
     return;
   }
   const int tk = kind == kTcBF16 ? 64 : 32;
@@ -186,13 +198,14 @@ void tc_selftest(int device, int kind, int nprob, const int *Ms, const int *Ns, 
     for (double &v : x.A) v = U(rng) * std::pow(10.0, -3.0 * std::fabs(U(rng)));
     for (double &v : x.B) v = U(rng) * std::pow(10.0, -3.0 * std::fabs(U(rng)));
     for (double &v : x.C) v = U(rng);
+    if (given) take(*given, x.A, x.B, x.C);
     x.kseg = {0};
     const int nseg = segmented ? std::min(3, x.nk) : 1;
     for (int g = 1; g < nseg; ++g) x.kseg.push_back(x.nk * g / nseg * tk);
     x.kseg.push_back(x.K);
     if (segmented) {
       x.C0.resize(x.C.size());
-      for (double &v : x.C0) v = U(rng);
+      for (double &v : x.C0) v = given ? 0.0 : U(rng);
     }
     int nk_all = 0;
     for (size_t g = 0; g + 1 < x.kseg.size(); ++g) nk_all += (x.kseg[g + 1] - x.kseg[g] + tk - 1) / tk;
@@ -304,6 +317,10 @@ void tc_selftest(int device, int kind, int nprob, const int *Ms, const int *Ns, 
   for (auto &x : h) {
     std::vector<double> c(x.C.size());
     sck(cudaMemcpy(c.data(), (double *)dC.p + oc, c.size() * 8, cudaMemcpyDeviceToHost), "copy C back");
+    if (given) {
+      std::copy(c.begin(), c.end(), given->C);
+      return;
+    }
     double scale = 0.0, diff = 0.0;
     for (int n = 0; n < x.N; ++n)
       for (int m = 0; m < x.M; ++m) {

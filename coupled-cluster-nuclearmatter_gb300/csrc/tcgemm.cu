@@ -74,10 +74,11 @@ __device__ __forceinline__ double pair_widen(float hi, float lo, int ash, bool &
   const unsigned long long x = down ? w - t : w + t;
   return __longlong_as_double((long long)(x | ((unsigned long long)(u & 0x80000000u) << 32)));
 }
-// hi + lo += x, the rounding of the addition kept in lo (Knuth's two-sum)
-__device__ __forceinline__ void pair_add(float &hi, float &lo, float x) {
-  const float s = __fadd_rn(hi, x), t = __fsub_rn(s, hi);
-  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(x, t)));
+// hi + lo += x c, the rounding of the addition kept in lo (Knuth's two-sum); c: a power of two, which
+// costs nothing in the multiply-adds
+__device__ __forceinline__ void pair_add(float &hi, float &lo, float x, float c) {
+  const float s = __fmaf_rn(x, c, hi), t = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fmaf_rn(x, c, -t)));
   hi = s;
 }
 
@@ -336,6 +337,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
         // integers 0.77 and 0.81 in eight warps of 16 columns at a time, now 0.73 and 0.76;
         // PNM 66 nmax=4 140 and 93, 95 and 69, now 79 and 55 us.  Sixteen warps, because the
         // instructions of a warp wait for one another.
+        // Two and more are added as eighths (at most six), so that no sum of finite accumulators passes the
+        // FP32 range; what that loses is below 2^-146, some units of the accumulators' least number.
+        const int eighths = G.nacc > 1 ? 3 : 0;
         float hi[kTcCols], lo[kTcCols];
         for (int a = 0; a < G.nacc; ++a) {
           uint32_t r[kTcCols];
@@ -343,10 +347,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
           tmem_ld_wait();
           if (a == 0) {
 #pragma unroll
-            for (int j = 0; j < kTcCols; ++j) { hi[j] = __uint_as_float(r[j]); lo[j] = 0.0f; }
+            for (int j = 0; j < kTcCols; ++j) {
+              hi[j] = __uint_as_float(r[j]) * (eighths ? 0.125f : 1.0f);
+              lo[j] = 0.0f;
+            }
           } else {
 #pragma unroll
-            for (int j = 0; j < kTcCols; ++j) pair_add(hi[j], lo[j], __uint_as_float(r[j]));
+            for (int j = 0; j < kTcCols; ++j) pair_add(hi[j], lo[j], __uint_as_float(r[j]), 0.125f);
           }
         }
         if (c0 + 2 * kTcCols >= G.npad) {
@@ -363,8 +370,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
             // the pair's own sum first; infinities stay infinities
             const float l = fabsf(hi[j]) < __int_as_float(0x7f800000) ? lo[j] : 0.0f;
             lo[j] = 0.0f;
-            pair_add(hi[j], lo[j], l);
-            x[j] = pair_widen(hi[j], lo[j], ash, odd);
+            pair_add(hi[j], lo[j], l, 1.0f);
+            x[j] = pair_widen(hi[j], lo[j], ash + eighths, odd);
           }
         } else {
 #pragma unroll
@@ -376,8 +383,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(const TcProb *__restr
         if (__any_sync(0xffffffffu, odd && live)) {  // a subnormal, an infinity or a NaN
 #pragma unroll
           for (int j = 0; j < kTcCols; ++j) {
-            x[j] = f32_bits_to_f64(__float_as_uint(hi[j]), ash);
-            if (isfinite(hi[j])) x[j] += f32_bits_to_f64(__float_as_uint(lo[j]), ash);
+            x[j] = f32_bits_to_f64(__float_as_uint(hi[j]), ash + eighths);
+            if (isfinite(hi[j])) x[j] += f32_bits_to_f64(__float_as_uint(lo[j]), ash + eighths);
           }
         }
         if (keep && c0row) {

@@ -434,6 +434,10 @@ int ccx_device_fp64_peak(int32_t device, double *tflops);
  * *max_rel_err = max |C - C_ref| / max |1/2 A B| over the problems; *ms kernel time. */
 int ccx_selftest_tc_gemm(int32_t device, int32_t kind, int32_t nprob, const int32_t *M, const int32_t *N,
                          const int32_t *K, int32_t use_alo, uint64_t seed, double *max_rel_err, double *ms);
+/* The same kernels on the caller's operands (host memory): C = 1/2 A B, A (M x K) row-major,
+ * B (K x N) and C (M x N) column-major; kind and use_alo as above. */
+int ccx_selftest_tc_product(int32_t device, int32_t kind, int32_t M, int32_t N, int32_t K, int32_t use_alo,
+                            const double *A, const double *B, double *C);
 /* kernel launches issued by this engine since creation */
 int ccx_engine_launches(const ccx_engine *e, int64_t *launches);
 /* DIIS systems found singular (or with a non-finite solution) since creation; each one
