@@ -483,14 +483,18 @@ struct BitSplit {
       const uint32_t w = (uint32_t)(u >> 32), v = (uint32_t)u, sign = w & 0x80000000u;
       const int e = (int)((w >> 20) & 0x7ffu) - 896;
       // |x| cut to the 24 bits of a float and the 29 bits below; hi from the float, whose bit 8
-      // decides the rounding; the remainder of hi is exact, and takes the lower bits rounded to 24
+      // decides the rounding.  The remainder is d + t units of the last bit, with its own sign where hi
+      // was rounded up (d then counts from the next float, t back from it), so both are positive and
+      // cutting each to 24 bits leaves what its rounding to 8 bits asks for: one rounding.
       uint32_t f = ((w << 3) & 0x7ffff8u) | (v >> 29) | ((uint32_t)e << 23);
       f = e <= 0 ? 0u : e >= 255 ? 0x7f800000u : f;  // below the float range; beyond it or not finite
-      const uint32_t h = (f + 0x8000u) & 0xffff0000u;
-      const float tail = __uint2float_rn(v & 0x1fffffffu) * 0x1p-52f, unit = __uint_as_float(f & 0x7f800000u);
-      const float rem = __fmaf_rn(tail, unit, __fsub_rn(__uint_as_float(f), __uint_as_float(h)));
+      const uint32_t h = (f + 0x8000u) & 0xffff0000u, up = (f >> 15) & 1u;
+      const uint32_t t = up ? 0x20000000u - (v & 0x1fffffffu) : v & 0x1fffffffu;
+      const float unit = __uint_as_float(f & 0x7f800000u);
+      const float d = fabsf(__fsub_rn(__uint_as_float(f + up), __uint_as_float(h)));
+      const float rem = __fmaf_rz(__uint2float_rz(t) * 0x1p-52f, unit, d);
       hi = h | sign;
-      lo = ((__float_as_uint(rem) + 0x8000u) & 0xffff0000u) ^ sign;
+      lo = ((__float_as_uint(rem) + 0x8000u) & 0xffff0000u) ^ sign ^ (up << 31);
       return;
     }
     uint32_t sign;
