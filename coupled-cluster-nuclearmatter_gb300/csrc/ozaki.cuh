@@ -9,7 +9,9 @@
 // sum_k a_i(m,k) b_j(k,n) summed over the at most seven pairs of one level l = i + j is an
 // integer below 2^24 in magnitude when K is cut into chunks of kOzChunkTiles K tiles, so the FP32
 // tensor-memory accumulator of the level holds it exactly.  Levels below kOzSlices are kept (28
-// digit products); the dropped tail is below 2^-53 of K max|A(m,.)| max|B(.,n)|.  The levels of a
+// digit products); the dropped ones (six pairs of 2^14 2^-70 at level 7, a 256th of that at each
+// further one) and the rounding of the operands are below 2^-53 of K 2^(eA + eB), that is below 2^-51
+// of K max|A(m,.)| max|B(.,n)|, a maximum being at least half of its power of two.  The levels of a
 // chunk are added into two 64-bit integers, converted to FP64 once per tile.
 //
 // Digits of 8 bits and a sign, 28 products of which one MMA per K step covers a digit of A, do
