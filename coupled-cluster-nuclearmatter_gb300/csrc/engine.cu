@@ -286,10 +286,14 @@ class Engine final : public IEngine {
     int units = 0;
     auto flush = [&] {
       if (!units) return;
-      copyjobs_.alloc(jobs.size() * sizeof(PackJob), &bytes_);
-      CK(cudaMemcpyAsync(copyjobs_.p, jobs.data(), jobs.size() * sizeof(PackJob), cudaMemcpyHostToDevice, st_));
-      launch_pack_jobs<S>(D_, kind, (const PackJob *)copyjobs_.p, (int)jobs.size(), units, dst, flag_.as<int>(), st_);
-      CK(cudaStreamSynchronize(st_));  // the job table on the host is reused or goes out of scope
+      PackJob *list = nullptr;
+      if (jobs.size() > 1) {
+        copyjobs_.alloc(jobs.size() * sizeof(PackJob), &bytes_);
+        list = (PackJob *)copyjobs_.p;
+        CK(cudaMemcpyAsync(list, jobs.data(), jobs.size() * sizeof(PackJob), cudaMemcpyHostToDevice, st_));
+      }
+      launch_pack_jobs<S>(D_, kind, list, jobs[0], (int)jobs.size(), units, dst, flag_.as<int>(), st_);
+      if (list) CK(cudaStreamSynchronize(st_));  // the job table on the host is reused or goes out of scope
       ++launches_;
       jobs.clear();
       std::fill(seen.begin(), seen.end(), 0);

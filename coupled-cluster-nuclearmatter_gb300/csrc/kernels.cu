@@ -1023,10 +1023,10 @@ __device__ __forceinline__ int job_of(const PackJob *__restrict__ jobs, int njob
 // 32 x 32 tile is read down its columns (consecutive source rows, so each host cache line is
 // fetched once) and written along its rows.
 template <typename S>
-__global__ void __launch_bounds__(256) k_pack_vblock_tr(DevLayout L, const PackJob *__restrict__ jobs, int njobs,
+__global__ void __launch_bounds__(256) k_pack_vblock_tr(DevLayout L, const PackJob *__restrict__ jobs, PackJob one, int njobs,
                                                         S *__restrict__ dst, int *flag) {
   __shared__ S tile[32][33];
-  const PackJob J = jobs[job_of(jobs, njobs, blockIdx.x)];
+  const PackJob J = jobs ? jobs[job_of(jobs, njobs, blockIdx.x)] : one;
   const int ch = J.ch, R = J.rows, P = J.cols, nct = (P + 31) / 32, loc = (int)blockIdx.x - J.first;
   const int r0 = loc / nct * 32, c0 = loc % nct * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
@@ -1054,10 +1054,10 @@ __global__ void __launch_bounds__(256) k_pack_vblock_tr(DevLayout L, const PackJ
 // block (the tile kernel above) reach a fraction of the link rate on a family of tens of
 // GB.
 template <typename S>
-__global__ void __launch_bounds__(512) k_pack_vpp_cols(DevLayout L, const PackJob *__restrict__ jobs, int njobs, int ncols,
+__global__ void __launch_bounds__(512) k_pack_vpp_cols(DevLayout L, const PackJob *__restrict__ jobs, PackJob one, int njobs, int ncols,
                                                        S *__restrict__ dst, int *flag) {
   for (int u = blockIdx.x; u < ncols; u += gridDim.x) {
-    const PackJob J = jobs[job_of(jobs, njobs, u)];
+    const PackJob J = jobs ? jobs[job_of(jobs, njobs, u)] : one;
     const int P = J.cols, c = u - J.first;
     const int *map = L.pp_row + L.pp_off[J.ch];
     const int64_t base = L.vpp_off[J.ch];
@@ -1067,9 +1067,9 @@ __global__ void __launch_bounds__(512) k_pack_vpp_cols(DevLayout L, const PackJo
 }
 // Kind 1 from host memory: consecutive packed rows are consecutive source rows already
 template <typename S>
-__global__ void __launch_bounds__(256) k_pack_vhh_jobs(DevLayout L, const PackJob *__restrict__ jobs, int njobs,
+__global__ void __launch_bounds__(256) k_pack_vhh_jobs(DevLayout L, const PackJob *__restrict__ jobs, PackJob one, int njobs,
                                                        S *__restrict__ dst, int *flag) {
-  const PackJob J = jobs[job_of(jobs, njobs, blockIdx.x)];
+  const PackJob J = jobs ? jobs[job_of(jobs, njobs, blockIdx.x)] : one;
   const int H = J.rows, *map = L.hh_row + L.hh_off[J.ch];
   const int beg = ((int)blockIdx.x - J.first) * kTileElems, end = min(beg + kTileElems, H * H);
   for (int e = beg + threadIdx.x; e < end; e += blockDim.x) {
@@ -1084,12 +1084,12 @@ int pack_units(int kind, int rows, int cols) {
   return (rows * cols + kTileElems - 1) / kTileElems;
 }
 template <typename S>
-void launch_pack_jobs(const DevLayout &L, int kind, const PackJob *jobs, int njobs, int units, S *dst, int *flag,
-                      cudaStream_t st) {
+void launch_pack_jobs(const DevLayout &L, int kind, const PackJob *jobs, const PackJob &one, int njobs, int units, S *dst,
+                      int *flag, cudaStream_t st) {
   if (units <= 0) return;
-  if (kind == 6) k_pack_vpp_cols<S><<<std::min(units, 304), 512, 0, st>>>(L, jobs, njobs, units, dst, flag);
-  else if (kind == 3) k_pack_vblock_tr<S><<<units, dim3(32, 8), 0, st>>>(L, jobs, njobs, dst, flag);
-  else k_pack_vhh_jobs<S><<<units, 256, 0, st>>>(L, jobs, njobs, dst, flag);
+  if (kind == 6) k_pack_vpp_cols<S><<<std::min(units, 304), 512, 0, st>>>(L, jobs, one, njobs, units, dst, flag);
+  else if (kind == 3) k_pack_vblock_tr<S><<<units, dim3(32, 8), 0, st>>>(L, jobs, one, njobs, dst, flag);
+  else k_pack_vhh_jobs<S><<<units, 256, 0, st>>>(L, jobs, one, njobs, dst, flag);
 }
 
 // one CTA per job; 16-byte copies where both ends and the length allow
@@ -1558,7 +1558,8 @@ void launch_unpack_t(const DevLayout &L, const DevOrdered &O, int c0, int c1, in
   template void launch_diis_gram<S>(int64_t, const S *const *, int, double *, double *, cudaStream_t);                \
   template void launch_combine<S>(int64_t, const S *const *, const double *, int, S *, cudaStream_t);                 \
   template void launch_pack_vblock<S>(const DevLayout &, int, int, int, const double *, S *, int *, cudaStream_t);    \
-  template void launch_pack_jobs<S>(const DevLayout &, int, const PackJob *, int, int, S *, int *, cudaStream_t);       \
+  template void launch_pack_jobs<S>(const DevLayout &, int, const PackJob *, const PackJob &, int, int, S *, int *,      \
+                                    cudaStream_t);                                                                     \
   template void launch_build_w<S>(const DevLayout &, const int2 *, const int64_t *, const int *, const double *, S *,  \
                                   int *, cudaStream_t);                                                                \
   template void launch_build_vph<S>(const DevLayout &, const S *, S *, cudaStream_t);                                 \

@@ -123,7 +123,8 @@ void launch_pack_vblock(const DevLayout &L, int kind, int ch, int n_rows, const 
 // memory the device can address (pinned and mapped): reads follow each block's
 // column-major order (consecutive rows), through a shared-memory transpose where the packed
 // layout is row-major (kind 3).  first: units of work (pack_units) in the jobs before this
-// one; a channel occurs once in a list.
+// one; a channel occurs once in a list.  jobs null: the one job given by value (a list on the
+// device costs a copy and a wait, 5 of the 24 us of a call with one block).
 struct PackJob {
   const double *src;
   int ch, n_rows;
@@ -132,8 +133,8 @@ struct PackJob {
 };
 int pack_units(int kind, int rows, int cols);
 template <typename S>
-void launch_pack_jobs(const DevLayout &L, int kind, const PackJob *jobs, int njobs, int units, S *dst, int *flag,
-                      cudaStream_t st);
+void launch_pack_jobs(const DevLayout &L, int kind, const PackJob *jobs, const PackJob &one, int njobs, int units, S *dst,
+                      int *flag, cudaStream_t st);
 // Copies of many blocks in one launch (n doubles from src to dst per job); src may be
 // mapped host memory.
 struct CopyJob {
