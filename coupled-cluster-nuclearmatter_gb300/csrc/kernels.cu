@@ -216,9 +216,7 @@ __device__ __forceinline__ void gemm_tile(const GemmProb<S> &pr, const GemmTile 
       if (j >= tl.nj) break;
       const int64_t o = (int64_t)row * pr.sCm + (int64_t)(tl.n0 + j) * pr.sCn;
       const S v = pr.alpha == 1.0 ? acc[i] : pr.alpha * acc[i];
-      if (pr.accumulate) pr.C[o] += v;
-      else if (pr.C0) pr.C[o] = pr.C0[o] + v;
-      else pr.C[o] = v;
+      pr.C[o] = pr.C0 ? pr.C0[o] + v : v;
     }
   }
 }

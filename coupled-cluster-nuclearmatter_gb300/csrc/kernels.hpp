@@ -11,7 +11,7 @@
 namespace ccx {
 
 // ---- grouped GEMM (FP64 / complex FP64) ------------------------------------
-// C(m,n) = [C or C0 or 0] + alpha sum_s sum_k A_s(m,k) B_s(k,n), element strides per operand.
+// C(m,n) = [C0 or 0] + alpha sum_s sum_k A_s(m,k) B_s(k,n), element strides per operand.
 template <typename S>
 struct GemmSeg {
   const S *A, *B;
@@ -25,9 +25,8 @@ struct GemmProb {
   int M, N;
   double alpha;
   S *C;
-  const S *C0;  // initial value when accumulate == 0 (nullptr: zero)
+  const S *C0;  // null: zero
   int64_t sCm, sCn;
-  int accumulate;
 };
 // The work of one warp: nm row tiles from m0 on, columns n0 .. n0 + nj - 1 (nj <= kGemmCols).
 struct GemmTile {
