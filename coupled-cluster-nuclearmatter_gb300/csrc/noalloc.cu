@@ -5,8 +5,8 @@
 // manages), or code running where an allocation would be an error.  For them this
 // entry point evaluates E = 1/4 sum_ch sum_{ab,ij} T(ab,ij) V(ij,ab) directly on their
 // buffers, in the reference's layout (ccm_energy.f90:4-71).  Its scratch -- one partial sum
-// per block -- is in the file-scope array g_energy_slots below (512 KiB), held by every GPU
-// that loads the library until the process exits.
+// per block, some 5 KiB -- is the file-scope array g_energy_slots below, held by every GPU that
+// loads the library until the process exits.
 //
 // Set-up: the first call in a CUDA context (with that context's device current) looks
 // up the device address of g_energy_slots with cudaGetSymbolAddress; make that first
@@ -26,15 +26,15 @@
 
 namespace {
 
-constexpr int kMaxChannels = 16384;
+constexpr int kMaxChannels = 16384;  // of the interface; the kernel's work per channel is a scan entry
 constexpr int kMaxDevices = 64;
+constexpr int kEnergyBlocks = 304, kEnergyThreads = 256, kScan = 4 * kEnergyThreads;
 
 struct __align__(16) EnergySlot {
   double re, im;  // partial sum of a block
-  double pad[2];
 };
 
-static __device__ __align__(256) EnergySlot g_energy_slots[kMaxChannels];
+static __device__ __align__(256) EnergySlot g_energy_slots[kEnergyBlocks];
 
 // per device: the context the cached address belongs to, and the address
 struct SlotCache {
@@ -77,7 +77,6 @@ unsigned long long current_context_id() {
 // at once.  One block per channel behind a scan kernel of its own left 25 blocks with a strided
 // V for a small lattice: 58 us a call at PNM 14 nmax=2 (1 MB of each), now 10.2; PNM 66 nmax=4
 // (129 MB of each) 1212 to 75 us.
-constexpr int kEnergyBlocks = 304, kEnergyThreads = 256, kScan = 4 * kEnergyThreads;
 // blocks of the call in progress that have written their partial sum: every launch counts it
 // round to 0 again
 static __device__ unsigned g_energy_done;
@@ -232,7 +231,7 @@ extern "C" int ccx_ccd_energy_noalloc(int32_t nch, const int32_t *dims, const do
     return CCX_EINVAL;
   }
   if (nch > kMaxChannels) {
-    ccx::set_last_error("ccx_ccd_energy_noalloc: more than 16384 channels (the size of its static scratch)");
+    ccx::set_last_error("ccx_ccd_energy_noalloc: more than 16384 channels");
     return CCX_EINVAL;
   }
   int dev = 0;

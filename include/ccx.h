@@ -256,8 +256,8 @@ int ccx_ccd_energy(ccx_engine *e, double ener[2]);
  * t2 / vhhpp: device, the t2_ccm(ch)%val (n_pp x n_hh) and vnn_hhpp(ch)%val
  * (n_hh x n_pp) blocks concatenated in channel order, complex interleaved; energy:
  * device, 2 doubles.  Asynchronous on stream (NULL: the legacy default stream).
- * Scratch is a static device array of 16384 channel slots (512 KiB) held by each
- * GPU that loads the library until exit; nch > 16384 is rejected.  The first call
+ * Scratch is a static device array of one partial sum a thread block (some 5 KiB) held by
+ * each GPU that loads the library until exit; nch > 16384 is rejected.  The first call
  * in a CUDA context looks up that array's address -- make it before any stream
  * capture; the address is cached with the context's id, so after cudaDeviceReset (or
  * in a caller's own context) the next call looks it up again.
