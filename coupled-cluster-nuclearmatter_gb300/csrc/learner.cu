@@ -183,9 +183,11 @@ __device__ __forceinline__ float silu(float z) { return z * sigm(z); }
 // R tm .. R tm + R - 1 and the columns 4 tn .. 4 tn + 3 and 64 + 4 tn .. 64 + 4 tn + 3 of every
 // layer, so silu'(Z1), silu'(Z2), silu'(Z3) stay in its registers for the way back, and only the
 // 128-wide operand of the next product goes through shared memory (k-major).  The weights of a
-// product are copied while the one before it runs.  FP32 FMAs bound it: 1.7 GFLOP for 8192
-// samples.  The layers as 25 separate launches of a 64 x 64 tile GEMM, the gradients and column
-// sums among them on a few dozen blocks, took 966 us with the copies to and from the host; now 127.
+// product are copied while the one before it runs.  The FMAs (1.7 GFLOP for 8192 samples) keep
+// their pipe 40% busy and the issue slots 51%: one block of eight warps an SM waits for its
+// shared-memory reads and barriers.  The layers as 25 separate launches of a 64 x 64 tile GEMM, the gradients and column
+// sums among them on a few dozen blocks, took 966 us with the copies to and from the host; now 125,
+// of which this kernel 48, the weight gradients 26 and their sum 6.
 constexpr int kPassThreads = 256;
 constexpr int kWRow = kMlW;  // floats of one k of a weight operand in shared memory
 template <int R>
@@ -1062,8 +1064,8 @@ class Learner final : public ILearner {
   }
 
   // Tiles of 64 samples, or of 32 while that many leave SMs without one (a tile's time is
-  // latency and FMAs of one SM, so half the samples take half of it): 8192 samples 143 us a call in
-  // tiles of 64 and 169 of 32, 4096 samples 128 and 115.
+  // latency and FMAs of one SM, so half the samples take half of it): 8192 samples 125 us a call in
+  // tiles of 64 and 141 of 32, 4096 samples 111 and 98.
   int run_pass(const PassArgs &a) {
     return a.n <= 152 * PassTile<2>::kSamples ? run_tiles<2>(a) : run_tiles<4>(a);
   }

@@ -234,10 +234,11 @@ constexpr unsigned long long kTermOrder = 0x596A84210ull;
 // thread then forms four pairs (both spins of k and c), which share half of their reads.
 // Gathering the factors pair by pair through slot tables, 36 gathers of some ten dependent
 // loads each, kept the integer pipe and L1 busy and the FP32 pipe idle.  ms before and now, FP32
-// / FP64 contractions: PNM 14 nmax=2 0.32 to 0.21 / 0.36 to 0.34, PNM 54 nmax=2 8.5 to 2.0 / 9.0
-// to 4.2, SNM 28 nmax=2 6.8 to 1.5 / 12.8 to 10.2, SNM 76 nmax=2 (6.3e8 pairs) 88.5 to 10.6 /
-// 171 to 83.5.  FP32 issues 2 of 4 instructions a clock, the rest is the latency of the gathers and
-// barriers; FP64 is bound by its pipe.
+// / FP64 contractions: PNM 14 nmax=2 0.33 to 0.22 / 0.37 to 0.35, PNM 54 nmax=2 8.4 to 2.0 / 9.0
+// to 4.2, SNM 28 nmax=2 6.8 to 1.6 / 12.9 to 9.8, SNM 76 nmax=2 (6.3e8 pairs) 89.8 to 11.6 /
+// 170 to 82.1.  FP32 contractions of complex engines issue in 45% of the cycles beside an FP64 pipe
+// that is 47% busy with the sum (FMA pipe 19%, shared memory 24%); the rest is the latency of the
+// gathers and barriers.  FP64 contractions are bound by their pipe.
 template <typename W> struct alignas(2 * sizeof(W)) SpinPair {
   W v[2];  // the two spins of the closing orbital
 };
@@ -247,7 +248,7 @@ template <typename W, int G> struct TripleShape {
   static constexpr int kKets = G == 4 ? 1 : (sizeof(W) == 16 ? 4 : 8);
   static constexpr int kItems = G == 4 ? 320 : 16;
   // Two sets of tables where a ket fills the block (both isospins: the gathers of one ket run
-  // beside the pairs of the other, SNM 76 nmax=2 10.5 ms against 11.5 with one), one set and
+  // beside the pairs of the other, a tenth of SNM 76 nmax=2), one set and
   // twice the resident blocks otherwise (PNM 54 nmax=2 2.0 ms against 2.5).  Complex FP64 with
   // both isospins takes one set and two rounds of half as many threads, so that three blocks fit.
   static constexpr int kBuffers = sizeof(W) == 16 || G == 2 ? 1 : 2;
@@ -844,8 +845,8 @@ class Triples final : public ITriples<S> {
     // strides, segment by segment: the first segments hold most of the kets, so each block must get
     // some of all.  A lattice with fewer than two such items a block (a step of kets takes some 5 us,
     // and an item three to get going) gives every block one, every nseg-th test of its triples: SNM 4
-    // nmax=2 1280 to 139 us with FP64 contractions and 563 to 78 with FP32, SNM 28 nmax=1 503 to 327
-    // and 118 to 79, with the states and their order above.
+    // nmax=2 1280 to 139 us with FP64 contractions and 563 to 78 with FP32, SNM 28 nmax=1 503 to 326
+    // and 118 to 90, with the states and their order above.
     const int64_t tests = (int64_t)TD_.npm * TD_.npm;
     int64_t seg = std::max<int64_t>(48 * Sh::kKets, (int64_t)TD_.nbra * tests / (64 * want));
     seg = std::min(tests, (seg + Sh::kThreads - 1) / Sh::kThreads * Sh::kThreads);
